@@ -658,14 +658,8 @@ __global__ void __launch_bounds__(128)
 			continue;
 		Node8 *nd = nodes + it.slot;
 		if (empty_scene) { // a node without children
-			for (int c = 0; c < 8; ++c) {
-				Child8 ch;
-				ch.lo_x = ch.lo_y = ch.lo_z = __int_as_float(0x7FC00000);
-				ch.hi_x = ch.hi_y = ch.hi_z = __int_as_float(0x7FC00000);
-				ch.ref = kNone;
-				ch.pad = 0u;
-				nd->c[c] = ch;
-			}
+			for (int c = 0; c < 8; ++c)
+				nd->c[c] = encode_child(make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0), kNone);
 			continue;
 		}
 		const uint32_t base = nb + inc_i - n_inner, obase = ob + inc_i - n_inner;
@@ -673,10 +667,7 @@ __global__ void __launch_bounds__(128)
 		uint32_t k_inner = 0;
 #pragma unroll
 		for (int c = 0; c < 8; ++c) {
-			// An unused slot gets a NaN box: no slab test passes it.
-			float4 lo = make_float4(__int_as_float(0x7FC00000), __int_as_float(0x7FC00000),
-			                        __int_as_float(0x7FC00000), 0.f),
-			       hi = lo;
+			float4 lo = make_float4(0, 0, 0, 0), hi = lo;
 			uint32_t ref = kNone;
 			if (c < nc) {
 				const uint32_t r = C[c];
@@ -699,16 +690,7 @@ __global__ void __launch_bounds__(128)
 					dst += N[c];
 				}
 			}
-			Child8 ch;
-			ch.lo_x = lo.x;
-			ch.lo_y = lo.y;
-			ch.lo_z = lo.z;
-			ch.ref = ref;
-			ch.hi_x = hi.x;
-			ch.hi_y = hi.y;
-			ch.hi_z = hi.z;
-			ch.pad = 0u;
-			nd->c[c] = ch;
+			nd->c[c] = encode_child(lo, hi, ref);
 		}
 	}
 }
@@ -789,27 +771,23 @@ __global__ void __launch_bounds__(256)
 	// Groups of 8 lanes never straddle the node range, but the warp does: every lane
 	// takes part in the shuffles, idle ones with an empty child.
 	const unsigned gmask = 0xFFu << (threadIdx.x & 24u);
-	Child8 ch;
+	uint32_t r = kNone;
+	float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
 	if (live) {
 		const float4 *src = reinterpret_cast<const float4 *>(&nodes[i].c[k]);
 		const float4 a = __ldg(src), b = __ldg(src + 1);
-		ch.lo_x = a.x;
-		ch.lo_y = a.y;
-		ch.lo_z = a.z;
-		ch.ref = __float_as_uint(a.w);
-		ch.hi_x = b.x;
-		ch.hi_y = b.y;
-		ch.hi_z = b.z;
-	} else {
-		ch.ref = kNone;
-		ch.lo_x = ch.lo_y = ch.lo_z = ch.hi_x = ch.hi_y = ch.hi_z = 0.0f;
+		lo[0] = child_lo(a.x, a.z);
+		hi[0] = child_hi(a.x, a.z);
+		lo[1] = child_lo(a.y, a.w);
+		hi[1] = child_hi(a.y, a.w);
+		lo[2] = child_lo(b.x, b.y);
+		hi[2] = child_hi(b.x, b.y);
+		r = __float_as_uint(b.z);
 	}
-	const uint32_t r = ch.ref;
 	const bool used = r != kNone;
 	const bool leaf = used && (r & kLeafBit);
 	uint32_t cb = (used && !leaf) ? r : kNone;
 	uint32_t tb = leaf ? leaf_first(r) : kNone;
-	float lo[3] = {ch.lo_x, ch.lo_y, ch.lo_z}, hi[3] = {ch.hi_x, ch.hi_y, ch.hi_z};
 	float mn[3], mx[3];
 	for (int a = 0; a < 3; ++a) {
 		mn[a] = used ? lo[a] : INFINITY;

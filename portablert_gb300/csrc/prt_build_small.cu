@@ -186,19 +186,6 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *words, uint
 }
 
 // An 8-wide node's child record (an empty slot: NaN bounds and kNone).
-__device__ __forceinline__ Child8 make_child(float4 lo, float4 hi, uint32_t ref) {
-	Child8 ch;
-	ch.lo_x = lo.x;
-	ch.lo_y = lo.y;
-	ch.lo_z = lo.z;
-	ch.ref = ref;
-	ch.hi_x = hi.x;
-	ch.hi_y = hi.y;
-	ch.hi_z = hi.z;
-	ch.pad = 0u;
-	return ch;
-}
-
 // Position i's nearest neighbour within kRadius positions among m clusters: the least
 // pair in the order (union area, distance, parity of the lower position, lower position;
 // the last three as fields of 4, 1 and 12 bits), a total order, so the loop's order does
@@ -764,9 +751,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 			// record, a single triangle's from the leaf-box array.
 			uint32_t nz = 0;
 			bool in = false;
-			const float4 none = make_float4(__int_as_float(0x7FC00000), __int_as_float(0x7FC00000),
-			                                __int_as_float(0x7FC00000), 0.f);
-			float4 lo = none, hi = none;
+			float4 lo = make_float4(0, 0, 0, 0), hi = lo;
 			if (has) {
 				nz = (y & kLeaf16) ? 1u : cnt_s[y];
 				in = child_inner(y, nz, leaf_size, use_cost, bits_s);
@@ -826,10 +811,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 							}
 						}
 					}
-					nodes[slot].c[k] = make_child(lo, hi, ref);
+					nodes[slot].c[k] = encode_child(lo, hi, ref);
 				}
 				if (c8 >= nc) // the slots after the last child
-					nodes[slot].c[c8] = make_child(none, none, kNone);
+					nodes[slot].c[c8] = encode_child(lo, hi, kNone);
 			}
 			n_nodes += total & 0xFFFFu;
 			next_items += total & 0xFFFFu;

@@ -35,13 +35,14 @@ enum : uint32_t {
 	kErrSah = 8u,      // SAH build: a range, node id or task list check failed
 };
 
-// One child of an 8-wide FP32 node: its box and its reference, 32 B, so the lane that
-// tests child c reads it with one 32-byte load and a node's 8 children are 256
-// contiguous bytes.
+// One child of an 8-wide FP32 node: its box as centre and half extent and its reference,
+// 32 B, so the lane that tests child c reads it with one 32-byte load and a node's 8
+// children are 256 contiguous bytes.  x and y sit in aligned pairs for the packed FP32
+// arithmetic of the slab test.  encode_child makes the record, child_lo / child_hi bound
+// the box from outside.
 struct alignas(16) Child8 {
-	float lo_x, lo_y, lo_z;
+	float cx, cy, ex, ey, cz, ez;
 	uint32_t ref;
-	float hi_x, hi_y, hi_z;
 	uint32_t pad;
 };
 struct alignas(16) Node8 {
@@ -110,15 +111,20 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 }
 
 // Per-ray constants.  `kind` selects the box test used on inner nodes:
-//   0 regular: all three reciprocals finite; the plain slab test is exact and safe.
-//   1 axis:    some reciprocal is infinite (a zero or denormal direction component);
-//              inner nodes use conservative_box below.
+//   0 regular: every origin component within 2^67 and every direction component between
+//              2^-58 and 2^60 in magnitude: the slab test on centres and half extents
+//              (child_passes in prt_traverse.cu) neither overflows nor meets a NaN.
+//   1 axis:    another finite ray, for instance with a zero direction component (infinite
+//              reciprocal); inner nodes use conservative_box below.
 //   2 all:     a non-finite component or all reciprocals infinite: every inner box
 //              passes and only the exact per-triangle test decides.
 struct RayC {
 	float ox, oy, oz, dx, dy, dz, fx, fy, fz;
 	int kind;
 };
+
+// (2^67 + 2^67) * 2^58 stays below FLT_MAX; 2^67 is about 1.5e20.
+constexpr float kCoordMax = 0x1p67f, kDirMax = 0x1p60f, kDirMin = 0x1p-58f;
 
 __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx, float dy,
                                          float dz) {
@@ -129,12 +135,53 @@ __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx,
 	r.fx = __frcp_rn(dx);
 	r.fy = __frcp_rn(dy);
 	r.fz = __frcp_rn(dz);
-	bool fin = isfinite(ox) && isfinite(oy) && isfinite(oz) && isfinite(dx) && isfinite(dy) &&
-	           isfinite(dz);
-	int n_inf = (int)isinf(r.fx) + (int)isinf(r.fy) + (int)isinf(r.fz);
-	r.kind = (!fin || n_inf == 3) ? 2 : (n_inf ? 1 : 0);
+	// (A NaN component fails its comparison, so it is never regular.)
+	const bool regular = fabsf(ox) <= kCoordMax && fabsf(oy) <= kCoordMax &&
+	                     fabsf(oz) <= kCoordMax && fabsf(dx) <= kDirMax &&
+	                     fabsf(dy) <= kDirMax && fabsf(dz) <= kDirMax && fabsf(dx) >= kDirMin &&
+	                     fabsf(dy) >= kDirMin && fabsf(dz) >= kDirMin;
+	r.kind = 0;
+	if (!regular) {
+		const bool fin = isfinite(ox) && isfinite(oy) && isfinite(oz) && isfinite(dx) &&
+		                 isfinite(dy) && isfinite(dz);
+		const int n_inf = (int)isinf(r.fx) + (int)isinf(r.fy) + (int)isinf(r.fz);
+		r.kind = (!fin || n_inf == 3) ? 2 : 1;
+	}
 	return r;
 }
+
+// One axis of a child record: centre c and half extent e with [lo, hi] inside
+// [c - e, c + e] and e wider than that needs by a factor 1 + 2^-21 (the margin that the
+// test's rounding uses up).  A bound beyond 2^67 makes the axis [-FLT_MAX, FLT_MAX].
+__device__ __forceinline__ void encode_axis(float lo, float hi, float &c, float &e) {
+	if (!(lo >= -kCoordMax && hi <= kCoordMax)) {
+		c = 0.0f;
+		e = 3.402823466e+38f;
+		return;
+	}
+	c = __fadd_rn(__fmul_rn(lo, 0.5f), __fmul_rn(hi, 0.5f));
+	e = __fmul_ru(fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo)), 1.0f + 0x1p-21f);
+}
+
+// The record of a child box; ref == kNone: an unused slot (a NaN box, which no regular
+// ray's test passes).
+__device__ __forceinline__ Child8 encode_child(const float4 &lo, const float4 &hi, uint32_t ref) {
+	Child8 ch;
+	if (ref == kNone) {
+		ch.cx = ch.cy = ch.cz = ch.ex = ch.ey = ch.ez = __int_as_float(0x7FC00000);
+	} else {
+		encode_axis(lo.x, hi.x, ch.cx, ch.ex);
+		encode_axis(lo.y, hi.y, ch.cy, ch.ey);
+		encode_axis(lo.z, hi.z, ch.cz, ch.ez);
+	}
+	ch.ref = ref;
+	ch.pad = 0u;
+	return ch;
+}
+
+// Bounds that contain the box a record was made from.
+__device__ __forceinline__ float child_lo(float c, float e) { return __fsub_rd(c, e); }
+__device__ __forceinline__ float child_hi(float c, float e) { return __fadd_ru(c, e); }
 
 // Slab test of portableRT's ray_box_intersect (bvh.hpp:195-222), bit for bit: each
 // t is (bound - origin) * reciprocal in round-to-nearest, combined with the select

@@ -149,28 +149,87 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 	return r;
 }
 
-// regular_box with its two comparisons folded into one: tmax >= 0 and tmin <= tmax hold
-// exactly when max(tmin, 0) <= tmax, and the 0 joins the last axis' minimum.  Same
-// products, same answer (an unused slot's NaN box: max(NaN, 0) = 0, and 0 <= NaN fails);
-// one ALU instruction fewer per child, which the half-rate ALU pipe of FP32-node steps
-// turns into 1 % more rays (compressed nodes measured 1 % slower with it, so they keep
-// regular_box).
-__device__ __forceinline__ bool regular_box_folded(const RayC &r, float lx, float hx, float ly,
-                                                   float hy, float lz, float hz) {
-	const float t1 = (lx - r.ox) * r.fx, t2 = (hx - r.ox) * r.fx;
-	const float t3 = (ly - r.oy) * r.fy, t4 = (hy - r.oy) * r.fy;
-	const float t5 = (lz - r.oz) * r.fz, t6 = (hz - r.oz) * r.fz;
-	const float tmin = max3f(fminf(t1, t2), fminf(t3, t4), fmaxf(fminf(t5, t6), 0.0f));
-	const float tmax = min3f(fmaxf(t1, t2), fmaxf(t3, t4), fmaxf(t5, t6));
-	return tmin <= tmax;
+// Packed FP32 pairs (sm_100 and later): one instruction for two lanes' worth of a
+// component, each half rounded as the scalar operation rounds it.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+	unsigned long long r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+	return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+	unsigned long long r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
 }
 
-template <bool REGULAR, bool FOLDED = false>
+// What the slab test on centres and half extents needs of a ray, x and y in pairs.
+struct SlabRay {
+	unsigned long long no, f, af, naf; // -origin, reciprocal, |reciprocal|, -|reciprocal|
+	float oz, fz, afz;
+};
+
+__device__ __forceinline__ SlabRay slab_ray(const RayC &r) {
+	SlabRay q;
+	q.no = pack2(-r.ox, -r.oy);
+	q.f = pack2(r.fx, r.fy);
+	q.af = pack2(fabsf(r.fx), fabsf(r.fy));
+	q.naf = pack2(-fabsf(r.fx), -fabsf(r.fy));
+	q.oz = r.oz;
+	q.fz = r.fz;
+	q.afz = fabsf(r.fz);
+	return q;
+}
+
+// Slab test of a regular ray (kind 0) on an inner box given as centre c and half extent e
+// (encode_axis): per axis t = (c - o) * f, near = t - e |f|, far = t + e |f|.  Passes
+// whenever the reference's slab test passes on some triangle box inside, so it prunes
+// nothing the exact test would accept:
+//  * with u = 2^-24, the computed near is at most its real value A plus 3.1 u |A| and far at
+//    least B less 3.1 u |B|: the rounding of t is relative to |t| <= |A| + e |f|, and the
+//    e |f| part is covered by the 8 u that encode_axis widens e by;
+//  * the reference's own near and far of a box inside, (bound - o) * f, are off by at most
+//    2.1 u of themselves;
+//  * so for a triangle the reference passes (0 <= its tmax, its tmin <= its tmax), the
+//    largest near (or 0) here is at most tmax (1 + 5.2 u) and the smallest far at least
+//    tmax (1 - 5.2 u), up to underflow (a few 2^-149): the factor 1 + 16 u and the
+//    2^-120 on the far side cover both, and the rounding of that product.
+// 13 FP instructions and 3 on the half-rate ALU pipe for a box, against 12 and 9 for
+// (bound - origin) * reciprocal on both bounds with its min / max per axis; x and y are
+// packed, so 9 + 3 are issued.  (2,073,600 camera and 4,194,304 secondary rays on the
+// 1,048,576-triangle heightfield: 1,514 -> 1,419 us under sustained load;
+// 363 -> 323 M warp instructions for 1.5M of those rays, ALU-pipe 147 -> 118 M.)
+__device__ __forceinline__ bool child_passes(const SlabRay &q, const float4 &a, const float4 &b) {
+	const unsigned long long t = mul2(add2(pack2(a.x, a.y), q.no), q.f);
+	const unsigned long long e = pack2(a.z, a.w);
+	float nx, ny, fx, fy;
+	unpack2(fma2(e, q.naf, t), nx, ny);
+	unpack2(fma2(e, q.af, t), fx, fy);
+	const float tz = (b.x - q.oz) * q.fz;
+	const float nz = __fmaf_rn(-b.y, q.afz, tz), fz = __fmaf_rn(b.y, q.afz, tz);
+	const float tmin = max3f(nx, ny, fmaxf(nz, 0.0f));
+	const float tmax = min3f(fx, fy, fz);
+	return tmin <= __fmaf_rn(tmax, 1.0f + 0x1p-20f, 0x1p-120f);
+}
+
+template <bool REGULAR>
 __device__ __forceinline__ bool box_test(const RayC &r, float lx, float hx, float ly, float hy,
                                          float lz, float hz) {
 	if (REGULAR || r.kind == 0)
-		return FOLDED ? regular_box_folded(r, lx, hx, ly, hy, lz, hz)
-		              : regular_box(r, lx, hx, ly, hy, lz, hz);
+		return regular_box(r, lx, hx, ly, hy, lz, hz);
 	return conservative_box(r, lx, hx, ly, hy, lz, hz);
 }
 
@@ -248,21 +307,26 @@ __device__ __forceinline__ void test_queued(const float4 *__restrict__ tri4, War
 // Child `k` of `node`: slab test and what it refers to.
 template <int FMT, bool REGULAR>
 __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const RayC &r,
-                                           uint32_t node, int k, bool &hit, bool &inner,
+                                           const SlabRay &q, uint32_t node, int k, bool &hit, bool &inner,
                                            uint32_t &child, uint32_t &leaf_n) {
 	hit = false;
 	inner = false;
 	child = 0;
 	leaf_n = 0;
 	if (FMT == PRT_NODES_FP32) {
-		float4 lo, hi;
-		ld_nc_256(&(static_cast<const Node8 *>(nodes) + node)->c[k], lo, hi);
-		const uint32_t ref = __float_as_uint(lo.w);
-		// An unused slot has a NaN box, which the plain slab test never passes; the
+		float4 a, b;
+		ld_nc_256(&(static_cast<const Node8 *>(nodes) + node)->c[k], a, b);
+		const uint32_t ref = __float_as_uint(b.z);
+		// An unused slot has a NaN box, which a regular ray's test never passes; the
 		// conservative test would, so only the general pass checks the reference.
 		if (REGULAR || ref != kNone) {
 			inner = !ref_is_leaf(ref);
-			hit = box_test<REGULAR, true>(r, lo.x, hi.x, lo.y, hi.y, lo.z, hi.z);
+			if (REGULAR || r.kind == 0)
+				hit = child_passes(q, a, b);
+			else
+				hit = conservative_box(r, child_lo(a.x, a.z), child_hi(a.x, a.z),
+				                       child_lo(a.y, a.w), child_hi(a.y, a.w),
+				                       child_lo(b.x, b.y), child_hi(b.x, b.y));
 			// A node index, or a leaf's first triangle: both below 2^27, under the
 			// leaf flag and count bits.
 			child = ref & kIndexMask;
@@ -360,6 +424,7 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		__syncwarp(); // the pops above are read before the pushes below overwrite them
 		const uint32_t slot = item >> kIndexBits, node = item & kIndexMask;
 		const RayC r = slot_ray(S, slot);
+		const SlabRay sr = slab_ray(r); // (FP32 nodes)
 		if (COUNT && work && s == 0)
 			++n_visits;
 
@@ -367,7 +432,7 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		uint32_t child[kChildPerLane], leaf_n[kChildPerLane];
 #pragma unroll
 		for (int j = 0; j < kChildPerLane; ++j) {
-			test_child<FMT, REGULAR>(nodes, r, node, s + kLanesPerNode * j, hit[j], inner[j],
+			test_child<FMT, REGULAR>(nodes, r, sr, node, s + kLanesPerNode * j, hit[j], inner[j],
 			                         child[j], leaf_n[j]);
 			hit[j] = hit[j] && work;
 		}
