@@ -27,12 +27,14 @@
 //    items are left.  Unused child slots hold NaN boxes, which no plain slab test
 //    passes.
 //  * A query of ray buffers is two launches: a regular pass over the batches whose 32
-//    rays all have finite reciprocals (the plain slab test only), which counts and skips
-//    the others, and a deferred pass over those with the conservative test for zero
-//    direction components (it returns at once when there are none).  Camera queries and
-//    counting runs are one general launch.  A request server's serving launch (pass 3)
-//    takes its batches from device queues that the host extends while it runs
-//    (claim_batch) and picks the plain or the general test per batch.
+//    rays are all regular (kind 0: the plain slab test only), which counts and skips
+//    the others, and a deferred pass over those with the conservative test, for instance for
+//    zero direction components (it returns at once when there are none).  Camera queries and
+//    counting runs are one general launch, in which a batch of regular rays takes the
+//    plain test; camera batches start with a packet descent (packet_descent).  A request
+//    server's serving launch (pass 3) takes its batches from device queues that the host
+//    extends while it runs (claim_batch) and picks the plain or the general test per
+//    batch.
 //  * When 32 triangles are queued, the 32 lanes test one each with the exact reference
 //    test and fold (t, primitive id) into the slot's 64-bit key with a shared atomicMin;
 //    with FP32 nodes the lane whose key the slot kept records its u, v (and a zero t's
@@ -67,6 +69,15 @@ constexpr int kLanesPerNode = PRT_TRAVERSE_LANES_PER_NODE;
 constexpr int kItems = 32 / kLanesPerNode;       // items per step (K)
 constexpr int kChildPerLane = 8 / kLanesPerNode;
 constexpr int kMaxDepth = 32;
+// Packet descent (packet_descent): rays that must share a node for the warp to test it for
+// all of them at once; its stack (one entry per lane); the per-ray lists of nodes it leaves
+// to item steps, and the length past which it stops descending.
+constexpr uint32_t kPacketMin = 8;
+constexpr uint32_t kPacketStack = 32;
+constexpr uint32_t kListWords = 64;
+constexpr uint32_t kListStop = kListWords - 8u - kPacketStack;
+// Items that admission from the lists fills the pool up to.
+constexpr uint32_t kAdmit = 24;
 
 struct TravArgs {
 	const SceneDesc *scenes; // scene table (n_segs > 0)
@@ -366,6 +377,22 @@ __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const
 	}
 }
 
+// What child `k` of `node` refers to, as a Node8 reference (kNone: an unused slot).
+template <int FMT>
+__device__ __forceinline__ uint32_t child_ref(const void *__restrict__ nodes, uint32_t node,
+                                              int k) {
+	if (FMT == PRT_NODES_FP32)
+		return __ldg(&(static_cast<const Node8 *>(nodes) + node)->c[k].ref);
+	const CNode8 *cn = static_cast<const CNode8 *>(nodes) + node;
+	const uint4 w0 = __ldg(reinterpret_cast<const uint4 *>(cn));
+	const uint2 w1 = __ldg(reinterpret_cast<const uint2 *>(cn) + 2);
+	const uint32_t ck = __ldg(reinterpret_cast<const uint2 *>(&cn->c[k])).y;
+	const uint32_t imask = byte_of(w0.w, 3), m = byte_of(ck, 2);
+	if ((imask >> k) & 1u)
+		return w1.x + __popc(imask & ((1u << k) - 1u));
+	return m ? make_leaf(w1.y + byte_of(ck, 3), m) : kNone;
+}
+
 // Resident blocks per SM the register budget is set for, per node format (measured on
 // the 1M-triangle heightfield: 9 blocks of 4 warps = 56 registers, with a few spilled
 // words, is fastest for both formats).
@@ -376,10 +403,110 @@ __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const
 #define PRT_TRAVERSE_MIN_BLOCKS_COMPRESSED 9
 #endif
 
+// The packet descent of a batch: from the root, every node that at least kPacketMin of the
+// warp's rays visit is tested for all of them at once, lane = slot, all lanes on the same
+// child (its record is one broadcast load).  Inner children that fewer rays pass go to
+// those rays' lists (`list`, local memory, `listed` entries), which the item steps then
+// take up; leaf triangles are queued.  The same tests on the same rays as item steps
+// make, so the same records.
+//
+// Why: a node that m rays of the warp visit costs m / 8 item steps of about 110 warp
+// instructions and 2 L1 wavefronts per ray; here it costs the same few hundred instructions
+// and 8 wavefronts for any m.  A camera's 32 neighbouring pixels share most of their nodes:
+// 2048 x 2048 pixels on a closed mesh of 4,968 triangles, traversal and shading 404 ->
+// 308 us (kPacketMin 8 / 12 / 16 / 20: 308 / 312 / 316 / 320).  Ray buffers keep the item
+// steps: on the heightfield's camera and secondary rays the descent at 16 / 20 measured
+// 1,644 / 1,618 us against 1,561 without, and incoherent rays share only the top levels.
+// (Tiles of 8 x 4 pixels instead of 32 of a row: 4 % fewer instructions, but 365 us: the
+// four rays of a tile with a zero x direction, which pass every box around x = 0, end up
+// in one warp, and the last of those tiles is the launch's tail.)
+//
+// Bounds: a node with fewer than 8 free stack entries, or met when some list is past
+// kListStop, is not opened but goes to its rays' lists; a list grows by at most 8 per
+// opened node and one per unopened entry, so it stays under kListWords.
+template <int FMT, bool LEAF1>
+__device__ __forceinline__ void packet_descent(const TravArgs &a, const SceneDesc &sd,
+                                               WarpFixed &S, uint32_t *queue, uint32_t nb,
+                                               int lane, uint32_t lt, uint32_t step_limit,
+                                               uint32_t *list, uint32_t &listed, uint32_t &q,
+                                               bool &fault) {
+	const float4 *__restrict__ tri4 = sd.tri4;
+	const void *__restrict__ nodes = sd.nodes;
+	// The stack: lane k holds entry k (a node and the slots that visit it).
+	uint32_t st_node = sd.root, st_rays = 0xFFFFFFFFu >> (32u - nb), sp = 1, steps = 0;
+	while (sp > 0u) {
+		--sp;
+		const uint32_t node = __shfl_sync(0xFFFFFFFFu, st_node, (int)sp);
+		const uint32_t rays = __shfl_sync(0xFFFFFFFFu, st_rays, (int)sp);
+		const bool mine = (rays >> lane) & 1u;
+		if (++steps > step_limit) { // a malformed tree
+			if (lane == 0)
+				atomicOr(a.err, kErrStack);
+			fault = true;
+			break;
+		}
+		if (__popc(rays) < (int)kPacketMin || sp + 8u > kPacketStack ||
+		    __any_sync(0xFFFFFFFFu, listed > kListStop)) {
+			if (mine)
+				list[listed++] = node;
+			continue;
+		}
+		const RayC r = slot_ray(S, (uint32_t)lane);
+		const SlabRay sr = slab_ray(r);
+		// Lane c: what child c refers to, and the rays that pass it.
+		const uint32_t c_ref = child_ref<FMT>(nodes, node, lane & 7);
+		uint32_t c_rays = 0;
+#pragma unroll 4
+		for (int c = 0; c < 8; ++c) {
+			bool hit, inner;
+			uint32_t child, leaf_n;
+			test_child<FMT, true>(nodes, r, sr, node, c, hit, inner, child, leaf_n);
+			const uint32_t b = __ballot_sync(0xFFFFFFFFu, hit && mine);
+			if (lane == c)
+				c_rays = b;
+		}
+		uint32_t todo = __ballot_sync(0xFFFFFFFFu, c_rays != 0u);
+		while (todo) {
+			const int c = __ffs(todo) - 1;
+			todo &= todo - 1u;
+			const uint32_t b = __shfl_sync(0xFFFFFFFFu, c_rays, c);
+			const uint32_t ref = __shfl_sync(0xFFFFFFFFu, c_ref, c);
+			const uint32_t n = __popc(b);
+			const bool in = (b >> lane) & 1u;
+			if (ref_is_leaf(ref)) {
+				const uint32_t m = LEAF1 ? 1u : leaf_count(ref);
+				for (uint32_t k = 0; k < m; ++k) {
+					if (in)
+						queue[q + __popc(b & lt)] =
+						    ((uint32_t)lane << kIndexBits) | ((ref & kIndexMask) + k);
+					q += n;
+					__syncwarp();
+					if (q >= 32u) {
+						q -= 32u;
+						uint32_t none = 0;
+						test_queued<false, FMT == PRT_NODES_FP32>(tri4, S, queue, q, 32u, lane,
+						                                          none);
+						__syncwarp();
+					}
+				}
+			} else if (n >= kPacketMin) {
+				if (lane == (int)sp) {
+					st_node = ref;
+					st_rays = b;
+				}
+				++sp;
+			} else if (in) {
+				list[listed++] = ref;
+			}
+		}
+	}
+}
+
 // The traversal of one batch of up to 32 rays (slots 0..nb-1 of S) through scene sd.
-// REGULAR: every ray of the batch has finite reciprocals, so inner boxes take the plain
-// slab test only (no branch to the conservative test per child).
-template <int FMT, bool COUNT, bool LEAF1, bool REGULAR>
+// REGULAR: every ray of the batch is regular (kind 0), so inner boxes take the plain slab
+// test only (no branch to the conservative test per child).  PACKET: it starts with a packet
+// descent.
+template <int FMT, bool COUNT, bool LEAF1, bool REGULAR, bool PACKET = false>
 __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uint32_t *queue,
                                             uint32_t *pool, const SceneDesc &sd, uint32_t nb,
                                             int lane, int g, int s, uint32_t lt,
@@ -389,13 +516,29 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 	const void *__restrict__ nodes = sd.nodes;
 	uint32_t top = 0;  // items in the pool (warp-uniform)
 	uint32_t q = 0;    // queued triangles (warp-uniform)
-	uint32_t next = 0; // next slot whose root is not yet in the pool
+	uint32_t next = 0; // next slot whose root is not yet in the pool; after a packet
+	                   // descent, the nodes left in this lane's list
 	uint32_t steps = 0;
+	uint32_t list[PACKET ? kListWords : 1u];
+	bool listed = PACKET; // some list may hold a node
+	if (PACKET)
+		packet_descent<FMT, LEAF1>(a, sd, S, queue, nb, lane, lt, step_limit, list, next, q,
+		                           fault);
 	for (;;) {
-		// Admit new rays while fewer than K items are pending (a branch the common step
+		// Admit new work while fewer than K items are pending (a branch the common step
 		// skips with one test).
 		if (top < (uint32_t)kItems) {
-			if (next < nb) {
+			if (PACKET) {
+				if (listed) {
+					const uint32_t left = __ballot_sync(0xFFFFFFFFu, next > 0u);
+					const uint32_t add = kAdmit - top, at = __popc(left & lt);
+					if (next > 0u && at < add)
+						pool[top + at] = ((uint32_t)lane << kIndexBits) | list[--next];
+					top += min(add, (uint32_t)__popc(left));
+					listed = left != 0u;
+					__syncwarp();
+				}
+			} else if (next < nb) {
 				const uint32_t add = min((uint32_t)kItems - top, nb - next);
 				if ((uint32_t)lane < add)
 					pool[top + lane] = ((next + lane) << kIndexBits) | sd.root;
@@ -741,8 +884,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, FMT == PRT_NODES_FP32
 			}
 			if (PASS == 2 && regular)
 				continue; // done by the regular pass
-			if (PASS == 3 && regular)
-				trace_batch<FMT, COUNT, LEAF1, true>(a, S, queue, pool, sd, nb, lane, g, s, lt,
+			constexpr bool kPacket = PASS == 0 && !COUNT;
+			if ((PASS == 3 || kPacket) && regular)
+				trace_batch<FMT, COUNT, LEAF1, true, kPacket>(a, S, queue, pool, sd, nb, lane, g, s, lt,
 				                                     step_limit, n_visits, n_tests, fault);
 			else
 				trace_batch<FMT, COUNT, LEAF1, PASS == 1>(a, S, queue, pool, sd, nb, lane, g, s,
@@ -937,7 +1081,8 @@ void launch(const TravArgs &a, int warps, int sm_count, cudaStream_t st) {
 
 void size_smem(TravArgs &a, uint32_t depth, int leaf_size) {
 	depth = std::max<uint32_t>(depth, 1u);
-	a.pool_cap = std::max<uint32_t>(256u, 7u * kItems * (depth - 1u) + 2u * kItems);
+	a.pool_cap = std::max<uint32_t>(256u, 7u * kItems * (depth - 1u) + kItems +
+	                                          (a.use_cam ? kAdmit : (uint32_t)kItems));
 	a.queue_cap = 32u + (uint32_t)kItems * 8u * (uint32_t)std::max(leaf_size, 1);
 	a.max_leaf = (uint32_t)std::max(leaf_size, 1);
 	a.max_batches = 0;
