@@ -99,7 +99,6 @@ struct BuildScratch {
 	DevBuf flags;                     // refit arrival counters
 	DevBuf items_a, items_b;          // collapse frontiers
 	DevBuf counters;                  // per-level frontier sizes, node / triangle counters
-	DevBuf perm;                      // leaf-order slot -> sorted index
 	DevBuf sort_hist, sort_tiles, sort_status;
 	DevBuf bounds;                    // centroid bounds, 6 ordered words per scene
 	DevBuf sah;                       // SAH build: records, task lists, bins, counters
