@@ -1159,7 +1159,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 		for (int k = 0; k < ahead && level < kMaxLevels; ++k, ++level) {
 			// No more blocks than the level can have items for.
 			const uint64_t items =
-			    std::min<uint64_t>((uint64_t)S << std::min(3 * level, 40), plan.node_cap);
+			    std::min<uint64_t>((uint64_t)S << std::min(3 * level, 30), plan.node_cap);
 			const unsigned grid = (unsigned)std::min<uint64_t>(
 			    1216, (items + kCollapseItems - 1) / kCollapseItems);
 			k_collapse<<<grid, 8 * kCollapseItems, 0, st>>>(A, items_of[level & 1], ctr + level,

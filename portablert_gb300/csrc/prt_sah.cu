@@ -12,11 +12,11 @@
 // number of boxes a ray passes does, which is what the heuristic minimises.
 //
 // Tasks are ranges still to be split, in three tiers by size:
-//   large (> 512 triangles): per level, blocks bin chunks of 2048 triangles into the
-//         task's 3 x 32 global bins (k_sah_bin), one warp per task picks the plane
-//         (k_sah_split), blocks scatter the triangles to the other buffer (k_sah_part);
-//   mid   (33-512): one warp per task per level does all three in shared memory with a
-//         stable ballot partition (k_sah_mid);
+//   large (> 512 triangles): level by level, one warp per task picks the plane from the
+//         task's 3 x 32 global bins (k_sah_split) and blocks scatter chunks of 1,024
+//         triangles to the other buffer, adding each to the bins of the child it goes to
+//         (k_sah_part; k_sah_bin fills the roots' bins);
+//   mid   (33-512): one block per task, all its levels in shared memory (k_sah_mid);
 //   small (<= 32): one warp builds the whole subtree, one triangle per lane, with an
 //         exact sweep over the sorted centres of each axis (k_sah_small).
 // Binning uses box centres; a task deeper than 48 levels, or one whose centres all fall
@@ -38,7 +38,8 @@ constexpr int kBins = 32;
 constexpr uint32_t kLarge = 512;    // larger tasks are binned by many blocks (512 / 1,024
                                     // / 4,096: heightfield build 3.05 / 3.16 / 3.83 ms)
 constexpr uint32_t kSmall = 32;     // tasks up to this size go to one warp each
-constexpr uint32_t kChunk = 2048;   // triangles per binning / partition block
+constexpr uint32_t kPer = 4;        // triangles per thread of a binning / partition block
+constexpr uint32_t kChunk = 256 * kPer; // triangles per such block
 constexpr uint32_t kDepthGuard = 48;
 constexpr int kMaxLevels = 96;
 constexpr int kLevelsPerCheck = 4;
@@ -47,19 +48,21 @@ constexpr uint32_t kOrdPosInf = 0xFF800000u; // f2ord(+inf)
 constexpr uint32_t kOrdNegInf = 0x007FFFFFu; // f2ord(-inf)
 constexpr uint32_t kHalves = 3;              // split "axis" meaning: first half / second half
 
-// Counter words.
+// Counter words: list sizes and node ids, then the large tasks and the chunks of each
+// level.
 enum : int {
-	kCtrLarge = 0, // [0], [1]: large tasks per list parity
-	kCtrMid = 2,   // [2], [3]: mid tasks per list parity
-	kCtrSmall = 4,
-	kCtrNodes = 5,
-	kCtrChunks = 6,
-	kCtrWordsSah = 8
+	kCtrSmall = 0,
+	kCtrMid = 1,
+	kCtrNodes = 2,
+	kCtrLarge = 4,
+	kCtrChunks = kCtrLarge + kMaxLevels + 2,
+	kCtrWordsSah = kCtrChunks + kMaxLevels + 2
 };
-static_assert(kCtrWordsSah + 1 <= kHostSahWords, "the SAH counters' pinned words");
 
 struct alignas(16) SahTask {
-	uint32_t begin, count, node, parent; // parent = (node << 1 | side), kNone at a root
+	uint32_t begin, count, node, parent; // parent = (node << 1 | side), kNone at a root;
+	                                     // a split large task keeps here the list slots
+	                                     // of its left and right child (kNone: not large)
 	uint32_t meta;                       // bit 0: buffer holding the range; bits 8-15: depth
 	uint32_t axis, split, n_left;        // the split chosen (large tasks)
 	float lo[3];
@@ -69,34 +72,35 @@ struct alignas(16) SahTask {
 };
 static_assert(sizeof(SahTask) == 64, "task layout");
 
-struct alignas(16) SmallTask {
+struct SmallTask {
 	uint32_t begin, meta, node, parent;  // meta: count | buffer << 8 | depth << 16
+	uint32_t base;                       // first id for the nodes below (kNone: to be drawn)
 };
 
 struct SahArgs {
 	float4 *rec[2];         // (lo, id) (hi, 0) per triangle, two buffers
 	SahTask *large[2];
 	uint32_t *bins[2];      // kBinWords per large task
-	SahTask *mid[2];
+	uint2 *chunk[2];        // per chunk of the level: large task, first triangle
+	SahTask *mid;
 	SmallTask *small;
-	uint32_t *chunk_off;    // per large task of the level: first chunk
 	uint32_t *ctr;
 	uint32_t *vals;         // out: position -> triangle index
 	float4 *lbox;           // out: leaf boxes by position
 	uint32_t *left, *right, *rfirst, *rlast;
 	float4 *ibox;
 	uint32_t *parent_int, *parent_leaf; // for the bottom-up cost pass of the collapse
-	uint32_t node_cap, max_large, max_mid, max_small;
+	uint32_t node_cap, max_large, max_mid, max_small, max_chunks;
 	uint32_t n;             // triangles (records per buffer)
 	uint32_t *err;
 };
 
-// Task counts clamped to the list capacities (a list that overflowed was flagged).
-__device__ __forceinline__ uint32_t n_large(const SahArgs &A, int par) {
-	return min(A.ctr[kCtrLarge + par], A.max_large);
+// Counts clamped to the list capacities (a list that overflowed was flagged).
+__device__ __forceinline__ uint32_t n_large(const SahArgs &A, int level) {
+	return min(A.ctr[kCtrLarge + level], A.max_large);
 }
-__device__ __forceinline__ uint32_t n_mid(const SahArgs &A, int par) {
-	return min(A.ctr[kCtrMid + par], A.max_mid);
+__device__ __forceinline__ uint32_t n_chunks(const SahArgs &A, int level) {
+	return min(A.ctr[kCtrChunks + level], A.max_chunks);
 }
 
 __device__ __forceinline__ bool range_ok(const SahArgs &A, uint32_t begin, uint32_t count) {
@@ -130,38 +134,88 @@ __device__ __forceinline__ float rec_c(const float4 &lo, const float4 &hi, int k
 
 __device__ __forceinline__ void flag(uint32_t *err) { atomicOr(err, kErrSah); }
 
-__device__ __forceinline__ void bins_init(uint32_t *b, int lane) {
-	for (int k = lane; k < kBinWords; k += 32) {
+__device__ __forceinline__ void bins_init(uint32_t *b, int at, int step, int words = kBinWords) {
+	for (int k = at; k < words; k += step) {
 		const int w = k % 7;
 		b[k] = w < 3 ? kOrdPosInf : (w < 6 ? kOrdNegInf : 0u);
 	}
 }
 
-// Adds each valid lane's triangle to the bins of all three axes (shared or global
-// words).  Counts go in once per group of lanes with the same bin; bounds only when
-// they improve what is there.
-__device__ __forceinline__ void bins_add(uint32_t *b, bool valid, const float4 &lo,
+// Adds each valid lane's triangle to the bins of all three axes; `set` selects one of two
+// sets of kBinWords words (with the lane's own frame).  Where the warp's triangles fall into
+// few bins (meshes list neighbours together), each group of lanes with the same bin reduces
+// first and one lane updates the bin; lanes of many bins update them one by one, bounds only
+// when they improve what is there.
+// 0 / 1 / 2 / 4 / 8: heightfield build 1.89 / 1.86 / 1.80 / 1.85 / 2.07 ms; the clusters, in
+// random order, 13.6 ms with 0 and 14.3 with 2: set for meshes, whose files list neighbours
+// together.
+constexpr int kBinGroups = 2;
+
+__device__ __forceinline__ void bins_add(uint32_t *b, bool valid, uint32_t set, const float4 &lo,
                                          const float4 &hi, const float *flo, const float *fsc,
                                          int lane) {
+	const uint32_t v[6] = {f2ord(lo.x), f2ord(lo.y), f2ord(lo.z),
+	                       f2ord(hi.x), f2ord(hi.y), f2ord(hi.z)};
 #pragma unroll
 	for (int a = 0; a < 3; ++a) {
-		const int bin = valid ? bin_of(rec_c(lo, hi, a), flo[a], fsc[a]) : -1;
+		const int bin =
+		    valid ? (int)set * 3 * kBins + a * kBins + bin_of(rec_c(lo, hi, a), flo[a], fsc[a]) : -1;
 		const uint32_t g = __match_any_sync(0xFFFFFFFFu, bin);
-		if (!valid)
+		const bool lead = valid && lane == __ffs(g) - 1;
+		uint32_t leads = __ballot_sync(0xFFFFFFFFu, lead);
+		uint32_t *w = b + bin * 7;
+		if (__popc(leads) <= kBinGroups) {
+			while (leads) { // one group of lanes at a time
+				const uint32_t m = __shfl_sync(0xFFFFFFFFu, g, __ffs(leads) - 1);
+				leads &= leads - 1u;
+				if ((m >> lane) & 1u) {
+					uint32_t x[6];
+#pragma unroll
+					for (int k = 0; k < 3; ++k)
+						x[k] = __reduce_min_sync(m, v[k]);
+#pragma unroll
+					for (int k = 3; k < 6; ++k)
+						x[k] = __reduce_max_sync(m, v[k]);
+					if (lead) {
+						atomicAdd(&w[6], (uint32_t)__popc(m));
+#pragma unroll
+						for (int k = 0; k < 3; ++k)
+							atomicMin(&w[k], x[k]);
+#pragma unroll
+						for (int k = 3; k < 6; ++k)
+							atomicMax(&w[k], x[k]);
+					}
+				}
+				__syncwarp();
+			}
+		} else if (valid) {
+			if (lead)
+				atomicAdd(&w[6], (uint32_t)__popc(g));
+#pragma unroll
+			for (int k = 0; k < 3; ++k)
+				if (v[k] < *(volatile uint32_t *)&w[k])
+					atomicMin(&w[k], v[k]);
+#pragma unroll
+			for (int k = 3; k < 6; ++k)
+				if (v[k] > *(volatile uint32_t *)&w[k])
+					atomicMax(&w[k], v[k]);
+		}
+	}
+}
+
+// Folds a block's bins of one task into the task's global bins.
+__device__ __forceinline__ void bins_merge(const uint32_t *sb, uint32_t *gbins) {
+	for (int k = threadIdx.x; k < kBinWords; k += blockDim.x) {
+		const int w = k % 7;
+		const uint32_t cnt = sb[k - w + 6];
+		if (cnt == 0)
 			continue;
-		uint32_t *w = b + (a * kBins + bin) * 7;
-		if (lane == __ffs(g) - 1)
-			atomicAdd(&w[6], (uint32_t)__popc(g));
-		const uint32_t v[6] = {f2ord(lo.x), f2ord(lo.y), f2ord(lo.z),
-		                       f2ord(hi.x), f2ord(hi.y), f2ord(hi.z)};
-#pragma unroll
-		for (int k = 0; k < 3; ++k)
-			if (v[k] < *(volatile uint32_t *)&w[k])
-				atomicMin(&w[k], v[k]);
-#pragma unroll
-		for (int k = 3; k < 6; ++k)
-			if (v[k] > *(volatile uint32_t *)&w[k])
-				atomicMax(&w[k], v[k]);
+		if (w < 3)
+			atomicMin(&gbins[k], sb[k]);
+		else if (w < 6)
+			atomicMax(&gbins[k], sb[k]);
+		else
+			atomicAdd(&gbins[k], cnt);
 	}
 }
 
@@ -283,13 +337,13 @@ __device__ __forceinline__ uint32_t new_node(const SahArgs &A, uint32_t k) {
 }
 
 // Files a child range as a task of the right tier (called by one lane).  `frame` gives
-// the binning frame of a large child.  Returns the list slot of a large child, whose
-// bins the calling warp then clears (init_new_bins), else kNone.
-__device__ uint32_t add_child(const SahArgs &A, int out_par, uint32_t begin, uint32_t count,
+// the binning frame of a large child, a task of `level`.  Returns the list slot of a large
+// child, which the calling warp then makes ready (open_large), else kNone.
+__device__ uint32_t add_child(const SahArgs &A, int level, uint32_t begin, uint32_t count,
                               uint32_t node, uint32_t parent, uint32_t buf, uint32_t depth,
                               const Box6 *frame, const float *pflo, const float *pfsc) {
 	if (count > kLarge) {
-		const uint32_t i = atomicAdd(&A.ctr[kCtrLarge + out_par], 1u);
+		const uint32_t i = atomicAdd(&A.ctr[kCtrLarge + level], 1u);
 		if (i >= A.max_large) {
 			flag(A.err);
 			return kNone;
@@ -317,10 +371,10 @@ __device__ uint32_t add_child(const SahArgs &A, int out_par, uint32_t begin, uin
 			}
 		}
 		t.cur_l = t.cur_r = 0;
-		A.large[out_par][i] = t;
+		A.large[level & 1][i] = t;
 		return i;
 	} else if (count > kSmall) {
-		const uint32_t i = atomicAdd(&A.ctr[kCtrMid + out_par], 1u);
+		const uint32_t i = atomicAdd(&A.ctr[kCtrMid], 1u);
 		if (i >= A.max_mid) {
 			flag(A.err);
 			return kNone;
@@ -332,35 +386,45 @@ __device__ uint32_t add_child(const SahArgs &A, int out_par, uint32_t begin, uin
 		t.node = node;
 		t.parent = parent;
 		t.meta = buf | (depth << 8);
-		A.mid[out_par][i] = t;
+		A.mid[i] = t;
 	} else {
 		const uint32_t i = atomicAdd(&A.ctr[kCtrSmall], 1u);
 		if (i >= A.max_small) {
 			flag(A.err);
 			return kNone;
 		}
-		A.small[i] = SmallTask{begin, count | (buf << 8) | (depth << 16), node, parent};
+		A.small[i] = SmallTask{begin, count | (buf << 8) | (depth << 16), node, parent, kNone};
 	}
 	return kNone;
 }
 
-// Clears the bins of the large tasks that lane `from_lane`'s add_child calls filed
-// (their slots); the whole warp calls this, 21 words per lane and task.  A single lane
-// clearing the 672 words of two children took most of k_sah_split's time.
-__device__ __forceinline__ void init_new_bins(const SahArgs &A, int out_par, uint32_t slot_a,
-                                              uint32_t slot_b, int from_lane, int lane) {
-	slot_a = __shfl_sync(0xFFFFFFFFu, slot_a, from_lane);
-	slot_b = __shfl_sync(0xFFFFFFFFu, slot_b, from_lane);
-	if (slot_a != kNone)
-		bins_init(A.bins[out_par] + (size_t)slot_a * kBinWords, lane);
-	if (slot_b != kNone)
-		bins_init(A.bins[out_par] + (size_t)slot_b * kBinWords, lane);
+// Makes a large task filed by lane 0 (its slot and range) ready for its level: the whole warp
+// clears its bins (a single lane clearing the 672 words of two children took most of
+// k_sah_split's time) and lists its chunks.
+__device__ __forceinline__ void open_large(const SahArgs &A, int level, uint32_t slot,
+                                           uint32_t begin, uint32_t count, int lane) {
+	slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
+	if (slot == kNone)
+		return;
+	bins_init(A.bins[level & 1] + (size_t)slot * kBinWords, lane, 32);
+	const uint32_t n = (count + kChunk - 1) / kChunk;
+	uint32_t at = 0;
+	if (lane == 0)
+		at = atomicAdd(&A.ctr[kCtrChunks + level], n);
+	at = __shfl_sync(0xFFFFFFFFu, at, 0);
+	if (at + n > A.max_chunks) {
+		if (lane == 0)
+			flag(A.err);
+		return;
+	}
+	for (uint32_t c = lane; c < n; c += 32)
+		A.chunk[level & 1][at + c] = make_uint2(slot, begin + c * kChunk);
 }
 
 // Writes node `t.node` (box, children, range) for split `s` and files both children
 // (lane 0 only).  Children whose range holds one triangle are leaves.  slots[] receive
 // the list slots of children filed as large tasks (kNone otherwise).
-__device__ void emit_split(const SahArgs &A, const SahTask &t, const Split &s, int out_par,
+__device__ void emit_split(const SahArgs &A, const SahTask &t, const Split &s, int level,
                            const float *flo, const float *fsc, uint32_t slots[2]) {
 	const uint32_t buf = (t.meta & 1u) ^ 1u, depth = ((t.meta >> 8) & 0xFFu) + 1u;
 	const uint32_t nl = s.n_left, nr = t.count - s.n_left;
@@ -401,9 +465,9 @@ __device__ void emit_split(const SahArgs &A, const SahTask &t, const Split &s, i
 	write_node_box(A, t.node, s.node, (binned && nl > 1) ? box_area(s.left) : -1.0f,
 	               (binned && nr > 1) ? box_area(s.right) : -1.0f);
 	const uint32_t pl = binned ? kNone : (t.node << 1), pr = binned ? kNone : ((t.node << 1) | 1u);
-	slots[0] = add_child(A, out_par, t.begin, nl, ids[0], pl, buf, depth,
+	slots[0] = add_child(A, level, t.begin, nl, ids[0], pl, buf, depth,
 	                     binned ? &s.left : nullptr, flo, fsc);
-	slots[1] = add_child(A, out_par, t.begin + nl, nr, ids[1], pr, buf, depth,
+	slots[1] = add_child(A, level, t.begin + nl, nr, ids[1], pr, buf, depth,
 	                     binned ? &s.right : nullptr, flo, fsc);
 }
 
@@ -516,141 +580,57 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uin
 			slot = add_child(A, 0, b, n, n > 1 ? s : kNone, kNone, 0u, 0u, nullptr, flo, fsc);
 		}
 	}
-	init_new_bins(A, 0, slot, kNone, 0, lane);
+	open_large(A, 0, slot, b, n, lane);
 }
 
 // ---------------------------------------------------------------------------------------
 // Large tasks.
 
-// First chunk of each large task of the level and the chunk total; clears the lists
-// the level fills.  One block.
-__global__ void __launch_bounds__(1024) k_sah_chunks(SahArgs A, int par) {
-	__shared__ uint32_t warp_sum[32];
-	__shared__ uint32_t carry;
-	const uint32_t n = n_large(A, par);
-	if (threadIdx.x == 0) {
-		carry = 0;
-		A.ctr[kCtrLarge + (par ^ 1)] = 0;
-		A.ctr[kCtrMid + (par ^ 1)] = 0;
-	}
-	__syncthreads();
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	for (uint32_t base = 0; base < n; base += blockDim.x) {
-		const uint32_t i = base + threadIdx.x;
-		uint32_t c = 0;
-		if (i < n) {
-			const SahTask &t = A.large[par][i];
-			c = range_ok(A, t.begin, t.count) ? (t.count + kChunk - 1) / kChunk : 0u;
-		}
-		uint32_t x = c;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-			if (lane >= o)
-				x += y;
-		}
-		if (lane == 31)
-			warp_sum[w] = x;
-		__syncthreads();
-		if (w == 0) {
-			uint32_t v = lane < (int)(blockDim.x >> 5) ? warp_sum[lane] : 0u;
-#pragma unroll
-			for (int o = 1; o < 32; o <<= 1) {
-				const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
-				if (lane >= o)
-					v += y;
-			}
-			warp_sum[lane] = v;
-		}
-		__syncthreads();
-		const uint32_t before = (w ? warp_sum[w - 1] : 0u) + x - c;
-		if (i < n)
-			A.chunk_off[i] = carry + before;
-		__syncthreads();
-		if (threadIdx.x == 0)
-			carry += warp_sum[(blockDim.x >> 5) - 1];
-		__syncthreads();
-	}
-	if (threadIdx.x == 0) {
-		A.chunk_off[n] = carry;
-		A.ctr[kCtrChunks] = carry;
-	}
-}
-
-__device__ __forceinline__ uint32_t task_of_chunk(const uint32_t *off, uint32_t n, uint32_t c) {
-	uint32_t lo = 0, hi = n; // off[lo] <= c < off[hi]
-	while (hi - lo > 1) {
-		const uint32_t m = (lo + hi) >> 1;
-		if (off[m] <= c)
-			lo = m;
-		else
-			hi = m;
-	}
-	return lo;
-}
-
-__global__ void __launch_bounds__(256) k_sah_bin(SahArgs A, int par) {
+// The roots' bins (the bins of later levels are filled by the partition above them).
+__global__ void __launch_bounds__(256) k_sah_bin(SahArgs A) {
 	__shared__ uint32_t sb[kBinWords];
-	const uint32_t n_tasks = n_large(A, par), n_chunks = A.ctr[kCtrChunks];
+	const uint32_t n = n_chunks(A, 0);
 	const int lane = threadIdx.x & 31;
-	for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-		const uint32_t ti = task_of_chunk(A.chunk_off, n_tasks, c);
-		const SahTask &t = A.large[par][ti];
-		const uint32_t lo_i = t.begin + (c - A.chunk_off[ti]) * kChunk;
-		const uint32_t hi_i = min(lo_i + kChunk, t.begin + t.count);
-		const float4 *src = A.rec[t.meta & 1u];
-		float flo[3], fsc[3];
-		for (int k = 0; k < 3; ++k) {
-			flo[k] = t.lo[k];
-			fsc[k] = t.scale[k];
-		}
-		for (int k = threadIdx.x; k < kBinWords; k += blockDim.x) {
-			const int w = k % 7;
-			sb[k] = w < 3 ? kOrdPosInf : (w < 6 ? kOrdNegInf : 0u);
-		}
-		__syncthreads();
-		for (uint32_t i0 = lo_i + (threadIdx.x & ~31u); i0 < hi_i; i0 += blockDim.x) {
-			const uint32_t i = i0 + lane;
-			const bool v = i < hi_i;
-			float4 lo = make_float4(0, 0, 0, 0), hi = lo;
-			if (v) {
-				lo = src[2 * (size_t)i];
-				hi = src[2 * (size_t)i + 1];
+	for (uint32_t c = blockIdx.x; c < n; c += gridDim.x) {
+		const uint2 ch = A.chunk[0][c];
+		const SahTask &t = A.large[0][ch.x];
+		const uint32_t end = min(ch.y + kChunk, t.begin + t.count);
+		const float4 *src = A.rec[0];
+		float4 lo[kPer], hi[kPer];
+#pragma unroll
+		for (uint32_t j = 0; j < kPer; ++j) {
+			const uint32_t i = ch.y + j * 256u + threadIdx.x;
+			lo[j] = hi[j] = make_float4(0, 0, 0, 0);
+			if (i < end) {
+				lo[j] = src[2 * (size_t)i];
+				hi[j] = src[2 * (size_t)i + 1];
 			}
-			bins_add(sb, v, lo, hi, flo, fsc, lane);
 		}
+		bins_init(sb, threadIdx.x, 256);
 		__syncthreads();
-		uint32_t *gbins = A.bins[par] + (size_t)ti * kBinWords;
-		for (int k = threadIdx.x; k < kBinWords; k += blockDim.x) {
-			const int w = k % 7;
-			const uint32_t cnt = sb[k - w + 6];
-			if (cnt == 0)
-				continue;
-			if (w < 3)
-				atomicMin(&gbins[k], sb[k]);
-			else if (w < 6)
-				atomicMax(&gbins[k], sb[k]);
-			else
-				atomicAdd(&gbins[k], cnt);
-		}
+#pragma unroll
+		for (uint32_t j = 0; j < kPer; ++j)
+			bins_add(sb, ch.y + j * 256u + threadIdx.x < end, 0u, lo[j], hi[j], t.lo, t.scale, lane);
+		__syncthreads();
+		bins_merge(sb, A.bins[0] + (size_t)ch.x * kBinWords);
 		__syncthreads();
 	}
 }
 
 // One warp per large task: the plane, the node and the child tasks.
-__global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int par) {
-	const uint32_t n_tasks = n_large(A, par);
+__global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
+	const uint32_t n_tasks = n_large(A, level);
 	const int lane = threadIdx.x & 31;
 	for (uint32_t ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ti < n_tasks;
 	     ti += (gridDim.x * blockDim.x) >> 5) {
-		SahTask &tr = A.large[par][ti];
+		SahTask &tr = A.large[level & 1][ti];
 		const SahTask t = tr;
 		if (!range_ok(A, t.begin, t.count)) {
 			if (lane == 0)
 				flag(A.err);
 			continue;
 		}
-		const uint32_t *b = A.bins[par] + (size_t)ti * kBinWords;
+		const uint32_t *b = A.bins[level & 1] + (size_t)ti * kBinWords;
 		float flo[3], fsc[3];
 		for (int k = 0; k < 3; ++k) {
 			flo[k] = t.lo[k];
@@ -678,162 +658,334 @@ __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int par) {
 			tr.n_left = s.n_left;
 			tr.cur_l = t.begin;
 			tr.cur_r = t.begin + s.n_left;
-			emit_split(A, t, s, par ^ 1, flo, fsc, slots);
+			emit_split(A, t, s, level + 1, flo, fsc, slots);
 		}
-		init_new_bins(A, par ^ 1, slots[0], slots[1], 0, lane);
+		if (lane == 0) {
+			tr.node = slots[0];
+			tr.parent = slots[1];
+		}
+		open_large(A, level + 1, slots[0], t.begin, s.n_left, lane);
+		open_large(A, level + 1, slots[1], t.begin + s.n_left, t.count - s.n_left, lane);
 	}
 }
 
-// Scatters the triangles of the large tasks to the other buffer, left side first.
-__global__ void __launch_bounds__(256) k_sah_part(SahArgs A, int par) {
-	const uint32_t n_tasks = n_large(A, par), n_chunks = A.ctr[kCtrChunks];
-	const int lane = threadIdx.x & 31;
+// Scatters the triangles of the large tasks to the other buffer, left side first, and adds
+// each to the bins of the child it goes to (when that is a large task).  A thread reads its
+// four triangles at once and the block reserves its places with one atomic per side: the
+// level is bound by the latency of its few dependent steps and by the shared-memory bins.
+// As two kernels, each reading every record, with a pair of atomics per 32 triangles and a
+// chunk table built by a third, a level of the 1,048,576-triangle heightfield took 60 to 90
+// us; now 33 to 64.
+__global__ void __launch_bounds__(256) k_sah_part(SahArgs A, int level) {
+	__shared__ uint32_t sb[2 * kBinWords];
+	__shared__ uint32_t cnt_l[8 * kPer], cnt_r[8 * kPer]; // per warp and j; then exclusive sums
+	__shared__ uint32_t base[2];
+	static_assert(8 * kPer == 32, "one warp scans the block's counts");
+	const uint32_t n = n_chunks(A, level);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const uint32_t lt = (1u << lane) - 1u;
-	for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-		const uint32_t ti = task_of_chunk(A.chunk_off, n_tasks, c);
-		SahTask &t = A.large[par][ti];
+	for (uint32_t c = blockIdx.x; c < n; c += gridDim.x) {
+		const uint2 ch = A.chunk[level & 1][c];
+		SahTask &t = A.large[level & 1][ch.x];
 		const uint32_t begin = t.begin, count = t.count, nl = t.n_left, axis = t.axis,
 		               split = t.split, buf = t.meta & 1u;
-		const uint32_t lo_i = begin + (c - A.chunk_off[ti]) * kChunk;
-		const uint32_t hi_i = min(lo_i + kChunk, begin + count);
+		const uint32_t end = min(ch.y + kChunk, begin + count);
+		const uint32_t slot[2] = {t.node, t.parent};
 		const float4 *src = A.rec[buf];
 		float4 *dst = A.rec[buf ^ 1u];
 		const float flo = axis < 3 ? t.lo[axis] : 0.0f, fsc = axis < 3 ? t.scale[axis] : 0.0f;
-		for (uint32_t i0 = lo_i + (threadIdx.x & ~31u); i0 < hi_i; i0 += blockDim.x) {
-			const uint32_t i = i0 + lane;
-			const bool v = i < hi_i;
-			float4 lo = make_float4(0, 0, 0, 0), hi = lo;
-			bool right = false;
-			if (v) {
-				lo = src[2 * (size_t)i];
-				hi = src[2 * (size_t)i + 1];
-				right = axis == kHalves ? (i - begin >= nl)
-				                        : (bin_of(rec_c(lo, hi, (int)axis), flo, fsc) > (int)split);
+		float4 lo[kPer], hi[kPer];
+		uint32_t side = 0; // bit j: triangle j goes right
+		uint32_t ml[kPer], mr[kPer];
+#pragma unroll
+		for (uint32_t j = 0; j < kPer; ++j) {
+			const uint32_t i = ch.y + j * 256u + threadIdx.x;
+			lo[j] = hi[j] = make_float4(0, 0, 0, 0);
+			if (i < end) {
+				lo[j] = src[2 * (size_t)i];
+				hi[j] = src[2 * (size_t)i + 1];
 			}
-			const uint32_t bl = __ballot_sync(0xFFFFFFFFu, v && !right);
-			const uint32_t br = __ballot_sync(0xFFFFFFFFu, v && right);
-			uint32_t base_l = 0, base_r = 0;
+		}
+		bins_init(sb, threadIdx.x, 256, 2 * kBinWords);
+#pragma unroll
+		for (uint32_t j = 0; j < kPer; ++j) {
+			const uint32_t i = ch.y + j * 256u + threadIdx.x;
+			const bool v = i < end;
+			const bool right =
+			    axis == kHalves ? (i - begin >= nl)
+			                    : (bin_of(rec_c(lo[j], hi[j], (int)axis), flo, fsc) > (int)split);
+			side |= (uint32_t)right << j;
+			ml[j] = __ballot_sync(0xFFFFFFFFu, v && !right);
+			mr[j] = __ballot_sync(0xFFFFFFFFu, v && right);
 			if (lane == 0) {
-				if (bl)
-					base_l = atomicAdd(&t.cur_l, (uint32_t)__popc(bl));
-				if (br)
-					base_r = atomicAdd(&t.cur_r, (uint32_t)__popc(br));
+				cnt_l[warp * kPer + j] = __popc(ml[j]);
+				cnt_r[warp * kPer + j] = __popc(mr[j]);
 			}
-			base_l = __shfl_sync(0xFFFFFFFFu, base_l, 0);
-			base_r = __shfl_sync(0xFFFFFFFFu, base_r, 0);
+		}
+		__syncthreads();
+		if (warp < 2) { // warp 0 the left side, warp 1 the right
+			uint32_t *cnt = warp ? cnt_r : cnt_l;
+			const uint32_t own = cnt[lane];
+			uint32_t x = own;
+#pragma unroll
+			for (int o = 1; o < 32; o <<= 1) {
+				const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+				if (lane >= o)
+					x += y;
+			}
+			cnt[lane] = x - own;
+			if (lane == 31)
+				base[warp] = x ? atomicAdd(warp ? &t.cur_r : &t.cur_l, x) : 0u;
+		}
+		__syncthreads();
+		float clo[2][3], csc[2][3]; // the children's binning frames
+#pragma unroll
+		for (int k = 0; k < 2; ++k) {
+			const SahTask &ct = A.large[(level + 1) & 1][slot[k] == kNone ? 0u : slot[k]];
+#pragma unroll
+			for (int q = 0; q < 3; ++q) {
+				clo[k][q] = slot[k] == kNone ? 0.0f : ct.lo[q];
+				csc[k][q] = slot[k] == kNone ? 0.0f : ct.scale[q];
+			}
+		}
+#pragma unroll
+		for (uint32_t j = 0; j < kPer; ++j) {
+			const bool v = ch.y + j * 256u + threadIdx.x < end;
+			const uint32_t right = (side >> j) & 1u;
 			if (v) {
-				const uint32_t pos = right ? base_r + __popc(br & lt) : base_l + __popc(bl & lt);
+				const uint32_t pos = right ? base[1] + cnt_r[warp * kPer + j] + __popc(mr[j] & lt)
+				                           : base[0] + cnt_l[warp * kPer + j] + __popc(ml[j] & lt);
 				const bool ok = right ? (pos >= begin + nl && pos < begin + count)
 				                      : (pos >= begin && pos < begin + nl);
 				if (ok) {
-					dst[2 * (size_t)pos] = lo;
-					dst[2 * (size_t)pos + 1] = hi;
+					dst[2 * (size_t)pos] = lo[j];
+					dst[2 * (size_t)pos + 1] = hi[j];
 				} else {
 					flag(A.err);
 				}
 			}
+			if (slot[0] != kNone || slot[1] != kNone) {
+				float f[3], g[3];
+#pragma unroll
+				for (int q = 0; q < 3; ++q) {
+					f[q] = right ? clo[1][q] : clo[0][q];
+					g[q] = right ? csc[1][q] : csc[0][q];
+				}
+				bins_add(sb, v && (right ? slot[1] : slot[0]) != kNone, right, lo[j], hi[j], f, g,
+				         lane);
+			}
 		}
+		__syncthreads();
+#pragma unroll
+		for (int k = 0; k < 2; ++k)
+			if (slot[k] != kNone)
+				bins_merge(sb + k * kBinWords,
+				           A.bins[(level + 1) & 1] + (size_t)slot[k] * kBinWords);
+		__syncthreads();
 	}
 }
 
 // ---------------------------------------------------------------------------------------
-// Mid tasks: one warp each, bins in shared memory, stable partition.
+// Mid tasks: one block each.  The task's records stay in shared memory while a permutation
+// of them is split level by level, one warp per range, down to ranges of at most 32, whose
+// records then go to the other buffer in order as small tasks.  (One launch per level, each
+// reading and writing every record, took 0.41 of the 2.17 ms build of the 1,048,576-triangle
+// heightfield, most of it waiting: 20 launches of 3 to 80 us.)  With the large tier's levels
+// halved as well, heightfield builds went from 0.80 to 0.53 ms (65,790 triangles) and 2.17 to
+// 1.81 ms (1,048,576), 8.4M clustered triangles from 15.2 to 14.3 ms, with the same trees.
 
-__global__ void __launch_bounds__(128) k_sah_mid(SahArgs A, int par) {
-	__shared__ uint32_t sb_all[4][kBinWords];
-	const uint32_t n_tasks = n_mid(A, par);
-	const int lane = threadIdx.x & 31;
+struct MidRange {
+	uint32_t begin, count; // within the task
+	uint32_t node, base;   // its node, and the first id for the nodes below it (count - 2)
+	uint32_t parent, depth;
+};
+
+constexpr int kMidWarps = 4;
+constexpr uint32_t kMidRanges = kLarge / (kSmall + 1) + 1;
+
+struct MidShared {
+	float4 rec[2 * kLarge];
+	uint32_t bins[kMidWarps][kBinWords];
+	MidRange range[2][kMidRanges];
+	uint32_t n_range[2];
+	uint32_t base;
+	uint16_t perm[2][kLarge];
+};
+
+// Splits one range (a warp): writes its node and files or queues its two parts.
+__device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, const MidRange &r,
+                                            int in, uint32_t task_begin, float4 *dst,
+                                            uint32_t dst_buf, uint32_t *sb, int lane) {
 	const uint32_t lt = (1u << lane) - 1u;
-	uint32_t *sb = sb_all[threadIdx.x >> 5];
-	for (uint32_t ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ti < n_tasks;
-	     ti += (gridDim.x * blockDim.x) >> 5) {
-		const SahTask t = A.mid[par][ti];
-		if (!range_ok(A, t.begin, t.count) || t.count > kLarge) {
+	const uint16_t *perm = S.perm[in] + r.begin;
+	uint16_t *out = S.perm[in ^ 1] + r.begin;
+	// Exact centre bounds of the range: the binning frame.
+	float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+	for (uint32_t i = lane; i < r.count; i += 32) {
+		const uint32_t p = perm[i];
+		const float4 lo = S.rec[p], hi = S.rec[kLarge + p];
+#pragma unroll
+		for (int k = 0; k < 3; ++k) {
+			const float c = rec_c(lo, hi, k);
+			mn[k] = fminf(mn[k], c);
+			mx[k] = fmaxf(mx[k], c);
+		}
+	}
+	float flo[3], fsc[3];
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		for (int o = 16; o > 0; o >>= 1) {
+			mn[k] = fminf(mn[k], __shfl_xor_sync(0xFFFFFFFFu, mn[k], o));
+			mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xFFFFFFFFu, mx[k], o));
+		}
+		flo[k] = mn[k];
+		fsc[k] = frame_scale(mn[k], mx[k]);
+	}
+	bins_init(sb, lane, 32);
+	__syncwarp();
+	for (uint32_t i0 = 0; i0 < r.count; i0 += 32) {
+		const bool v = i0 + lane < r.count;
+		float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+		if (v) {
+			const uint32_t p = perm[i0 + lane];
+			lo = S.rec[p];
+			hi = S.rec[kLarge + p];
+		}
+		bins_add(sb, v, 0u, lo, hi, flo, fsc, lane);
+	}
+	__syncwarp();
+	Split s = choose_split(sb, fsc, r.count, lane);
+	if (r.depth >= kDepthGuard) {
+		s.axis = kHalves;
+		s.n_left = r.count / 2;
+	}
+	// Stable partition of the permutation.
+	uint32_t nl_seen = 0, nr_seen = 0;
+	for (uint32_t i0 = 0; i0 < r.count; i0 += 32) {
+		const uint32_t i = i0 + lane;
+		const bool v = i < r.count;
+		bool right = false;
+		uint32_t p = 0;
+		if (v) {
+			p = perm[i];
+			right = s.axis == kHalves
+			            ? (i >= s.n_left)
+			            : (bin_of(rec_c(S.rec[p], S.rec[kLarge + p], (int)s.axis), flo[s.axis],
+			                      fsc[s.axis]) > (int)s.bin);
+		}
+		const uint32_t bl = __ballot_sync(0xFFFFFFFFu, v && !right);
+		const uint32_t br = __ballot_sync(0xFFFFFFFFu, v && right);
+		if (v) {
+			const uint32_t pos = right ? s.n_left + nr_seen + __popc(br & lt)
+			                           : nl_seen + __popc(bl & lt);
+			if (pos < r.count)
+				out[pos] = (uint16_t)p;
+		}
+		nl_seen += __popc(bl);
+		nr_seen += __popc(br);
+	}
+	__syncwarp();
+	const uint32_t nl = s.n_left, nr = r.count - nl;
+	if (nl_seen != nl || nl == 0 || nl >= r.count || r.node >= A.node_cap ||
+	    r.base + r.count - 2u > A.node_cap) {
+		if (lane == 0)
+			flag(A.err);
+		return;
+	}
+	const bool binned = s.axis != kHalves;
+	// Ids below the node in order: the left child, its nodes, the right child, its nodes.
+	const uint32_t id_l = r.base, id_r = r.base + nl - 1u;
+	const uint32_t pos_l = task_begin + r.begin, pos_r = pos_l + nl;
+	if (lane == 0) {
+		A.left[r.node] = nl > 1 ? id_l : (kLeafBit | pos_l);
+		A.right[r.node] = nr > 1 ? id_r : (kLeafBit | pos_r);
+		A.rfirst[r.node] = pos_l;
+		A.rlast[r.node] = pos_l + r.count - 1u;
+		if (nl > 1)
+			A.parent_int[id_l] = r.node;
+		else
+			A.parent_leaf[pos_l] = r.node;
+		if (nr > 1)
+			A.parent_int[id_r] = r.node;
+		else
+			A.parent_leaf[pos_r] = r.node;
+		// Children's areas: known now for a binned split (leaves keep -1); after halves each
+		// child writes its own when it is split.
+		write_node_box(A, r.node, s.node, (binned && nl > 1) ? box_area(s.left) : -1.0f,
+		               (binned && nr > 1) ? box_area(s.right) : -1.0f);
+		write_parent_area(A, r.parent, box_area(s.node));
+	}
+#pragma unroll
+	for (int k = 0; k < 2; ++k) {
+		const uint32_t begin = r.begin + (k ? nl : 0u), count = k ? nr : nl;
+		const uint32_t node = count > 1 ? (k ? id_r : id_l) : kNone;
+		const uint32_t parent = binned ? kNone : ((r.node << 1) | (uint32_t)k);
+		if (count > kSmall) {
+			uint32_t at = 0;
 			if (lane == 0)
+				at = atomicAdd(&S.n_range[in ^ 1], 1u);
+			if (lane == 0 && at < kMidRanges)
+				S.range[in ^ 1][at] = MidRange{begin, count, node, node + 1u, parent, r.depth + 1u};
+		} else {
+			if ((uint32_t)lane < count) {
+				const uint32_t p = S.perm[in ^ 1][begin + lane];
+				dst[2 * (size_t)(task_begin + begin + lane)] = S.rec[p];
+				dst[2 * (size_t)(task_begin + begin + lane) + 1] = S.rec[kLarge + p];
+			}
+			if (lane == 0) {
+				const uint32_t i = atomicAdd(&A.ctr[kCtrSmall], 1u);
+				if (i < A.max_small)
+					A.small[i] = SmallTask{task_begin + begin,
+					                       count | (dst_buf << 8) | ((r.depth + 1u) << 16), node,
+					                       parent, count > 2 ? node + 1u : kNone};
+				else
+					flag(A.err);
+			}
+		}
+	}
+}
+
+__global__ void __launch_bounds__(32 * kMidWarps) k_sah_mid(SahArgs A) {
+	__shared__ MidShared S;
+	const uint32_t n_tasks = min(A.ctr[kCtrMid], A.max_mid);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	for (uint32_t ti = blockIdx.x; ti < n_tasks; ti += gridDim.x) {
+		const SahTask t = A.mid[ti];
+		if (!range_ok(A, t.begin, t.count) || t.count > kLarge || t.count <= kSmall) {
+			if (threadIdx.x == 0)
 				flag(A.err);
 			continue;
 		}
 		const uint32_t buf = t.meta & 1u;
 		const float4 *src = A.rec[buf];
-		float4 *dst = A.rec[buf ^ 1u];
-		// Exact centre bounds of the range: the binning frame.
-		float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-		for (uint32_t i = t.begin + lane; i < t.begin + t.count; i += 32) {
-			const float4 lo = src[2 * (size_t)i], hi = src[2 * (size_t)i + 1];
-#pragma unroll
-			for (int k = 0; k < 3; ++k) {
-				const float c = rec_c(lo, hi, k);
-				mn[k] = fminf(mn[k], c);
-				mx[k] = fmaxf(mx[k], c);
+		for (uint32_t i = threadIdx.x; i < t.count; i += 32 * kMidWarps) {
+			S.rec[i] = src[2 * (size_t)(t.begin + i)];
+			S.rec[kLarge + i] = src[2 * (size_t)(t.begin + i) + 1];
+			S.perm[0][i] = (uint16_t)i;
+		}
+		if (threadIdx.x == 0) {
+			const uint32_t base = new_node(A, t.count - 2u);
+			S.range[0][0] = MidRange{0u, t.count, t.node, base, t.parent, (t.meta >> 8) & 0xFFu};
+			S.n_range[0] = base == kNone ? 0u : 1u;
+			S.n_range[1] = 0u;
+		}
+		__syncthreads();
+		for (int level = 0;; ++level) {
+			const int in = level & 1;
+			const uint32_t n = min(S.n_range[in], kMidRanges);
+			if (n == 0u)
+				break;
+			for (uint32_t k = warp; k < n; k += kMidWarps) {
+				const MidRange r = S.range[in][k];
+				split_range(A, S, r, in, t.begin, A.rec[buf ^ 1u], buf ^ 1u, S.bins[warp], lane);
+				__syncwarp();
 			}
+			__syncthreads();
+			if (threadIdx.x == 0)
+				S.n_range[in] = 0u;
+			__syncthreads();
 		}
-		float flo[3], fsc[3];
-#pragma unroll
-		for (int k = 0; k < 3; ++k) {
-			for (int o = 16; o > 0; o >>= 1) {
-				mn[k] = fminf(mn[k], __shfl_xor_sync(0xFFFFFFFFu, mn[k], o));
-				mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xFFFFFFFFu, mx[k], o));
-			}
-			flo[k] = mn[k];
-			fsc[k] = frame_scale(mn[k], mx[k]);
-		}
-		bins_init(sb, lane);
-		__syncwarp();
-		for (uint32_t i0 = t.begin; i0 < t.begin + t.count; i0 += 32) {
-			const uint32_t i = i0 + lane;
-			const bool v = i < t.begin + t.count;
-			float4 lo = make_float4(0, 0, 0, 0), hi = lo;
-			if (v) {
-				lo = src[2 * (size_t)i];
-				hi = src[2 * (size_t)i + 1];
-			}
-			bins_add(sb, v, lo, hi, flo, fsc, lane);
-		}
-		__syncwarp();
-		Split s = choose_split(sb, fsc, t.count, lane);
-		if (((t.meta >> 8) & 0xFFu) >= kDepthGuard) {
-			s.axis = kHalves;
-			s.n_left = t.count / 2;
-		}
-		// Stable partition into the other buffer.
-		uint32_t nl_seen = 0, nr_seen = 0;
-		for (uint32_t i0 = t.begin; i0 < t.begin + t.count; i0 += 32) {
-			const uint32_t i = i0 + lane;
-			const bool v = i < t.begin + t.count;
-			float4 lo = make_float4(0, 0, 0, 0), hi = lo;
-			bool right = false;
-			if (v) {
-				lo = src[2 * (size_t)i];
-				hi = src[2 * (size_t)i + 1];
-				right = s.axis == kHalves
-				            ? (i - t.begin >= s.n_left)
-				            : (bin_of(rec_c(lo, hi, (int)s.axis), flo[s.axis], fsc[s.axis]) >
-				               (int)s.bin);
-			}
-			const uint32_t bl = __ballot_sync(0xFFFFFFFFu, v && !right);
-			const uint32_t br = __ballot_sync(0xFFFFFFFFu, v && right);
-			if (v) {
-				const uint32_t pos = right ? t.begin + s.n_left + nr_seen + __popc(br & lt)
-				                           : t.begin + nl_seen + __popc(bl & lt);
-				const bool ok = right ? (pos < t.begin + t.count) : (pos < t.begin + s.n_left);
-				if (ok) {
-					dst[2 * (size_t)pos] = lo;
-					dst[2 * (size_t)pos + 1] = hi;
-				} else {
-					flag(A.err);
-				}
-			}
-			nl_seen += __popc(bl);
-			nr_seen += __popc(br);
-		}
-		uint32_t slots[2] = {kNone, kNone}; // children of mid tasks are never large
-		if (lane == 0) {
-			if (nl_seen != s.n_left)
-				flag(A.err);
-			write_parent_area(A, t.parent, box_area(s.node));
-			emit_split(A, t, s, par ^ 1, flo, fsc, slots);
-		}
-		__syncwarp();
+		__syncthreads(); // the ranges are read before the next task's overwrite them
 	}
 }
 
@@ -948,10 +1100,12 @@ __global__ void __launch_bounds__(128) k_sah_small(SahArgs A) {
 			__syncwarp();
 		}
 		if (m >= 2) {
-			uint32_t base = 0;
-			if (lane == 0 && m > 2)
-				base = new_node(A, m - 2);
-			base = __shfl_sync(0xFFFFFFFFu, base, 0);
+			uint32_t base = m > 2 ? st.base : 0u;
+			if (m > 2 && base == kNone) {
+				if (lane == 0)
+					base = new_node(A, m - 2);
+				base = __shfl_sync(0xFFFFFFFFu, base, 0);
+			}
 			if (base == kNone || st.node == kNone || st.node >= A.node_cap) {
 				if (lane == 0 && base != kNone)
 					flag(A.err);
@@ -1131,28 +1285,29 @@ __global__ void k_sah_bounds_init(uint32_t *gb, uint32_t n_scenes) {
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
 struct Layout {
-	size_t max_large, max_mid, max_small;
+	size_t max_large, max_mid, max_small, max_chunks;
 	size_t off[12];
 	size_t total;
 };
 
 // Regions of the scratch, 256-byte aligned: records x2, then per parity large tasks,
-// bins and mid tasks, then small tasks, chunk offsets and counters.
+// bins and chunks, then mid tasks, small tasks and counters.
 Layout layout(uint32_t n, uint32_t S) {
 	Layout L;
 	L.max_large = n / (kLarge + 1) + S + 1;
 	L.max_mid = n / (kSmall + 1) + S + 1;
 	L.max_small = (size_t)n + S + 1;
+	L.max_chunks = n / kChunk + L.max_large;
 	const size_t sz[12] = {32ull * n,
 	                       32ull * n,
 	                       64 * L.max_large,
 	                       4ull * kBinWords * L.max_large,
-	                       64 * L.max_mid,
+	                       8 * L.max_chunks,
 	                       64 * L.max_large,
 	                       4ull * kBinWords * L.max_large,
+	                       8 * L.max_chunks,
 	                       64 * L.max_mid,
-	                       16 * L.max_small,
-	                       4 * (L.max_large + 1),
+	                       sizeof(SmallTask) * L.max_small,
 	                       4 * kCtrWordsSah,
 	                       0};
 	size_t at = 0;
@@ -1184,10 +1339,10 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	for (int k = 0; k < 2; ++k) {
 		A.large[k] = reinterpret_cast<SahTask *>(p + L.off[2 + 3 * k]);
 		A.bins[k] = reinterpret_cast<uint32_t *>(p + L.off[3 + 3 * k]);
-		A.mid[k] = reinterpret_cast<SahTask *>(p + L.off[4 + 3 * k]);
+		A.chunk[k] = reinterpret_cast<uint2 *>(p + L.off[4 + 3 * k]);
 	}
-	A.small = reinterpret_cast<SmallTask *>(p + L.off[8]);
-	A.chunk_off = reinterpret_cast<uint32_t *>(p + L.off[9]);
+	A.mid = reinterpret_cast<SahTask *>(p + L.off[8]);
+	A.small = reinterpret_cast<SmallTask *>(p + L.off[9]);
 	A.ctr = reinterpret_cast<uint32_t *>(p + L.off[10]);
 	A.vals = ws.vals.as<uint32_t>();
 	A.lbox = ws.lbox.as<float4>();
@@ -1202,6 +1357,7 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	A.max_large = (uint32_t)L.max_large;
 	A.max_mid = (uint32_t)L.max_mid;
 	A.max_small = (uint32_t)L.max_small;
+	A.max_chunks = (uint32_t)L.max_chunks;
 	A.n = n;
 	A.err = d_err;
 
@@ -1216,67 +1372,48 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	k_sah_first_id<<<1, 1, 0, st>>>(A.ctr, S);
 	k_sah_roots<<<blocks_for(32ull * S, 128), 128, 0, st>>>(A, d_toff, S, gb,
 	                                                        ws.roots.as<uint32_t>());
-	int level = 0;
-	bool large_left = true; // children are smaller than their parent: once no large task
-	                        // is left, none comes back, and its four kernels are skipped
-	// Before the first look at the level counters (a host wait each): as many levels as
-	// halving splits need to bring the largest scene under the large-task size, since a
-	// split leaves at least one triangle on each side and most leave about half.
-	// For scenes of at most 64 Ki triangles the mid levels too (down to the small-task
-	// size): their empty large-tier launches cost less than the wait they save.
-	int ahead = 1;
-	{
-		uint32_t biggest = 0;
-		for (uint32_t sc = 0; sc < S; ++sc)
-			biggest = std::max(biggest, plan.toff[sc + 1] - plan.toff[sc]);
-		const uint32_t floor = biggest <= 65536u ? kSmall : kLarge;
-		for (uint64_t c = biggest; c > floor; c = (c + 1) / 2)
-			++ahead;
-		ahead = std::max(ahead, kLevelsPerCheck);
+	// Before the first look at the level counters (a host wait): as many levels as halving
+	// splits need to bring the largest scene under the large-task size, since a split
+	// leaves at least one triangle on each side and most leave about half.
+	uint32_t biggest = 0;
+	for (uint32_t sc = 0; sc < S; ++sc)
+		biggest = std::max(biggest, plan.toff[sc + 1] - plan.toff[sc]);
+	int ahead = 0;
+	for (uint64_t c = biggest; c > kLarge; c = (c + 1) / 2)
+		++ahead;
+	if (ahead) {
+		k_sah_bin<<<(unsigned)std::min<size_t>(1216, L.max_chunks), 256, 0, st>>>(A);
+		ahead += 2;
 	}
-	for (;;) {
+	for (int level = 0; ahead;) {
 		for (int k = 0; k < ahead && level < kMaxLevels; ++k, ++level) {
-			const int par = level & 1;
 			// Grids no larger than the work the level can hold: each task has at most two
-			// children, so level L has at most S * 2^L tasks of a tier (a small scene's
-			// levels are then a few blocks each instead of 1216 idle ones).
-			const uint64_t tasks = (uint64_t)S << std::min(level, 40);
-			const unsigned g_chunk =
-			    (unsigned)std::min<uint64_t>(1216, n / kChunk + std::min<uint64_t>(tasks, L.max_large));
-			const unsigned g_split = (unsigned)std::min<uint64_t>(152, (tasks + 3) / 4);
-			const unsigned g_mid =
-			    (unsigned)std::min<uint64_t>(1216, (std::min<uint64_t>(tasks, L.max_mid) + 3) / 4);
-			if (large_left) {
-				k_sah_chunks<<<1, 1024, 0, st>>>(A, par);
-				k_sah_bin<<<g_chunk, 256, 0, st>>>(A, par);
-				k_sah_split<<<g_split, 128, 0, st>>>(A, par);
-				k_sah_part<<<g_chunk, 256, 0, st>>>(A, par);
-			} else {
-				// What k_sah_chunks does besides: clear the lists this level fills.
-				cudaMemsetAsync(A.ctr + kCtrLarge + (par ^ 1), 0, 4, st);
-				cudaMemsetAsync(A.ctr + kCtrMid + (par ^ 1), 0, 4, st);
-			}
-			k_sah_mid<<<g_mid, 128, 0, st>>>(A, par);
+			// children, so level L has at most S * 2^L tasks (a small scene's levels are then
+			// a few blocks each instead of 1216 idle ones).
+			const uint64_t tasks = std::min<uint64_t>((uint64_t)S << std::min(level, 30), L.max_large);
+			const unsigned g_chunk = (unsigned)std::min<uint64_t>(1216, n / kChunk + tasks);
+			const unsigned g_split = (unsigned)std::min<uint64_t>(304, (tasks + 3) / 4);
+			k_sah_split<<<g_split, 128, 0, st>>>(A, level);
+			k_sah_part<<<g_chunk, 256, 0, st>>>(A, level);
 		}
 		uint32_t *h = ws.h_sah;
-		cudaError_t e = cudaMemcpyAsync(h, A.ctr, 4 * kCtrWordsSah, cudaMemcpyDeviceToHost, st);
+		cudaError_t e =
+		    cudaMemcpyAsync(h, A.ctr + kCtrLarge + level, 4, cudaMemcpyDeviceToHost, st);
 		if (e == cudaSuccess)
 			e = cudaStreamSynchronize(st);
 		if (e != cudaSuccess) {
 			msg = std::string("sah build: ") + cudaGetErrorString(e);
 			return PRT_ERR_CUDA;
 		}
-		const int par = level & 1;
-		if (h[kCtrLarge + par] == 0 && h[kCtrMid + par] == 0)
+		if (h[0] == 0)
 			break;
-		if (h[kCtrLarge + par] == 0)
-			large_left = false;
 		if (level >= kMaxLevels) {
 			msg = "sah build: more than " + std::to_string(kMaxLevels) + " levels";
 			return PRT_ERR_LIMIT;
 		}
 		ahead = kLevelsPerCheck;
 	}
+	k_sah_mid<<<(unsigned)std::min<size_t>(1216, L.max_mid), 32 * kMidWarps, 0, st>>>(A);
 	k_sah_small<<<2432, 128, 0, st>>>(A);
 	// Every node id handed out must have been written before the collapse follows the
 	// children: check the error word and the node count first.
@@ -1285,8 +1422,8 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 		const uint32_t ns = plan.toff[s + 1] - plan.toff[s];
 		want += ns >= 2 ? ns - 2 : 0;
 	}
-	uint32_t *h = ws.h_sah, *h_errw = h + kCtrWordsSah;
-	cudaError_t e = cudaMemcpyAsync(h, A.ctr, 4 * kCtrWordsSah, cudaMemcpyDeviceToHost, st);
+	uint32_t *h = ws.h_sah, *h_errw = h + 4;
+	cudaError_t e = cudaMemcpyAsync(h, A.ctr, 16, cudaMemcpyDeviceToHost, st);
 	if (e == cudaSuccess)
 		e = cudaMemcpyAsync(h_errw, d_err, 4, cudaMemcpyDeviceToHost, st);
 	if (e == cudaSuccess)
