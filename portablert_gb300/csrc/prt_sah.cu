@@ -156,10 +156,14 @@ __device__ __forceinline__ void bins_add(uint32_t *b, bool valid, uint32_t set, 
                                          int lane) {
 	const uint32_t v[6] = {f2ord(lo.x), f2ord(lo.y), f2ord(lo.z),
 	                       f2ord(hi.x), f2ord(hi.y), f2ord(hi.z)};
+	int bins[3] = {-1, -1, -1};
+	if (valid)
+#pragma unroll
+		for (int a = 0; a < 3; ++a)
+			bins[a] = ((int)set * 3 + a) * kBins + bin_of(rec_c(lo, hi, a), flo[a], fsc[a]);
 #pragma unroll
 	for (int a = 0; a < 3; ++a) {
-		const int bin =
-		    valid ? (int)set * 3 * kBins + a * kBins + bin_of(rec_c(lo, hi, a), flo[a], fsc[a]) : -1;
+		const int bin = bins[a];
 		const uint32_t g = __match_any_sync(0xFFFFFFFFu, bin);
 		const bool lead = valid && lane == __ffs(g) - 1;
 		uint32_t leads = __ballot_sync(0xFFFFFFFFu, lead);
@@ -788,7 +792,9 @@ __global__ void __launch_bounds__(256) k_sah_part(SahArgs A, int level) {
 // ---------------------------------------------------------------------------------------
 // Mid tasks: one block each.  The task's records stay in shared memory while a permutation
 // of them is split level by level, one warp per range, down to ranges of at most 32, whose
-// records then go to the other buffer in order as small tasks.  (One launch per level, each
+// records then go to the other buffer in order as small tasks.  The first range is split by
+// all four warps and the next two by two each: with one warp each, three waited 42 % of the
+// kernel's time for the others (8.4M clustered triangles 14.3 -> 13.4 ms).  (One launch per level, each
 // reading and writing every record, took 0.41 of the 2.17 ms build of the 1,048,576-triangle
 // heightfield, most of it waiting: 20 launches of 3 to 80 us.)  With the large tier's levels
 // halved as well, heightfield builds went from 0.80 to 0.53 ms (65,790 triangles) and 2.17 to
@@ -800,7 +806,7 @@ struct MidRange {
 	uint32_t parent, depth;
 };
 
-constexpr int kMidWarps = 4;
+constexpr int kMidWarps = 4; // (teams of 4, 2 and 1 warps)
 constexpr uint32_t kMidRanges = kLarge / (kSmall + 1) + 1;
 
 struct MidShared {
@@ -808,20 +814,36 @@ struct MidShared {
 	uint32_t bins[kMidWarps][kBinWords];
 	MidRange range[2][kMidRanges];
 	uint32_t n_range[2];
-	uint32_t base;
+	float bound[kMidWarps][6];
+	uint32_t choice[kMidWarps][3], left_of[kMidWarps], total[kMidWarps];
 	uint16_t perm[2][kLarge];
 };
 
-// Splits one range (a warp): writes its node and files or queues its two parts.
+// A barrier of the `team` warps that split one range (the block's warps in order, so teams
+// of equal size are numbered by their first warp).
+__device__ __forceinline__ void team_sync(int team, int warp) {
+	if (team == 1)
+		__syncwarp();
+	else
+		asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / team), "r"(32 * team) : "memory");
+}
+
+// Splits one range with a team of 1, 2 or 4 warps: writes its node and files or queues its
+// two parts.  Each warp takes a slice of the range; the first chooses the split.
 __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, const MidRange &r,
                                             int in, uint32_t task_begin, float4 *dst,
-                                            uint32_t dst_buf, uint32_t *sb, int lane) {
+                                            uint32_t dst_buf, int team, int warp, int lane) {
 	const uint32_t lt = (1u << lane) - 1u;
+	const int lead = warp - warp % team;
 	const uint16_t *perm = S.perm[in] + r.begin;
 	uint16_t *out = S.perm[in ^ 1] + r.begin;
+	uint32_t *sb = S.bins[lead];
+	const uint32_t slice = (r.count + 32u * team - 1u) / (32u * team) * 32u;
+	const uint32_t i_lo = min(slice * (uint32_t)(warp - lead), r.count);
+	const uint32_t i_hi = min(i_lo + slice, r.count);
 	// Exact centre bounds of the range: the binning frame.
 	float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-	for (uint32_t i = lane; i < r.count; i += 32) {
+	for (uint32_t i = i_lo + lane; i < i_hi; i += 32) {
 		const uint32_t p = perm[i];
 		const float4 lo = S.rec[p], hi = S.rec[kLarge + p];
 #pragma unroll
@@ -833,18 +855,34 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 	}
 	float flo[3], fsc[3];
 #pragma unroll
-	for (int k = 0; k < 3; ++k) {
+	for (int k = 0; k < 3; ++k)
 		for (int o = 16; o > 0; o >>= 1) {
 			mn[k] = fminf(mn[k], __shfl_xor_sync(0xFFFFFFFFu, mn[k], o));
 			mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xFFFFFFFFu, mx[k], o));
 		}
+	bins_init(sb, 32 * (warp - lead) + lane, 32 * team);
+	if (team > 1) {
+		if (lane == 0)
+			for (int k = 0; k < 3; ++k) {
+				S.bound[warp][k] = mn[k];
+				S.bound[warp][3 + k] = mx[k];
+			}
+		team_sync(team, warp);
+		for (int w = lead; w < lead + team; ++w)
+#pragma unroll
+			for (int k = 0; k < 3; ++k) {
+				mn[k] = fminf(mn[k], S.bound[w][k]);
+				mx[k] = fmaxf(mx[k], S.bound[w][3 + k]);
+			}
+	}
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
 		flo[k] = mn[k];
 		fsc[k] = frame_scale(mn[k], mx[k]);
 	}
-	bins_init(sb, lane, 32);
 	__syncwarp();
-	for (uint32_t i0 = 0; i0 < r.count; i0 += 32) {
-		const bool v = i0 + lane < r.count;
+	for (uint32_t i0 = i_lo; i0 < i_hi; i0 += 32) {
+		const bool v = i0 + lane < i_hi;
 		float4 lo = make_float4(0, 0, 0, 0), hi = lo;
 		if (v) {
 			const uint32_t p = perm[i0 + lane];
@@ -853,26 +891,56 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 		}
 		bins_add(sb, v, 0u, lo, hi, flo, fsc, lane);
 	}
-	__syncwarp();
-	Split s = choose_split(sb, fsc, r.count, lane);
-	if (r.depth >= kDepthGuard) {
-		s.axis = kHalves;
-		s.n_left = r.count / 2;
-	}
-	// Stable partition of the permutation.
-	uint32_t nl_seen = 0, nr_seen = 0;
-	for (uint32_t i0 = 0; i0 < r.count; i0 += 32) {
-		const uint32_t i = i0 + lane;
-		const bool v = i < r.count;
-		bool right = false;
-		uint32_t p = 0;
-		if (v) {
-			p = perm[i];
-			right = s.axis == kHalves
-			            ? (i >= s.n_left)
-			            : (bin_of(rec_c(S.rec[p], S.rec[kLarge + p], (int)s.axis), flo[s.axis],
-			                      fsc[s.axis]) > (int)s.bin);
+	team_sync(team, warp);
+	Split s;
+	if (warp == lead) {
+		s = choose_split(sb, fsc, r.count, lane);
+		if (r.depth >= kDepthGuard) {
+			s.axis = kHalves;
+			s.n_left = r.count / 2;
 		}
+		if (team > 1 && lane == 0) {
+			S.choice[lead][0] = s.axis;
+			S.choice[lead][1] = s.bin;
+			S.choice[lead][2] = s.n_left;
+		}
+	}
+	if (team > 1) {
+		team_sync(team, warp);
+		if (warp != lead) {
+			s.axis = S.choice[lead][0];
+			s.bin = S.choice[lead][1];
+			s.n_left = S.choice[lead][2];
+		}
+	}
+	// Stable partition of the permutation: each warp counts its slice's left part first when
+	// the slices have to be placed after one another.
+	auto goes_right = [&](uint32_t i, uint32_t p) {
+		return s.axis == kHalves
+		           ? (i >= s.n_left)
+		           : (bin_of(rec_c(S.rec[p], S.rec[kLarge + p], (int)s.axis),
+		                     s.axis == 0 ? flo[0] : (s.axis == 1 ? flo[1] : flo[2]),
+		                     s.axis == 0 ? fsc[0] : (s.axis == 1 ? fsc[1] : fsc[2])) > (int)s.bin);
+	};
+	uint32_t nl_seen = 0, nr_seen = 0;
+	if (team > 1) {
+		uint32_t mine = 0;
+		for (uint32_t i0 = i_lo; i0 < i_hi; i0 += 32) {
+			const uint32_t i = i0 + lane;
+			mine += __popc(__ballot_sync(0xFFFFFFFFu, i < i_hi && !goes_right(i, perm[min(i, i_hi - 1u)])));
+		}
+		if (lane == 0)
+			S.left_of[warp] = mine;
+		team_sync(team, warp);
+		for (int w = lead; w < warp; ++w)
+			nl_seen += S.left_of[w];
+		nr_seen = i_lo - nl_seen;
+	}
+	for (uint32_t i0 = i_lo; i0 < i_hi; i0 += 32) {
+		const uint32_t i = i0 + lane;
+		const bool v = i < i_hi;
+		const uint32_t p = perm[min(i, i_hi - 1u)];
+		const bool right = goes_right(i, p);
 		const uint32_t bl = __ballot_sync(0xFFFFFFFFu, v && !right);
 		const uint32_t br = __ballot_sync(0xFFFFFFFFu, v && right);
 		if (v) {
@@ -883,6 +951,14 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 		}
 		nl_seen += __popc(bl);
 		nr_seen += __popc(br);
+	}
+	if (team > 1) {
+		if (warp == lead + team - 1 && lane == 0)
+			S.total[lead] = nl_seen; // (its own word: left_of may still be read)
+		team_sync(team, warp);
+		if (warp != lead)
+			return;
+		nl_seen = S.total[lead];
 	}
 	__syncwarp();
 	const uint32_t nl = s.n_left, nr = r.count - nl;
@@ -975,9 +1051,11 @@ __global__ void __launch_bounds__(32 * kMidWarps) k_sah_mid(SahArgs A) {
 			const uint32_t n = min(S.n_range[in], kMidRanges);
 			if (n == 0u)
 				break;
-			for (uint32_t k = warp; k < n; k += kMidWarps) {
+			// One range: all four warps split it; two: two each; more: one warp each.
+			const int team = n == 1u ? 4 : (n == 2u ? 2 : 1);
+			for (uint32_t k = warp / team; k < n; k += kMidWarps / team) {
 				const MidRange r = S.range[in][k];
-				split_range(A, S, r, in, t.begin, A.rec[buf ^ 1u], buf ^ 1u, S.bins[warp], lane);
+				split_range(A, S, r, in, t.begin, A.rec[buf ^ 1u], buf ^ 1u, team, warp, lane);
 				__syncwarp();
 			}
 			__syncthreads();
