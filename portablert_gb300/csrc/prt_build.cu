@@ -14,9 +14,10 @@
 //   2. 30-bit Morton codes        (k_morton; 10 bits per axis, centroids normalised)
 //   3. onesweep radix sort        (prt_sort.cu; 4 digit passes, +1 or 2 for the scene)
 //   4. Karras hierarchy           (k_karras; Karras 2012 within each scene's range)
-//   5. bottom-up refit            (k_leaf_boxes + k_refit; atomic arrival counters)
-//   6. collapse to 8-wide nodes   (k_collapse_cost: bottom-up least expected cost per
-//                                  ray, which subtrees become nodes and which leaves;
+//   5. bottom-up pass             (k_bottom_up: boxes and, for the collapse, the least
+//                                  expected cost per ray: which subtrees become nodes and
+//                                  which leaves)
+//   6. collapse to 8-wide nodes   (after step 5's costs, which SAH builds compute as well;
 //                                  then k_collapse, one launch per level, per-level
 //                                  counters, so the host checks progress every few levels;
 //                                  with each node its optional 8-bit encoding, outward-
@@ -54,7 +55,7 @@ bool alloc_failure_due() {
 
 void BuildScratch::release() {
 	DevBuf *all[] = {&keys,        &vals,     &keys2,      &vals2,    &scene_of,   &int_off,
-	                 &left,        &right,    &parent_int, &parent_leaf, &rfirst,  &rlast,
+	                 &left,        &right,    &splits,     &rfirst,   &rlast,
 	                 &ibox,        &lbox,     &flags,      &items_a,  &items_b,    &counters,
 	                 &sort_hist, &sort_tiles, &sort_status, &bounds,
 	                 &sah,         &roots,    &cost};
@@ -96,10 +97,15 @@ __global__ void k_scene_of(const uint32_t *tri_off, uint32_t n_scenes, uint32_t 
 			scene_of[i] = s;
 }
 
-__global__ void k_bounds_init(uint32_t *gb, uint32_t n_scenes) {
+// Empty bounds, and no split after each scene's last leaf.
+__global__ void k_bounds_init(uint32_t *gb, uint32_t n_scenes, const uint32_t *tri_off,
+                              uint4 *splits) {
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 * n_scenes;
-	     i += gridDim.x * blockDim.x)
+	     i += gridDim.x * blockDim.x) {
 		gb[i] = (i % 6) < 3 ? 0xFFFFFFFFu : 0u;
+		if (i < n_scenes && tri_off[i + 1] > tri_off[i])
+			splits[tri_off[i + 1] - 1u] = PRT_NO_SPLIT;
+	}
 }
 
 // Per-scene centroid bounds as ordered words: a warp whose triangles all belong to one
@@ -249,8 +255,8 @@ __device__ __forceinline__ int kdelta(const K *__restrict__ k, int n, int i, int
 template <typename K>
 __global__ void k_karras(const K *__restrict__ keys, uint32_t n_int, const uint32_t *tri_off,
                          const uint32_t *int_off, uint32_t n_scenes, uint32_t *left,
-                         uint32_t *right, uint32_t *parent_int, uint32_t *parent_leaf,
-                         uint32_t *rfirst, uint32_t *rlast) {
+                         uint32_t *right, uint4 *splits, uint32_t *rfirst,
+                         uint32_t *rlast) {
 	const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
 	if (gi >= n_int)
 		return;
@@ -293,38 +299,9 @@ __global__ void k_karras(const K *__restrict__ keys, uint32_t n_int, const uint3
 	const uint32_t rc = rleaf ? (kLeafBit | (first + gamma + 1)) : (ibase + gamma + 1);
 	left[gi] = lc;
 	right[gi] = rc;
-	if (lleaf)
-		parent_leaf[first + gamma] = gi;
-	else
-		parent_int[ibase + gamma] = gi;
-	if (rleaf)
-		parent_leaf[first + gamma + 1] = gi;
-	else
-		parent_int[ibase + gamma + 1] = gi;
+	splits[first + gamma] = make_uint4(first + lo, first + hi, gi, 0u);
 	rfirst[gi] = first + lo;
 	rlast[gi] = first + hi;
-	if (i == 0)
-		parent_int[gi] = kNone;
-}
-
-__global__ void k_leaf_boxes(const float *__restrict__ tris, const uint32_t *__restrict__ vals,
-                             uint32_t n, float4 *lbox) {
-	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n)
-		return;
-	const float *t = tris + 9 * (size_t)vals[i];
-	float4 lo, hi;
-	if (tri_finite(t)) {
-		lo = make_float4(fminf(t[0], fminf(t[3], t[6])), fminf(t[1], fminf(t[4], t[7])),
-		                 fminf(t[2], fminf(t[5], t[8])), 0.0f);
-		hi = make_float4(fmaxf(t[0], fmaxf(t[3], t[6])), fmaxf(t[1], fmaxf(t[4], t[7])),
-		                 fmaxf(t[2], fmaxf(t[5], t[8])), 0.0f);
-	} else {
-		lo = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
-		hi = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
-	}
-	lbox[2 * i] = lo;
-	lbox[2 * i + 1] = hi;
 }
 
 // atomicAdd(p, 1) with acquire-release ordering at device scope.
@@ -343,45 +320,6 @@ __device__ __forceinline__ void child_box(uint32_t ref, const float4 *ibox, cons
 	} else {
 		lo = __ldcg(&ibox[2 * ref]);
 		hi = __ldcg(&ibox[2 * ref + 1]);
-	}
-}
-
-// One thread per leaf walks towards its scene's root; at each binary node the first
-// thread to arrive stops and the second, which then sees both children's boxes, writes
-// the union and continues.  No thread waits on another.  A scene of one triangle has
-// no binary node (parent_leaf stays kNone).  The unused w slots of a node's box carry
-// the surface areas of its two children (-1 for a leaf child), which the collapse
-// reads together with the child indices when it opens the node.
-__global__ void k_refit(uint32_t n, uint32_t n_int, const uint32_t *__restrict__ parent_leaf,
-                        const uint32_t *__restrict__ parent_int, const uint32_t *__restrict__ left,
-                        const uint32_t *__restrict__ right, const float4 *lbox, float4 *ibox,
-                        uint32_t *flags, uint32_t *err) {
-	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n)
-		return;
-	uint32_t p = parent_leaf[i];
-	// A path to the root passes each binary node once; a longer walk (or an index out
-	// of range) means corrupt parents, reported instead of followed.
-	for (uint32_t steps = 0; p != kNone; ++steps) {
-		if (p >= n_int || steps >= n_int) {
-			atomicOr(err, kErrCollapse);
-			return;
-		}
-		// Release: the union this thread wrote one level down is visible before its
-		// arrival counts.  Acquire: the sibling's union is read after its arrival.
-		if (arrive_acq_rel(&flags[p]) == 0u)
-			return;
-		float4 alo, ahi, blo, bhi;
-		const uint32_t l = left[p], r = right[p];
-		child_box(l, ibox, lbox, alo, ahi);
-		child_box(r, ibox, lbox, blo, bhi);
-		const float al = (l & kLeafBit) ? -1.0f : half_area(alo, ahi);
-		const float ar = (r & kLeafBit) ? -1.0f : half_area(blo, bhi);
-		__stcg(&ibox[2 * p], make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y),
-		                                 fminf(alo.z, blo.z), al));
-		__stcg(&ibox[2 * p + 1], make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y),
-		                                     fmaxf(ahi.z, bhi.z), ar));
-		p = parent_int[p];
 	}
 }
 
@@ -404,38 +342,282 @@ __device__ __forceinline__ float3 child_costs(uint32_t y, const CostNode *cost,
 	return half_extent(__ldcg(&ibox[2 * y]), __ldcg(&ibox[2 * y + 1]));
 }
 
-// One thread per leaf walks towards the root like k_refit; the second thread to arrive
-// at a binary node computes its costs from both children's.
-__global__ void k_collapse_cost(uint32_t n, uint32_t n_ids, const uint32_t *__restrict__ parent_leaf,
-                                const uint32_t *__restrict__ parent_int,
-                                const uint32_t *__restrict__ left, const uint32_t *__restrict__ right,
-                                const uint32_t *__restrict__ rfirst,
-                                const uint32_t *__restrict__ rlast, const float4 *__restrict__ ibox,
-                                const float4 *__restrict__ lbox, uint32_t *flags, CostNode *cost,
-                                uint32_t leaf_size, uint32_t *err) {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n)
-		return;
-	uint32_t p = parent_leaf[i];
-	for (uint32_t steps = 0; p != kNone; ++steps) {
-		if (p >= n_ids || steps >= n_ids) {
-			atomicOr(err, kErrCollapse);
-			return;
+struct UpArgs {
+	const float *tris;        // REFIT: the triangles, by vals
+	const uint32_t *vals;
+	uint32_t n, n_ids;
+	const uint4 *splits;
+	const uint32_t *left, *right;
+	float4 *ibox, *lbox;
+	uint32_t *flags;          // arrivals at nodes that several blocks' leaves reach
+	CostNode *cost;
+	uint32_t leaf_size;
+	uint32_t *walks, *n_walks; // slots at which the blocks' parts end
+	uint32_t walk_cap;
+	uint32_t *err;
+};
+
+constexpr uint32_t kUpLeaves = 256; // leaf positions per block
+
+// What a block knows of the subtrees inside its leaf positions.  The binary node that splits
+// after a leaf position has that position as its slot: every node has one, every position but
+// a scene's last, and the parent of the subtree over leaves [f, l] is the node of slot l (it
+// is its left child) or of slot f - 1 (its right child).
+struct UpShared {
+	uint32_t first[kUpLeaves], last[kUpLeaves], node[kUpLeaves]; // `splits` of the positions
+	float lbox[6][kUpLeaves];  // boxes of the leaves ...
+	float nbox[6][kUpLeaves];  // ... and of the nodes, by slot
+	float cost[8][kUpLeaves];  // c1 and cd of the nodes done
+	uint32_t count[kUpLeaves]; // children done
+	uint32_t n_ready[kUpLeaves + 2]; // nodes that became ready for round k
+	uint32_t escape[kUpLeaves], n_escape; // slots (global) that the block's part ends at
+	uint32_t walk_at;
+	uint16_t child[2][kUpLeaves]; // children done: leaf position | kUpLeaf, or slot
+	uint16_t ready[2][kUpLeaves];
+};
+constexpr uint16_t kUpLeaf = 0x8000u;
+
+// A subtree (leaf position or slot `ref`, global leaf range [f, l]) is done: its parent gets
+// it.  Round `round` takes up the parents that are complete then.
+__device__ __forceinline__ void up_deliver(const UpArgs &A, UpShared &S, uint32_t b0,
+                                           uint16_t ref, uint32_t f, uint32_t l,
+                                           uint32_t round) {
+	const bool is_left = S.first[l - b0] == f;
+	if (!is_left && f == b0) {
+		if (f > 0u && __ldg(&A.splits[f - 1u]).y == l) {
+			const uint32_t at = atomicAdd(&S.n_escape, 1u);
+			if (at < kUpLeaves)
+				S.escape[at] = f - 1u;
 		}
-		if (arrive_acq_rel(&flags[p]) == 0u)
-			return;
-		float cl[8], cr[8];
-		const float3 el = child_costs(left[p], cost, ibox, lbox, cl);
-		const float3 er = child_costs(right[p], cost, ibox, lbox, cr);
-		const float3 ep = half_extent(__ldcg(&ibox[2 * p]), __ldcg(&ibox[2 * p + 1]));
-		const CostNode c =
-		    merge_costs(cl, cr, el, er, ep, rlast[p] - rfirst[p] + 1u, leaf_size);
-		__stcg(&cost[p].c1, c.c1);
+		return; // (or a root)
+	}
+	const uint32_t slot = is_left ? l - b0 : f - 1u - b0;
+	if (!is_left && S.last[slot] != l)
+		return; // a root
+	if (S.first[slot] < b0 || S.last[slot] >= b0 + kUpLeaves) {
+		const uint32_t at = atomicAdd(&S.n_escape, 1u);
+		if (at < kUpLeaves)
+			S.escape[at] = b0 + slot;
+		return;
+	}
+	S.child[is_left ? 0 : 1][slot] = ref;
+	if (atomicAdd(&S.count[slot], 1u) == 1u) {
+		const uint32_t at = atomicAdd(&S.n_ready[round], 1u);
+		if (at < kUpLeaves)
+			S.ready[round & 1u][at] = (uint16_t)slot;
+	}
+}
+
+__device__ __forceinline__ void up_child(const UpShared &S, uint16_t ref, float4 &lo, float4 &hi,
+                                         float cs[8], bool cost) {
+	const bool leaf = (ref & kUpLeaf) != 0;
+	const uint32_t at = ref & (kUpLeaves - 1u);
+	const float(*b)[kUpLeaves] = leaf ? S.lbox : S.nbox;
+	lo = make_float4(b[0][at], b[1][at], b[2][at], 0.0f);
+	hi = make_float4(b[3][at], b[4][at], b[5][at], 0.0f);
+	if (!cost)
+		return;
+	if (leaf) {
+		leaf_costs(cs);
+	} else {
+		CostNode c;
+		c.c1 = S.cost[0][at];
 #pragma unroll
-		for (int k = 0; k < 7; ++k)
-			__stcg(&cost[p].cd[k], c.cd[k]);
-		__stcg(&cost[p].bits, c.bits);
-		p = parent_int[p];
+		for (int j = 0; j < 7; ++j)
+			c.cd[j] = S.cost[1 + j][at];
+		node_costs(c, cs);
+	}
+}
+
+// The bottom-up pass over the binary trees.  REFIT: boxes of the leaves (from the triangles in
+// sorted order) and of the nodes, whose unused w words carry the surface areas of their two
+// children (-1 for a leaf child), which the collapse by area reads together with the child
+// indices.  COST: the least expected costs of each node (CostNode).
+//
+// A block takes 256 consecutive leaves and finishes every node whose leaves are all among
+// them from shared memory, round by round, full warps on the nodes that became complete in
+// the round before; the subtrees it ends with go to k_walk_up.  With one thread per leaf
+// walking all the way, refit and costs apart, 5 of 32 lanes were active and every step was
+// an acquire-release atomic and two dependent reads through L2: leaf boxes, refit and costs
+// of a batch of 4.6M triangles took 110 + 252 + 694 us, the costs of the 1,048,576-triangle
+// heightfield 209; now 389 + 71 and 86 + 60 (builds: 1.73 -> 1.65 ms; 8.4M clustered
+// triangles 13.4 -> 12.7 ms; the batch's graph 10.95 -> 10.38 ms).
+template <bool REFIT, bool COST>
+__global__ void __launch_bounds__(kUpLeaves) k_bottom_up(UpArgs A) {
+	__shared__ UpShared S;
+	const uint32_t b0 = blockIdx.x * kUpLeaves, t = threadIdx.x, i = b0 + t;
+	const bool live = i < A.n;
+	S.count[t] = 0;
+	const uint4 sp = live ? A.splits[i] : PRT_NO_SPLIT;
+	S.first[t] = sp.x;
+	S.last[t] = sp.y;
+	S.node[t] = sp.z;
+	if (!REFIT && sp.z != kNone && sp.x >= b0 && sp.y < b0 + kUpLeaves) {
+		if (sp.z >= A.n_ids) {
+			atomicOr(A.err, kErrCollapse);
+			S.node[t] = 0u;
+		} else {
+			const float4 lo = A.ibox[2 * (size_t)sp.z], hi = A.ibox[2 * (size_t)sp.z + 1];
+			S.nbox[0][t] = lo.x;
+			S.nbox[1][t] = lo.y;
+			S.nbox[2][t] = lo.z;
+			S.nbox[3][t] = hi.x;
+			S.nbox[4][t] = hi.y;
+			S.nbox[5][t] = hi.z;
+		}
+	}
+	for (uint32_t k = t; k < kUpLeaves + 2u; k += kUpLeaves)
+		S.n_ready[k] = 0;
+	if (t == 0)
+		S.n_escape = 0;
+	if (live) {
+		float4 lo, hi;
+		if (REFIT) {
+			const float *v = A.tris + 9 * (size_t)A.vals[i];
+			if (tri_finite(v)) {
+				lo = make_float4(fminf(v[0], fminf(v[3], v[6])), fminf(v[1], fminf(v[4], v[7])),
+				                 fminf(v[2], fminf(v[5], v[8])), 0.0f);
+				hi = make_float4(fmaxf(v[0], fmaxf(v[3], v[6])), fmaxf(v[1], fmaxf(v[4], v[7])),
+				                 fmaxf(v[2], fmaxf(v[5], v[8])), 0.0f);
+			} else {
+				lo = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
+				hi = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
+			}
+			__stcg(&A.lbox[2 * (size_t)i], lo);
+			__stcg(&A.lbox[2 * (size_t)i + 1], hi);
+		} else {
+			lo = A.lbox[2 * (size_t)i];
+			hi = A.lbox[2 * (size_t)i + 1];
+		}
+		S.lbox[0][t] = lo.x;
+		S.lbox[1][t] = lo.y;
+		S.lbox[2][t] = lo.z;
+		S.lbox[3][t] = hi.x;
+		S.lbox[4][t] = hi.y;
+		S.lbox[5][t] = hi.z;
+	}
+	__syncthreads();
+	if (live)
+		up_deliver(A, S, b0, (uint16_t)(t | kUpLeaf), i, i, 0u);
+	for (uint32_t round = 0;; ++round) { // at most kUpLeaves: each round finishes a node
+		__syncthreads();
+		const uint32_t m = min(S.n_ready[round], kUpLeaves);
+		if (m == 0u || round > kUpLeaves)
+			break;
+		if (t < m) {
+			const uint32_t slot = S.ready[round & 1u][t];
+			const uint32_t p = min(S.node[slot], A.n_ids - 1u);
+			const uint32_t f = S.first[slot], l = S.last[slot];
+			const uint16_t cl16 = S.child[0][slot], cr16 = S.child[1][slot];
+			float4 llo, lhi, rlo, rhi, lo, hi;
+			float cl[8], cr[8];
+			up_child(S, cl16, llo, lhi, cl, COST);
+			up_child(S, cr16, rlo, rhi, cr, COST);
+			if (REFIT) {
+				lo = make_float4(fminf(llo.x, rlo.x), fminf(llo.y, rlo.y), fminf(llo.z, rlo.z),
+				                 (cl16 & kUpLeaf) ? -1.0f : half_area(llo, lhi));
+				hi = make_float4(fmaxf(lhi.x, rhi.x), fmaxf(lhi.y, rhi.y), fmaxf(lhi.z, rhi.z),
+				                 (cr16 & kUpLeaf) ? -1.0f : half_area(rlo, rhi));
+				__stcg(&A.ibox[2 * (size_t)p], lo);
+				__stcg(&A.ibox[2 * (size_t)p + 1], hi);
+				S.nbox[0][slot] = lo.x;
+				S.nbox[1][slot] = lo.y;
+				S.nbox[2][slot] = lo.z;
+				S.nbox[3][slot] = hi.x;
+				S.nbox[4][slot] = hi.y;
+				S.nbox[5][slot] = hi.z;
+			} else {
+				lo = make_float4(S.nbox[0][slot], S.nbox[1][slot], S.nbox[2][slot], 0.0f);
+				hi = make_float4(S.nbox[3][slot], S.nbox[4][slot], S.nbox[5][slot], 0.0f);
+			}
+			if (COST) {
+				const CostNode c =
+				    merge_costs(cl, cr, half_extent(llo, lhi), half_extent(rlo, rhi),
+				                half_extent(lo, hi), l - f + 1u, A.leaf_size);
+				S.cost[0][slot] = c.c1;
+				__stcg(&A.cost[p].c1, c.c1);
+#pragma unroll
+				for (int k = 0; k < 7; ++k) {
+					S.cost[1 + k][slot] = c.cd[k];
+					__stcg(&A.cost[p].cd[k], c.cd[k]);
+				}
+				__stcg(&A.cost[p].bits, c.bits);
+			}
+			up_deliver(A, S, b0, (uint16_t)slot, f, l, round + 1u);
+		}
+	}
+	const uint32_t n_out = min(S.n_escape, kUpLeaves);
+	if (t == 0 && n_out)
+		S.walk_at = atomicAdd(A.n_walks, n_out);
+	__syncthreads();
+	if (t < n_out) {
+		if (S.walk_at + t < A.walk_cap)
+			A.walks[S.walk_at + t] = S.escape[t];
+		else
+			atomicOr(A.err, kErrCollapse);
+	}
+}
+
+// The rest of the bottom-up pass: one thread per subtree that a block ended with walks
+// towards the root; at each node the first to arrive stops and the second, which sees both
+// children, goes on (nobody waits).  What does not depend on the sibling is read before the
+// arrival: a step is bound by its atomic and the reads after it.  A launch of its own,
+// because a block of k_bottom_up kept its place for the longest of its walks.
+template <bool REFIT, bool COST>
+__global__ void __launch_bounds__(128) k_walk_up(UpArgs A) {
+	const uint32_t n = min(*A.n_walks, A.walk_cap);
+	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+		uint4 at = A.splits[A.walks[k]];
+		// A path to the root passes each binary node once; a longer walk (or an index out of
+		// range) means corrupt splits, reported instead of followed.
+		for (uint32_t steps = 0;; ++steps) {
+			const uint32_t p = at.z;
+			if (p >= A.n_ids || steps >= A.n_ids || at.y >= A.n) {
+				atomicOr(A.err, kErrCollapse);
+				break;
+			}
+			const uint32_t l = A.left[p], r = A.right[p];
+			const uint4 as_left = A.splits[at.y]; // the parent, if p is its left child ...
+			const uint4 as_right = at.x > 0u ? A.splits[at.x - 1u] : PRT_NO_SPLIT; // ... or right
+			float4 lo, hi;
+			if (!REFIT) {
+				lo = A.ibox[2 * (size_t)p];
+				hi = A.ibox[2 * (size_t)p + 1];
+			}
+			// Release: what was written below is visible before this arrival counts.
+			// Acquire: the sibling's results are read after its arrival.
+			if (arrive_acq_rel(&A.flags[p]) == 0u)
+				break;
+			if (REFIT) {
+				float4 llo, lhi, rlo, rhi;
+				child_box(l, A.ibox, A.lbox, llo, lhi);
+				child_box(r, A.ibox, A.lbox, rlo, rhi);
+				lo = make_float4(fminf(llo.x, rlo.x), fminf(llo.y, rlo.y), fminf(llo.z, rlo.z),
+				                 (l & kLeafBit) ? -1.0f : half_area(llo, lhi));
+				hi = make_float4(fmaxf(lhi.x, rhi.x), fmaxf(lhi.y, rhi.y), fmaxf(lhi.z, rhi.z),
+				                 (r & kLeafBit) ? -1.0f : half_area(rlo, rhi));
+				__stcg(&A.ibox[2 * (size_t)p], lo);
+				__stcg(&A.ibox[2 * (size_t)p + 1], hi);
+			}
+			if (COST) {
+				float cl[8], cr[8];
+				const float3 el = child_costs(l, A.cost, A.ibox, A.lbox, cl);
+				const float3 er = child_costs(r, A.cost, A.ibox, A.lbox, cr);
+				const CostNode c = merge_costs(cl, cr, el, er, half_extent(lo, hi),
+				                               at.y - at.x + 1u, A.leaf_size);
+				__stcg(&A.cost[p].c1, c.c1);
+#pragma unroll
+				for (int j = 0; j < 7; ++j)
+					__stcg(&A.cost[p].cd[j], c.cd[j]);
+				__stcg(&A.cost[p].bits, c.bits);
+			}
+			if (as_left.x == at.x)
+				at = as_left;
+			else if (as_right.y == at.y)
+				at = as_right;
+			else
+				break; // a root
+		}
 	}
 }
 
@@ -945,8 +1127,7 @@ int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compre
 	BUILD_TRY(ws.int_off.reserve(4ull * (S + 1)));
 	BUILD_TRY(ws.left.reserve(4 * ni));
 	BUILD_TRY(ws.right.reserve(4 * ni));
-	BUILD_TRY(ws.parent_int.reserve(4 * ni));
-	BUILD_TRY(ws.parent_leaf.reserve(4 * nn));
+	BUILD_TRY(ws.splits.reserve(16 * nn));
 	BUILD_TRY(ws.rfirst.reserve(4 * ni));
 	BUILD_TRY(ws.rlast.reserve(4 * ni));
 	BUILD_TRY(ws.flags.reserve(4 * ni));
@@ -995,7 +1176,8 @@ static int lbvh_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch
 	const size_t nn = std::max<uint32_t>(n, 1);
 	uint32_t *gb = ws.bounds.as<uint32_t>();
 	svals = ws.vals.as<uint32_t>();
-	k_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S);
+	k_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S, d_toff,
+	                                                         ws.splits.as<uint4>());
 	if (n)
 		k_centroid_bounds<<<std::min(blocks_for(n, 256), 2048u), 256, 0, st>>>(d_tris, n, scene_of,
 		                                                                        gb);
@@ -1022,27 +1204,17 @@ static int lbvh_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch
 		svals = where ? ws.vals2.as<uint32_t>() : ws.vals.as<uint32_t>();
 	}
 
-	BUILD_TRY(cudaMemsetAsync(ws.parent_leaf.p, 0xFF, 4 * nn, st));
 	if (n_int) {
 		if (plan.multi)
 			k_karras<uint64_t><<<blocks_for(n_int, 256), 256, 0, st>>>(
 			    static_cast<const uint64_t *>(skeys), n_int, d_toff, d_ioff, S,
-			    ws.left.as<uint32_t>(), ws.right.as<uint32_t>(), ws.parent_int.as<uint32_t>(),
-			    ws.parent_leaf.as<uint32_t>(), ws.rfirst.as<uint32_t>(), ws.rlast.as<uint32_t>());
+			    ws.left.as<uint32_t>(), ws.right.as<uint32_t>(), ws.splits.as<uint4>(),
+			    ws.rfirst.as<uint32_t>(), ws.rlast.as<uint32_t>());
 		else
 			k_karras<uint32_t><<<blocks_for(n_int, 256), 256, 0, st>>>(
 			    static_cast<const uint32_t *>(skeys), n_int, d_toff, d_ioff, S,
-			    ws.left.as<uint32_t>(), ws.right.as<uint32_t>(), ws.parent_int.as<uint32_t>(),
-			    ws.parent_leaf.as<uint32_t>(), ws.rfirst.as<uint32_t>(), ws.rlast.as<uint32_t>());
-		BUILD_TRY(cudaMemsetAsync(ws.flags.p, 0, 4 * ni, st));
-	}
-	if (n) {
-		k_leaf_boxes<<<blocks_for(n, 256), 256, 0, st>>>(d_tris, svals, n, ws.lbox.as<float4>());
-		if (n_int)
-			k_refit<<<blocks_for(n, 256), 256, 0, st>>>(
-			    n, n_int, ws.parent_leaf.as<uint32_t>(), ws.parent_int.as<uint32_t>(),
-			    ws.left.as<uint32_t>(), ws.right.as<uint32_t>(), ws.lbox.as<float4>(),
-			    ws.ibox.as<float4>(), ws.flags.as<uint32_t>(), d_err);
+			    ws.left.as<uint32_t>(), ws.right.as<uint32_t>(), ws.splits.as<uint4>(),
+			    ws.rfirst.as<uint32_t>(), ws.rlast.as<uint32_t>());
 	}
 	return PRT_OK;
 }
@@ -1106,19 +1278,44 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 	}
 	// Binary node ids run up to n_int (LBVH) or n_int + S (SAH: scene s's root is s).
 	const uint32_t n_ids = n_int + (plan.sah ? S : 0u);
-	const CostNode *cost = nullptr;
-	if (plan.collapse_cost && n_int) {
-		BUILD_TRY(cudaMemsetAsync(ws.flags.p, 0, 4ull * n_ids, st));
-		k_collapse_cost<<<blocks_for(n, 256), 256, 0, st>>>(
-		    n, n_ids, ws.parent_leaf.as<uint32_t>(), ws.parent_int.as<uint32_t>(),
-		    ws.left.as<uint32_t>(), ws.right.as<uint32_t>(), ws.rfirst.as<uint32_t>(),
-		    ws.rlast.as<uint32_t>(), ws.ibox.as<float4>(), ws.lbox.as<float4>(),
-		    ws.flags.as<uint32_t>(), ws.cost.as<CostNode>(), (uint32_t)plan.leaf_size, d_err);
-		cost = ws.cost.as<CostNode>();
-	}
-
 	uint32_t *ctr = ws.counters.as<uint32_t>();
 	BUILD_TRY(cudaMemsetAsync(ctr, 0, 4 * kCtrWords, st));
+	const bool use_cost = plan.collapse_cost && n_int;
+	if (n && (!plan.sah || use_cost)) {
+		UpArgs U;
+		U.tris = d_tris;
+		U.vals = svals;
+		U.n = n;
+		U.n_ids = n_ids;
+		U.splits = ws.splits.as<uint4>();
+		U.left = ws.left.as<uint32_t>();
+		U.right = ws.right.as<uint32_t>();
+		U.ibox = ws.ibox.as<float4>();
+		U.lbox = ws.lbox.as<float4>();
+		U.flags = ws.flags.as<uint32_t>();
+		U.cost = ws.cost.as<CostNode>();
+		U.leaf_size = (uint32_t)plan.leaf_size;
+		U.err = d_err;
+		BUILD_TRY(cudaMemsetAsync(ws.flags.p, 0, 4ull * std::max<uint32_t>(n_ids, 1u), st));
+		// (items_a is free until the collapse, which starts after the walks.)
+		U.walks = ws.items_a.as<uint32_t>();
+		U.walk_cap = 2u * plan.node_cap;
+		U.n_walks = ctr + kCtrWalks;
+		const unsigned grid = blocks_for(n, kUpLeaves);
+		const unsigned g_walk = std::min(1216u, blocks_for(n, 128));
+		if (plan.sah) {
+			k_bottom_up<false, true><<<grid, kUpLeaves, 0, st>>>(U);
+			k_walk_up<false, true><<<g_walk, 128, 0, st>>>(U);
+		} else if (use_cost) {
+			k_bottom_up<true, true><<<grid, kUpLeaves, 0, st>>>(U);
+			k_walk_up<true, true><<<g_walk, 128, 0, st>>>(U);
+		} else {
+			k_bottom_up<true, false><<<grid, kUpLeaves, 0, st>>>(U);
+			k_walk_up<true, false><<<g_walk, 128, 0, st>>>(U);
+		}
+	}
+	const CostNode *cost = use_cost ? ws.cost.as<CostNode>() : nullptr;
+
 	Item *items_of[2] = {ws.items_a.as<Item>(), ws.items_b.as<Item>()};
 	k_collapse_roots<<<blocks_for(S, 128), 128, 0, st>>>(d_toff, roots, S, items_of[0], ctr);
 	CollapseArgs A;

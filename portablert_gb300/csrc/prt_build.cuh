@@ -87,13 +87,18 @@ struct SceneGPU {
 // word as the host reads them between levels (a copy into pageable memory is staged).
 constexpr int kHostSahWords = 16;
 
+// `splits` entry of a scene's last leaf position, after which no node splits.
+#define PRT_NO_SPLIT make_uint4(kNone, kNone, kNone, kNone)
+
 // Scratch reused across builds (grow-only).
 struct BuildScratch {
 	DevBuf keys, vals, keys2, vals2;  // Morton keys (u32 or u64) and triangle indices
 	DevBuf scene_of;                  // scene of each input triangle (several scenes)
 	DevBuf int_off;                   // first binary node of each scene
 	DevBuf left, right;               // children of the binary nodes (bit 31 = leaf)
-	DevBuf parent_int, parent_leaf;   // parents of binary nodes and of leaves
+	DevBuf splits;                    // uint4 per leaf position: the binary node that splits
+	                                  // after it (first leaf, last leaf, node id), or
+	                                  // PRT_NO_SPLIT at the end of a scene
 	DevBuf rfirst, rlast;             // leaf range of each binary node
 	DevBuf ibox, lbox;                // boxes of binary nodes and of leaves (2 float4 each)
 	DevBuf flags;                     // refit arrival counters

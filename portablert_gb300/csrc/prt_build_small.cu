@@ -121,7 +121,7 @@ __device__ __forceinline__ float union_area(const Box &a, const Box &b) {
 	return fminf(dx * dy + dz * (dx + dy), FLT_MAX);
 }
 
-// The box of a triangle as the other builders make it (k_leaf_boxes): [-FLT_MAX,
+// The box of a triangle as the other builders make it (k_bottom_up): [-FLT_MAX,
 // FLT_MAX]^3 for a non-finite vertex.
 __device__ __forceinline__ Box tri_box(const float t[9], bool fin) {
 	if (!fin)

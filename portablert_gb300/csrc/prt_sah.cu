@@ -89,7 +89,7 @@ struct SahArgs {
 	float4 *lbox;           // out: leaf boxes by position
 	uint32_t *left, *right, *rfirst, *rlast;
 	float4 *ibox;
-	uint32_t *parent_int, *parent_leaf; // for the bottom-up cost pass of the collapse
+	uint4 *splits;          // out: by leaf position, for the bottom-up cost pass
 	uint32_t node_cap, max_large, max_mid, max_small, max_chunks;
 	uint32_t n;             // triangles (records per buffer)
 	uint32_t *err;
@@ -456,14 +456,7 @@ __device__ void emit_split(const SahArgs &A, const SahTask &t, const Split &s, i
 	A.right[t.node] = rr;
 	A.rfirst[t.node] = t.begin;
 	A.rlast[t.node] = t.begin + t.count - 1u;
-	if (nl > 1)
-		A.parent_int[ids[0]] = t.node;
-	else
-		A.parent_leaf[t.begin] = t.node;
-	if (nr > 1)
-		A.parent_int[ids[1]] = t.node;
-	else
-		A.parent_leaf[t.begin + nl] = t.node;
+	A.splits[t.begin + nl - 1u] = make_uint4(t.begin, t.begin + t.count - 1u, t.node, 0u);
 	// Children's areas: known now for a binned split (leaves keep -1); after halves each
 	// child writes its own when it is split.
 	write_node_box(A, t.node, s.node, (binned && nl > 1) ? box_area(s.left) : -1.0f,
@@ -576,6 +569,7 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uin
 	if (lane == 0) {
 		roots[s] = s;
 		if (n) {
+			A.splits[b + n - 1u] = PRT_NO_SPLIT;
 			float flo[3], fsc[3];
 			for (int k = 0; k < 3; ++k) {
 				flo[k] = ord2f(gb[6 * s + k]);
@@ -977,14 +971,7 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 		A.right[r.node] = nr > 1 ? id_r : (kLeafBit | pos_r);
 		A.rfirst[r.node] = pos_l;
 		A.rlast[r.node] = pos_l + r.count - 1u;
-		if (nl > 1)
-			A.parent_int[id_l] = r.node;
-		else
-			A.parent_leaf[pos_l] = r.node;
-		if (nr > 1)
-			A.parent_int[id_r] = r.node;
-		else
-			A.parent_leaf[pos_r] = r.node;
+		A.splits[pos_r - 1u] = make_uint4(pos_l, pos_l + r.count - 1u, r.node, 0u);
 		// Children's areas: known now for a binned split (leaves keep -1); after halves each
 		// child writes its own when it is split.
 		write_node_box(A, r.node, s.node, (binned && nl > 1) ? box_area(s.left) : -1.0f,
@@ -1120,14 +1107,7 @@ __device__ __forceinline__ void write_small_node(const SahArgs &A, uint32_t node
 	A.right[node] = nr > 1 ? id_r : (kLeafBit | (first + nl));
 	A.rfirst[node] = first;
 	A.rlast[node] = first + nl + nr - 1u;
-	if (nl > 1)
-		A.parent_int[id_l] = node;
-	else
-		A.parent_leaf[first] = node;
-	if (nr > 1)
-		A.parent_int[id_r] = node;
-	else
-		A.parent_leaf[first + nl] = node;
+	A.splits[first + nl - 1u] = make_uint4(first, first + nl + nr - 1u, node, 0u);
 	write_node_box(A, node, box_union(lb, rb), nl > 1 ? box_area(lb) : -1.0f,
 	               nr > 1 ? box_area(rb) : -1.0f);
 }
@@ -1429,8 +1409,7 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	A.rfirst = ws.rfirst.as<uint32_t>();
 	A.rlast = ws.rlast.as<uint32_t>();
 	A.ibox = ws.ibox.as<float4>();
-	A.parent_int = ws.parent_int.as<uint32_t>();
-	A.parent_leaf = ws.parent_leaf.as<uint32_t>();
+	A.splits = ws.splits.as<uint4>();
 	A.node_cap = plan.n_int + S;
 	A.max_large = (uint32_t)L.max_large;
 	A.max_mid = (uint32_t)L.max_mid;
@@ -1441,9 +1420,6 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 
 	uint32_t *gb = ws.bounds.as<uint32_t>();
 	cudaMemsetAsync(A.ctr, 0, 4 * kCtrWordsSah, st);
-	// No parent: the roots and the triangles of one-triangle scenes keep these.
-	cudaMemsetAsync(A.parent_int, 0xFF, 4ull * A.node_cap, st);
-	cudaMemsetAsync(A.parent_leaf, 0xFF, 4ull * n, st);
 	k_sah_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S);
 	if (n)
 		k_sah_records<<<blocks_for(n, 256), 256, 0, st>>>(d_tris, n, scene_of, A.rec[0], gb);

@@ -60,3 +60,32 @@ def test_levels_across_blocks(gpu_backend, oracle_lib, count, leaf, cost):
         b.set_option("leaf_size", 1)
         b.set_option("collapse_cost", 1)
         b.set_option("node_format", 0)
+
+
+@pytest.mark.parametrize("n", [2, 3, 255, 256, 257, 258, 511, 512, 513, 769, 5000])
+@pytest.mark.parametrize("sah,cost", [(0, 0), (0, 1), (1, 1)])
+def test_bottom_up_across_blocks(gpu_backend, oracle_lib, n, sah, cost):
+    """The bottom-up pass finishes the nodes of 256 leaves in one block and walks the rest:
+    scenes at the block boundary, one of them a chain of ever larger gaps (one deep tree)."""
+    b = gpu_backend
+    chain = W.soup_tris(60, n)
+    chain[:, 0::3] = (chain[:, 0::3] + (1.02 ** np.arange(n))[:, None]).astype(np.float32)
+    rays = W.soup_rays(61, 1000)
+    rays_c = rays.copy()
+    rays_c[:, 3:] = chain.reshape(-1, 3, 3).mean(1)[np.arange(1000) % n] - rays[:, :3]
+    try:
+        b.set_option("build_small", 0)
+        b.set_option("build_sah", sah)
+        b.set_option("collapse_cost", cost)
+        for tris, r in ((W.soup_tris(62, n), rays), (chain, rays_c)):
+            want = oracle_lib.brute_force(tris, r)
+            b.set_tris(tris)
+            got = b.nearest_hits(r, hitreg.TAGS)
+            v = want["valid"] != 0
+            assert np.array_equal(got["valid"], want["valid"])
+            assert np.array_equal(got["t"].view(np.uint32), want["t"].view(np.uint32))
+            assert np.array_equal(got["primitive_id"][v], want["primitive_id"][v])
+    finally:
+        b.set_option("build_small", 1)
+        b.set_option("build_sah", 1)
+        b.set_option("collapse_cost", 1)
