@@ -502,6 +502,11 @@ __device__ __forceinline__ void packet_descent(const TravArgs &a, const SceneDes
 	}
 }
 
+// (Small launches hold both box tests: 64 registers, which 8 blocks allow, spill nothing.)
+#ifndef PRT_TRAVERSE_MIN_BLOCKS_SMALL
+#define PRT_TRAVERSE_MIN_BLOCKS_SMALL 8
+#endif
+
 // The traversal of one batch of up to 32 rays (slots 0..nb-1 of S) through scene sd.
 // REGULAR: every ray of the batch is regular (kind 0), so inner boxes take the plain slab
 // test only (no branch to the conservative test per child).  PACKET: it starts with a packet
@@ -741,9 +746,11 @@ __device__ __forceinline__ bool claim_batch(const ServeQueues &q, uint32_t held[
 // in the kernel at all: 8 % faster), the others counted in a.deferred and skipped; 2 =
 // the skipped batches with the general test (returns at once when there are none); 3 =
 // a serving launch: batches claimed from the serving queues (claim_batch), the plain or
-// the general test chosen per batch, descriptors and rays read around L1.
+// the general test chosen per batch, descriptors and rays read around L1; 4 = a small launch
+// of one run: every batch, the test chosen per batch, without counters.
 template <int FMT, bool COUNT, bool LEAF1, bool BOUNDED, int PASS>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, FMT == PRT_NODES_FP32
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_MIN_BLOCKS_SMALL
+                                                       : FMT == PRT_NODES_FP32
                                                            ? PRT_TRAVERSE_MIN_BLOCKS_FP32
                                                            : PRT_TRAVERSE_MIN_BLOCKS_COMPRESSED)
     k_trace8(TravArgs a) {
@@ -761,6 +768,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, FMT == PRT_NODES_FP32
 	if (PASS == 2 && *(volatile const uint32_t *)a.deferred == 0u)
 		return; // the regular pass took every batch (it ran before, on the same stream)
 
+	uint32_t dealt = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * a.batch; // PASS 4
 	if (BOUNDED && lane == 0)
 		S.batches = 0;
 	if (PASS == 3 && lane == 0) {
@@ -778,8 +786,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, FMT == PRT_NODES_FP32
 				++S.batches;
 		}
 		// Batches are taken in order from a counter (the deferred pass has its own, so
-		// the few batches it works on spread over all warps); a serving launch claims
-		// them from its queues.
+		// the few batches it works on spread over all warps); a small launch deals them
+		// out by warp; a serving launch claims them from its queues.
 		uint32_t base = 0;
 		const SegDesc *segs = a.segs;
 		if (PASS == 3) {
@@ -810,9 +818,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, FMT == PRT_NODES_FP32
 				S.cached_q = qsel;
 			}
 		} else {
-			if (lane == 0)
-				base = atomicAdd(PASS == 2 ? a.deferred + 1 : a.counter, a.batch);
-			base = __shfl_sync(0xFFFFFFFFu, base, 0);
+			if (PASS == 4) {
+				base = dealt;
+				dealt += gridDim.x * (blockDim.x >> 5) * a.batch;
+			} else {
+				if (lane == 0)
+					base = atomicAdd(PASS == 2 ? a.deferred + 1 : a.counter, a.batch);
+				base = __shfl_sync(0xFFFFFFFFu, base, 0);
+			}
 			if (base >= a.n_virtual)
 				break;
 			// The run these rays belong to (runs are padded to whole warps of 32, and
@@ -885,7 +898,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, FMT == PRT_NODES_FP32
 			if (PASS == 2 && regular)
 				continue; // done by the regular pass
 			constexpr bool kPacket = PASS == 0 && !COUNT;
-			if ((PASS == 3 || kPacket) && regular)
+			if ((PASS == 3 || PASS == 4 || kPacket) && regular)
 				trace_batch<FMT, COUNT, LEAF1, true, kPacket>(a, S, queue, pool, sd, nb, lane, g, s, lt,
 				                                     step_limit, n_visits, n_tests, fault);
 			else
@@ -1052,6 +1065,49 @@ void launch_t(const TravArgs &a, int warps, int sm_count, cudaStream_t st) {
 	    <<<(unsigned)grid, 32 * warps, (size_t)a.warp_bytes * warps, st>>>(a);
 }
 
+int warps_for(const TravConfig &cfg) {
+	return (cfg.block >= 32 && cfg.block <= 32 * kWarpsPerBlock && cfg.block % 32 == 0)
+	           ? cfg.block / 32
+	           : kWarpsPerBlock;
+}
+
+// A launch of one run with at most 32 rays per resident warp (155,648 on 152 SMs): one kernel,
+// no counters, batches of 4 rays while every warp gets at most one, else of 8, dealt out by
+// warp.  The two passes cost two memsets and a second launch more, which is most of a small
+// query, and a warp's serial chain is shorter with fewer rays.  Measured (back to back, us;
+// 4,096-triangle soup / 65,790-triangle heightfield / 1M clustered triangles):
+//     rays       two passes        4 per batch       8                16
+//     1,000      26 / 23 / 36      13 / 12 / 23      18 / 15 / 29     28 / 25 / 39
+//     8,192      26 / 68 / 41      15 / 31 / 25      19 / 43 / 33     29 / 60 / 45
+//     32,768     37 / 79 / 55      29 / 35 / 45      25 / 43 / 45     33 / 68 / 62
+//     65,536     52 / 39 / 65      48 / 28 / 68      45 / 31 / 61     44 / 44 / 68
+//     131,072    87 / 48 / 101     92 / 43 / 119     81 / 39 / 107    84 / 50 / 103
+//     200,000    116 / 65 / 137    138 / 62 / 174    119 / 55 / 148   117 / 56 / 144
+constexpr uint32_t kSmallPerWarp = 32;
+
+template <int FMT, bool LEAF1>
+bool launch_small(TravArgs a, int warps, int sm_count, cudaStream_t st) {
+	const uint64_t slots = (uint64_t)sm_count * warps *
+	                       blocks_per_sm<FMT, false, LEAF1, false, 4>(warps, a.warp_bytes);
+	const uint64_t per = (a.n_virtual + slots - 1) / slots;
+	if (per > kSmallPerWarp)
+		return false;
+	a.batch = per <= 4u ? 4u : 8u;
+	launch_t<FMT, false, LEAF1, false, 4>(a, warps, sm_count, st);
+	return true;
+}
+
+bool try_small(const TravArgs &a, const TravConfig &cfg, int warps, int sm_count,
+               cudaStream_t st) {
+	if (a.n_segs || a.use_cam || cfg.count || a.max_batches)
+		return false;
+	if (cfg.format == PRT_NODES_COMPRESSED)
+		return a.max_leaf <= 1u ? launch_small<PRT_NODES_COMPRESSED, true>(a, warps, sm_count, st)
+		                        : launch_small<PRT_NODES_COMPRESSED, false>(a, warps, sm_count, st);
+	return a.max_leaf <= 1u ? launch_small<PRT_NODES_FP32, true>(a, warps, sm_count, st)
+	                        : launch_small<PRT_NODES_FP32, false>(a, warps, sm_count, st);
+}
+
 template <int FMT, bool LEAF1>
 void launch_passes(const TravArgs &a, int warps, int sm_count, cudaStream_t st) {
 	if (a.max_batches > 0)
@@ -1100,19 +1156,15 @@ uint32_t batch_rays(uint64_t m, int sm_count, uint32_t max_batches) {
 	return m >= wave ? 16 : 8;
 }
 
-int warps_for(const TravConfig &cfg) {
-	return (cfg.block >= 32 && cfg.block <= 32 * kWarpsPerBlock && cfg.block % 32 == 0)
-	           ? cfg.block / 32
-	           : kWarpsPerBlock;
-}
-
 cudaError_t dispatch(const TravArgs &a, const TravConfig &cfg, int sm_count, cudaStream_t st) {
+	const int warps = warps_for(cfg);
+	if (try_small(a, cfg, warps, sm_count, st))
+		return cudaGetLastError();
 	cudaError_t e = cudaMemsetAsync(a.counter, 0, 4, st);
 	if (e == cudaSuccess)
 		e = cudaMemsetAsync(a.deferred, 0, 8, st);
 	if (e != cudaSuccess)
 		return e;
-	const int warps = warps_for(cfg);
 	if (cfg.format == PRT_NODES_COMPRESSED) {
 		if (cfg.count)
 			launch<PRT_NODES_COMPRESSED, true>(a, warps, sm_count, st);
