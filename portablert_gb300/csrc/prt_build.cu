@@ -354,6 +354,7 @@ struct UpArgs {
 	uint32_t leaf_size;
 	uint32_t *walks, *n_walks; // slots at which the blocks' parts end
 	uint32_t walk_cap;
+	const uint32_t *gate;     // null, or: nothing to do unless it is 0
 	uint32_t *err;
 };
 
@@ -446,6 +447,8 @@ template <bool REFIT, bool COST>
 __global__ void __launch_bounds__(kUpLeaves) k_bottom_up(UpArgs A) {
 	__shared__ UpShared S;
 	const uint32_t b0 = blockIdx.x * kUpLeaves, t = threadIdx.x, i = b0 + t;
+	if (A.gate && *A.gate)
+		return;
 	const bool live = i < A.n;
 	S.count[t] = 0;
 	const uint4 sp = live ? A.splits[i] : PRT_NO_SPLIT;
@@ -637,7 +640,7 @@ __global__ void k_collapse_roots(const uint32_t *tri_off, const uint32_t *int_of
                                  uint32_t n_scenes, Item *items, uint32_t *ctr) {
 	const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
 	if (s == 0) {
-		ctr[0] = n_scenes;
+		ctr[0] = ctr[kCtrGate] ? 0u : n_scenes; // (incomplete trees: no items, no levels)
 		ctr[kCtrNodes] = n_scenes;
 	}
 	if (s >= n_scenes)
@@ -1233,53 +1236,18 @@ static cudaError_t write_dead_node(const BuildPlan &plan, SceneGPU &sc, cudaStre
 	return e;
 }
 
-int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, BuildScratch &ws,
-                  cudaStream_t st, uint32_t *d_err, bool host_checks, std::string &msg) {
+// From the binary trees to the 8-wide ones: the bottom-up pass and the collapse.  With host
+// checks it waits, and the counters (kCtrGate among them) are in ws.h_counters.
+static int collapse_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc,
+                            BuildScratch &ws, const uint32_t *svals, const uint32_t *roots,
+                            cudaStream_t st, uint32_t *d_err, bool host_checks,
+                            std::string &msg) {
 	const uint32_t S = plan.S, n = plan.n, n_int = plan.n_int;
-	if (plan.sah && !host_checks) {
-		msg = "the SAH build reads its level counters on the host";
-		return PRT_ERR_ARG;
-	}
-	if (plan.small) {
-		// One block: PLOC, collapse and re-layout in one launch, which also zeroes the
-		// counters, writes the empty node and leaves the counters in the pinned host
-		// buffer; the compression reads the node count on the device, so the host only
-		// waits, once, at the end.
-		uint32_t *ctr = ws.counters.as<uint32_t>();
-		BUILD_TRY(launch_build_small(d_tris, n, (uint32_t)plan.leaf_size, plan.collapse_cost,
-		                             plan.compressed, ws, sc, plan.node_cap, ctr, ws.h_counters,
-		                             d_err, st));
-		sc.built_small = true;
-		if (plan.compressed) {
-			k_compress<<<blocks_for(8ull * plan.node_cap, 256), 256, 0, st>>>(
-			    sc.nodes.as<Node8>(), ctr + kCtrNodes, sc.cnodes.as<CNode8>());
-			sc.has_cnodes = true;
-		}
-		BUILD_TRY(cudaGetLastError());
-		return host_checks ? build_finish(sc, ws, st, msg, true) : PRT_OK;
-	}
-	BUILD_TRY(write_dead_node(plan, sc, st));
 	uint32_t *d_toff = sc.tri_off.as<uint32_t>();
-	uint32_t *d_ioff = ws.int_off.as<uint32_t>();
 	uint32_t *scene_of = plan.multi ? ws.scene_of.as<uint32_t>() : nullptr;
-	if (plan.multi)
-		k_scene_of<<<std::min(S, 4096u), 256, 0, st>>>(d_toff, S, scene_of);
-	const uint32_t *svals = ws.vals.as<uint32_t>();
-	const uint32_t *roots = d_ioff;
-	if (plan.sah) {
-		int rc = sah_build_enqueue(d_tris, plan, ws, d_toff, scene_of, st, d_err, msg);
-		if (rc != PRT_OK)
-			return rc;
-		roots = ws.roots.as<uint32_t>();
-	} else {
-		int rc = lbvh_enqueue(d_tris, plan, ws, d_toff, d_ioff, scene_of, st, d_err, svals, msg);
-		if (rc != PRT_OK)
-			return rc;
-	}
+	uint32_t *ctr = ws.counters.as<uint32_t>();
 	// Binary node ids run up to n_int (LBVH) or n_int + S (SAH: scene s's root is s).
 	const uint32_t n_ids = n_int + (plan.sah ? S : 0u);
-	uint32_t *ctr = ws.counters.as<uint32_t>();
-	BUILD_TRY(cudaMemsetAsync(ctr, 0, 4 * kCtrWords, st));
 	const bool use_cost = plan.collapse_cost && n_int;
 	if (n && (!plan.sah || use_cost)) {
 		UpArgs U;
@@ -1295,6 +1263,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 		U.flags = ws.flags.as<uint32_t>();
 		U.cost = ws.cost.as<CostNode>();
 		U.leaf_size = (uint32_t)plan.leaf_size;
+		U.gate = plan.sah ? ctr + kCtrGate : nullptr;
 		U.err = d_err;
 		BUILD_TRY(cudaMemsetAsync(ws.flags.p, 0, 4ull * std::max<uint32_t>(n_ids, 1u), st));
 		// (items_a is free until the collapse, which starts after the walks.)
@@ -1367,7 +1336,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 			break;
 		BUILD_TRY(cudaMemcpyAsync(ws.h_counters, ctr, 4 * kCtrWords, cudaMemcpyDeviceToHost, st));
 		BUILD_TRY(cudaStreamSynchronize(st));
-		if (ws.h_counters[level] == 0)
+		if (ws.h_counters[level] == 0 || ws.h_counters[kCtrGate] != 0)
 			break;
 		if (level >= kMaxLevels) {
 			msg = "tree deeper than " + std::to_string(kMaxLevels) + " levels";
@@ -1375,8 +1344,74 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 		}
 		ahead = kLevelsPerCheck;
 	}
-	sc.has_cnodes = plan.compressed;
 	BUILD_TRY(cudaGetLastError());
+	return PRT_OK;
+}
+
+int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, BuildScratch &ws,
+                  cudaStream_t st, uint32_t *d_err, bool host_checks, std::string &msg) {
+	const uint32_t S = plan.S, n = plan.n;
+	if (plan.sah && !host_checks) {
+		msg = "the SAH build reads its level counters on the host";
+		return PRT_ERR_ARG;
+	}
+	if (plan.small) {
+		// One block: PLOC, collapse and re-layout in one launch, which also zeroes the
+		// counters, writes the empty node and leaves the counters in the pinned host
+		// buffer; the compression reads the node count on the device, so the host only
+		// waits, once, at the end.
+		uint32_t *ctr = ws.counters.as<uint32_t>();
+		BUILD_TRY(launch_build_small(d_tris, n, (uint32_t)plan.leaf_size, plan.collapse_cost,
+		                             plan.compressed, ws, sc, plan.node_cap, ctr, ws.h_counters,
+		                             d_err, st));
+		sc.built_small = true;
+		if (plan.compressed) {
+			k_compress<<<blocks_for(8ull * plan.node_cap, 256), 256, 0, st>>>(
+			    sc.nodes.as<Node8>(), ctr + kCtrNodes, sc.cnodes.as<CNode8>());
+			sc.has_cnodes = true;
+		}
+		BUILD_TRY(cudaGetLastError());
+		return host_checks ? build_finish(sc, ws, st, msg, true) : PRT_OK;
+	}
+	BUILD_TRY(write_dead_node(plan, sc, st));
+	uint32_t *d_toff = sc.tri_off.as<uint32_t>();
+	uint32_t *d_ioff = ws.int_off.as<uint32_t>();
+	uint32_t *scene_of = plan.multi ? ws.scene_of.as<uint32_t>() : nullptr;
+	if (plan.multi)
+		k_scene_of<<<std::min(S, 4096u), 256, 0, st>>>(d_toff, S, scene_of);
+	const uint32_t *svals = ws.vals.as<uint32_t>();
+	const uint32_t *roots = d_ioff;
+	uint32_t *ctr = ws.counters.as<uint32_t>();
+	int sah_level = 0; // large levels of the SAH build queued so far
+	BUILD_TRY(cudaMemsetAsync(ctr, 0, 4 * kCtrWords, st));
+	if (plan.sah) {
+		int rc = sah_build_enqueue(d_tris, plan, ws, d_toff, scene_of, st, d_err, ctr + kCtrGate,
+		                           sah_level, msg);
+		if (rc != PRT_OK)
+			return rc;
+		roots = ws.roots.as<uint32_t>();
+	} else {
+		int rc = lbvh_enqueue(d_tris, plan, ws, d_toff, d_ioff, scene_of, st, d_err, svals, msg);
+		if (rc != PRT_OK)
+			return rc;
+	}
+	int rc = collapse_enqueue(d_tris, plan, sc, ws, svals, roots, st, d_err, host_checks, msg);
+	while (rc == PRT_OK && plan.sah && ws.h_counters[kCtrGate] != 0) {
+		if (ws.h_counters[kCtrGate] != kGateLevels) {
+			BUILD_TRY(cudaMemsetAsync(d_err, 0, 4, st));
+			BUILD_TRY(cudaStreamSynchronize(st));
+			msg = "sah build: internal check failed";
+			return PRT_ERR_DEVICE;
+		}
+		// Splits more uneven than the levels queued ahead allow for: the rest of them.
+		BUILD_TRY(cudaMemsetAsync(ctr, 0, 4 * kCtrWords, st));
+		rc = sah_build_more(plan, ws, st, d_err, ctr + kCtrGate, sah_level, msg);
+		if (rc == PRT_OK)
+			rc = collapse_enqueue(d_tris, plan, sc, ws, svals, roots, st, d_err, host_checks, msg);
+	}
+	if (rc != PRT_OK)
+		return rc;
+	sc.has_cnodes = plan.compressed;
 	return host_checks ? build_finish(sc, ws, st, msg, true) : PRT_OK;
 }
 

@@ -13,11 +13,12 @@ namespace prt {
 constexpr int kMaxLevels = 32;     // 8-wide levels (the traversal's depth limit)
 constexpr int kLevelsPerCheck = 4; // collapse launches between host checks
 // counters layout: [0, kMaxLevels] frontier size per level, then nodes used, triangles placed,
-// walks of the bottom-up pass
+// walks of the bottom-up pass, gate
 constexpr int kCtrNodes = kMaxLevels + 1;
 constexpr int kCtrTris = kMaxLevels + 2;
 constexpr int kCtrWalks = kMaxLevels + 3; // subtrees the bottom-up pass's blocks ended with
-constexpr int kCtrWords = kMaxLevels + 4;
+constexpr int kCtrGate = kMaxLevels + 4;  // SAH builds: kGate* (0: the binary trees are complete)
+constexpr int kCtrWords = kMaxLevels + 5;
 
 // Surface area (up to a constant) of a box; FLT_MAX when it overflows.
 __device__ __forceinline__ float half_area(float4 lo, float4 hi) {

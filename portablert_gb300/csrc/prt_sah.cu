@@ -53,7 +53,7 @@ constexpr uint32_t kHalves = 3;              // split "axis" meaning: first half
 enum : int {
 	kCtrSmall = 0,
 	kCtrMid = 1,
-	kCtrNodes = 2,
+	kCtrNodesSah = 2,
 	kCtrLarge = 4,
 	kCtrChunks = kCtrLarge + kMaxLevels + 2,
 	kCtrWordsSah = kCtrChunks + kMaxLevels + 2
@@ -79,7 +79,7 @@ struct SmallTask {
 
 struct SahArgs {
 	float4 *rec[2];         // (lo, id) (hi, 0) per triangle, two buffers
-	SahTask *large[2];
+	SahTask *large[2];      // (these three by level % 2)
 	uint32_t *bins[2];      // kBinWords per large task
 	uint2 *chunk[2];        // per chunk of the level: large task, first triangle
 	SahTask *mid;
@@ -264,16 +264,22 @@ struct Split {
 	Box6 node, left, right;     // left / right valid for a binned split
 };
 
-// The best plane over the three axes' bins (lane = bin).  Ties go to the lower axis,
-// then the lower bin.  Every lane returns the same result.
-__device__ Split choose_split(const uint32_t *b, const float *fsc, uint32_t count, int lane) {
+// The best plane over the three axes' bins (word(a, k): word k of bin `lane` on axis a).  Ties
+// go to the lower axis, then the lower bin.  Every lane returns the same result.
+template <class Word>
+__device__ __forceinline__ Split choose_split(Word word, const float *fsc, uint32_t count,
+                                              int lane) {
 	Split s;
 	s.axis = kHalves;
 	s.bin = 0;
 	s.n_left = count / 2;
 	uint64_t best = ~0ull;
+#pragma unroll
 	for (int a = 0; a < 3; ++a) {
-		const uint32_t *w = b + (a * kBins + lane) * 7;
+		uint32_t w[7];
+#pragma unroll
+		for (int k = 0; k < 7; ++k)
+			w[k] = word(a, k);
 		Box6 p{ord2f(w[0]), ord2f(w[1]), ord2f(w[2]), ord2f(w[3]), ord2f(w[4]), ord2f(w[5])};
 		uint32_t pc = w[6];
 		Box6 q = p;
@@ -332,7 +338,7 @@ __device__ __forceinline__ void write_parent_area(const SahArgs &A, uint32_t par
 }
 
 __device__ __forceinline__ uint32_t new_node(const SahArgs &A, uint32_t k) {
-	const uint32_t id = atomicAdd(&A.ctr[kCtrNodes], k);
+	const uint32_t id = atomicAdd(&A.ctr[kCtrNodesSah], k);
 	if (id + k > A.node_cap) {
 		flag(A.err);
 		return kNone;
@@ -340,27 +346,38 @@ __device__ __forceinline__ uint32_t new_node(const SahArgs &A, uint32_t k) {
 	return id;
 }
 
-// Files a child range as a task of the right tier (called by one lane).  `frame` gives
-// the binning frame of a large child, a task of `level`.  Returns the list slot of a large
-// child, which the calling warp then makes ready (open_large), else kNone.
-__device__ uint32_t add_child(const SahArgs &A, int level, uint32_t begin, uint32_t count,
-                              uint32_t node, uint32_t parent, uint32_t buf, uint32_t depth,
-                              const Box6 *frame, const float *pflo, const float *pfsc) {
+// A place in the list of the tier that a range of `count` triangles belongs to (large tasks by
+// level); kNone, flagged, when the list is full.
+__device__ __forceinline__ uint32_t list_slot(const SahArgs &A, int level, uint32_t count) {
+	const bool large = count > kLarge, mid = !large && count > kSmall;
+	const uint32_t word = large ? kCtrLarge + level : (mid ? kCtrMid : kCtrSmall);
+	const uint32_t cap = large ? A.max_large : (mid ? A.max_mid : A.max_small);
+	const uint32_t i = atomicAdd(&A.ctr[word], 1u);
+	if (i < cap)
+		return i;
+	flag(A.err);
+	return kNone;
+}
+
+// Writes a child range as a task into place `i` of its tier's list.  `frame` gives the binning
+// frame of a large child (null: its parent's).
+__device__ __forceinline__ void put_child(const SahArgs &A, int level, uint32_t i, uint32_t begin,
+                                          uint32_t count, uint32_t node, uint32_t parent,
+                                          uint32_t buf, uint32_t depth, const Box6 *frame,
+                                          const float *pflo, const float *pfsc) {
+	if (count <= kSmall) {
+		A.small[i] = SmallTask{begin, count | (buf << 8) | (depth << 16), node, parent, kNone};
+		return;
+	}
+	SahTask t;
+	memset(&t, 0, sizeof(t));
+	t.begin = begin;
+	t.count = count;
+	t.node = node;
+	t.parent = parent;
+	t.meta = buf | (depth << 8);
 	if (count > kLarge) {
-		const uint32_t i = atomicAdd(&A.ctr[kCtrLarge + level], 1u);
-		if (i >= A.max_large) {
-			flag(A.err);
-			return kNone;
-		}
-		SahTask t;
-		t.begin = begin;
-		t.count = count;
-		t.node = node;
-		t.parent = parent;
-		t.meta = buf | (depth << 8);
 		t.axis = kHalves;
-		t.split = 0;
-		t.n_left = 0;
 		if (frame) {
 			t.lo[0] = frame->lx;
 			t.lo[1] = frame->ly;
@@ -374,48 +391,23 @@ __device__ uint32_t add_child(const SahArgs &A, int level, uint32_t begin, uint3
 				t.scale[k] = pfsc[k];
 			}
 		}
-		t.cur_l = t.cur_r = 0;
 		A.large[level & 1][i] = t;
-		return i;
-	} else if (count > kSmall) {
-		const uint32_t i = atomicAdd(&A.ctr[kCtrMid], 1u);
-		if (i >= A.max_mid) {
-			flag(A.err);
-			return kNone;
-		}
-		SahTask t;
-		memset(&t, 0, sizeof(t));
-		t.begin = begin;
-		t.count = count;
-		t.node = node;
-		t.parent = parent;
-		t.meta = buf | (depth << 8);
-		A.mid[i] = t;
 	} else {
-		const uint32_t i = atomicAdd(&A.ctr[kCtrSmall], 1u);
-		if (i >= A.max_small) {
-			flag(A.err);
-			return kNone;
-		}
-		A.small[i] = SmallTask{begin, count | (buf << 8) | (depth << 16), node, parent, kNone};
+		A.mid[i] = t;
 	}
-	return kNone;
 }
 
-// Makes a large task filed by lane 0 (its slot and range) ready for its level: the whole warp
-// clears its bins (a single lane clearing the 672 words of two children took most of
-// k_sah_split's time) and lists its chunks.
-__device__ __forceinline__ void open_large(const SahArgs &A, int level, uint32_t slot,
-                                           uint32_t begin, uint32_t count, int lane) {
-	slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
+// Makes a large task that lane `from` filed (its slot and first chunk place) ready for its
+// level: the whole warp clears its bins (a single lane clearing the 672 words of two children
+// took most of k_sah_split's time) and lists its chunks.
+__device__ __forceinline__ void open_large(const SahArgs &A, int level, uint32_t slot, uint32_t at,
+                                           uint32_t begin, uint32_t count, int from, int lane) {
+	slot = __shfl_sync(0xFFFFFFFFu, slot, from);
+	at = __shfl_sync(0xFFFFFFFFu, at, from);
 	if (slot == kNone)
 		return;
 	bins_init(A.bins[level & 1] + (size_t)slot * kBinWords, lane, 32);
 	const uint32_t n = (count + kChunk - 1) / kChunk;
-	uint32_t at = 0;
-	if (lane == 0)
-		at = atomicAdd(&A.ctr[kCtrChunks + level], n);
-	at = __shfl_sync(0xFFFFFFFFu, at, 0);
 	if (at + n > A.max_chunks) {
 		if (lane == 0)
 			flag(A.err);
@@ -425,47 +417,55 @@ __device__ __forceinline__ void open_large(const SahArgs &A, int level, uint32_t
 		A.chunk[level & 1][at + c] = make_uint2(slot, begin + c * kChunk);
 }
 
-// Writes node `t.node` (box, children, range) for split `s` and files both children
-// (lane 0 only).  Children whose range holds one triangle are leaves.  slots[] receive
-// the list slots of children filed as large tasks (kNone otherwise).
-__device__ void emit_split(const SahArgs &A, const SahTask &t, const Split &s, int level,
-                           const float *flo, const float *fsc, uint32_t slots[2]) {
+// Writes node `t.node` (box, children, range) for split `s` of a large task and files its
+// children, lane 0 the left one and lane 1 the right one; children whose range holds one
+// triangle are leaves.  Lanes 0 and 1 return the list slot of a child filed as a large task
+// (else kNone).
+__device__ __forceinline__ uint32_t file_children(const SahArgs &A, const SahTask &t,
+                                                  const Split &s, int level, int lane) {
 	const uint32_t buf = (t.meta & 1u) ^ 1u, depth = ((t.meta >> 8) & 0xFFu) + 1u;
-	const uint32_t nl = s.n_left, nr = t.count - s.n_left;
-	slots[0] = slots[1] = kNone;
-	if (nl == 0 || nl >= t.count || t.node == kNone || t.node >= A.node_cap) {
-		flag(A.err);
-		return;
-	}
+	const uint32_t nl = s.n_left, nr = t.count - nl;
 	const bool binned = s.axis != kHalves;
-	uint32_t ids[2] = {kNone, kNone};
-	const uint32_t need = (nl > 1) + (nr > 1);
-	if (need) {
-		const uint32_t id = new_node(A, need);
-		if (id == kNone)
-			return;
-		uint32_t k = 0;
-		if (nl > 1)
-			ids[0] = id + k++;
-		if (nr > 1)
-			ids[1] = id + k;
+	const bool right = lane == 1, mine = lane < 2;
+	const uint32_t begin = right ? t.begin + nl : t.begin, count = right ? nr : nl;
+	const uint32_t n_ids = (nl > 1) + (nr > 1);
+	// Every atomic of the task before any of their results is needed.
+	uint32_t id = 0, slot = kNone, at = 0;
+	if (lane == 2 && n_ids)
+		id = new_node(A, n_ids);
+	if (mine && count > kLarge)
+		at = atomicAdd(&A.ctr[kCtrChunks + level], (count + kChunk - 1) / kChunk);
+	if (mine)
+		slot = list_slot(A, level, count);
+	id = __shfl_sync(0xFFFFFFFFu, id, 2);
+	if (id == kNone || !__all_sync(0xFFFFFFFFu, !mine || slot != kNone))
+		return kNone; // (flagged)
+	const uint32_t id_l = id, id_r = id + (nl > 1 ? 1u : 0u);
+	if (mine) {
+		const uint32_t node = count > 1 ? (right ? id_r : id_l) : kNone;
+		// Children's areas: known now for a binned split (leaves keep -1); after halves each
+		// child writes its own when it is split.
+		const uint32_t parent = binned ? kNone : ((t.node << 1) | (right ? 1u : 0u));
+		Box6 frame{t.lo[0], t.lo[1], t.lo[2], 0.0f, 0.0f, 0.0f};
+		if (binned)
+			frame = right ? s.right : s.left;
+		put_child(A, level, slot, begin, count, node, parent, buf, depth, binned ? &frame : nullptr,
+		          t.lo, t.scale);
+		if (!right) {
+			A.left[t.node] = nl > 1 ? id_l : (kLeafBit | t.begin);
+			A.right[t.node] = nr > 1 ? id_r : (kLeafBit | (t.begin + nl));
+			A.rfirst[t.node] = t.begin;
+			A.rlast[t.node] = t.begin + t.count - 1u;
+			A.splits[t.begin + nl - 1u] = make_uint4(t.begin, t.begin + t.count - 1u, t.node, 0u);
+			write_node_box(A, t.node, s.node, (binned && nl > 1) ? box_area(s.left) : -1.0f,
+			               (binned && nr > 1) ? box_area(s.right) : -1.0f);
+		}
 	}
-	const uint32_t rl = nl > 1 ? ids[0] : (kLeafBit | t.begin);
-	const uint32_t rr = nr > 1 ? ids[1] : (kLeafBit | (t.begin + nl));
-	A.left[t.node] = rl;
-	A.right[t.node] = rr;
-	A.rfirst[t.node] = t.begin;
-	A.rlast[t.node] = t.begin + t.count - 1u;
-	A.splits[t.begin + nl - 1u] = make_uint4(t.begin, t.begin + t.count - 1u, t.node, 0u);
-	// Children's areas: known now for a binned split (leaves keep -1); after halves each
-	// child writes its own when it is split.
-	write_node_box(A, t.node, s.node, (binned && nl > 1) ? box_area(s.left) : -1.0f,
-	               (binned && nr > 1) ? box_area(s.right) : -1.0f);
-	const uint32_t pl = binned ? kNone : (t.node << 1), pr = binned ? kNone : ((t.node << 1) | 1u);
-	slots[0] = add_child(A, level, t.begin, nl, ids[0], pl, buf, depth,
-	                     binned ? &s.left : nullptr, flo, fsc);
-	slots[1] = add_child(A, level, t.begin + nl, nr, ids[1], pr, buf, depth,
-	                     binned ? &s.right : nullptr, flo, fsc);
+	if (count <= kLarge)
+		slot = kNone;
+	open_large(A, level, slot, at, t.begin, nl, 0, lane);
+	open_large(A, level, slot, at, t.begin + nl, nr, 1, lane);
+	return slot;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -555,7 +555,7 @@ __global__ void k_sah_records(const float *__restrict__ tris, uint32_t n,
 	}
 }
 
-__global__ void k_sah_first_id(uint32_t *ctr, uint32_t S) { ctr[kCtrNodes] = S; }
+__global__ void k_sah_first_id(uint32_t *ctr, uint32_t S) { ctr[kCtrNodesSah] = S; }
 
 // One warp per scene: lane 0 files the root task, the warp clears a large root's bins.
 __global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uint32_t n_scenes,
@@ -565,7 +565,7 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uin
 	if (s >= n_scenes)
 		return;
 	const uint32_t b = tri_off[s], n = tri_off[s + 1] - b;
-	uint32_t slot = kNone;
+	uint32_t slot = kNone, at = 0;
 	if (lane == 0) {
 		roots[s] = s;
 		if (n) {
@@ -575,10 +575,14 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uin
 				flo[k] = ord2f(gb[6 * s + k]);
 				fsc[k] = frame_scale(flo[k], ord2f(gb[6 * s + 3 + k]));
 			}
-			slot = add_child(A, 0, b, n, n > 1 ? s : kNone, kNone, 0u, 0u, nullptr, flo, fsc);
+			if (n > kLarge)
+				at = atomicAdd(&A.ctr[kCtrChunks], (n + kChunk - 1) / kChunk);
+			slot = list_slot(A, 0, n);
+			if (slot != kNone)
+				put_child(A, 0, slot, b, n, n > 1 ? s : kNone, kNone, 0u, 0u, nullptr, flo, fsc);
 		}
 	}
-	open_large(A, 0, slot, b, n, lane);
+	open_large(A, 0, n > kLarge ? slot : kNone, at, b, n, 0, lane);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -615,55 +619,59 @@ __global__ void __launch_bounds__(256) k_sah_bin(SahArgs A) {
 	}
 }
 
-// One warp per large task: the plane, the node and the child tasks.
+// One warp per large task: the plane, the node and the child tasks.  A level has few tasks, so
+// the launch takes as long as one warp's chain of dependent reads and atomics: the bins of
+// all axes are read at once, and lanes 0 and 1 file one child each while lane 2 draws the
+// node ids (10 -> 7.5 us per level).
 __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
 	const uint32_t n_tasks = n_large(A, level);
 	const int lane = threadIdx.x & 31;
 	for (uint32_t ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ti < n_tasks;
 	     ti += (gridDim.x * blockDim.x) >> 5) {
 		SahTask &tr = A.large[level & 1][ti];
+		const uint32_t *b = A.bins[level & 1] + (size_t)ti * kBinWords;
+		uint32_t w[3][7];
+#pragma unroll
+		for (int a = 0; a < 3; ++a)
+#pragma unroll
+			for (int k = 0; k < 7; ++k)
+				w[a][k] = b[(a * kBins + lane) * 7 + k];
 		const SahTask t = tr;
 		if (!range_ok(A, t.begin, t.count)) {
 			if (lane == 0)
 				flag(A.err);
 			continue;
 		}
-		const uint32_t *b = A.bins[level & 1] + (size_t)ti * kBinWords;
-		float flo[3], fsc[3];
-		for (int k = 0; k < 3; ++k) {
-			flo[k] = t.lo[k];
-			fsc[k] = t.scale[k];
-		}
-		Split s = choose_split(b, fsc, t.count, lane);
-		uint32_t slots[2] = {kNone, kNone};
-		uint32_t total = b[lane * 7 + 6]; // the axis-0 bins hold every triangle once
-		for (int o = 16; o > 0; o >>= 1)
-			total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
+		Split s = choose_split([&](int a, int k) { return w[a][k]; }, t.scale, t.count, lane);
+		const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, w[0][6]); // every triangle once
 		if (((t.meta >> 8) & 0xFFu) >= kDepthGuard) {
 			s.axis = kHalves;
 			s.n_left = t.count / 2;
 		}
-		if (lane == 0 && total != t.count) {
+		uint32_t slot = kNone; // lanes 0, 1: the child's list slot when it is a large task
+		if (total != t.count || s.n_left == 0 || s.n_left >= t.count || t.node >= A.node_cap) {
 			// Nothing placed: the partition then writes no triangle of this task.
-			flag(A.err);
-			tr.axis = kHalves;
-			tr.n_left = 0;
-			tr.cur_l = tr.cur_r = A.n;
-		} else if (lane == 0) {
-			write_parent_area(A, t.parent, box_area(s.node));
-			tr.axis = s.axis;
-			tr.split = s.bin;
-			tr.n_left = s.n_left;
-			tr.cur_l = t.begin;
-			tr.cur_r = t.begin + s.n_left;
-			emit_split(A, t, s, level + 1, flo, fsc, slots);
+			if (lane == 0) {
+				flag(A.err);
+				tr.axis = kHalves;
+				tr.n_left = 0;
+				tr.cur_l = tr.cur_r = A.n;
+			}
+		} else {
+			slot = file_children(A, t, s, level + 1, lane);
+			if (lane == 0) {
+				write_parent_area(A, t.parent, box_area(s.node));
+				tr.axis = s.axis;
+				tr.split = s.bin;
+				tr.n_left = s.n_left;
+				tr.cur_l = t.begin;
+				tr.cur_r = t.begin + s.n_left;
+			}
 		}
-		if (lane == 0) {
-			tr.node = slots[0];
-			tr.parent = slots[1];
-		}
-		open_large(A, level + 1, slots[0], t.begin, s.n_left, lane);
-		open_large(A, level + 1, slots[1], t.begin + s.n_left, t.count - s.n_left, lane);
+		if (lane == 0)
+			tr.node = slot;
+		if (lane == 1)
+			tr.parent = slot;
 	}
 }
 
@@ -673,7 +681,8 @@ __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
 // level is bound by the latency of its few dependent steps and by the shared-memory bins.
 // As two kernels, each reading every record, with a pair of atomics per 32 triangles and a
 // chunk table built by a third, a level of the 1,048,576-triangle heightfield took 60 to 90
-// us; now 33 to 64.
+// us; now 33 to 64.  (The split of the children in a task's last block, without a launch of
+// its own: 53 us per level against 38 + 10, with its fences and 80 registers.)
 __global__ void __launch_bounds__(256) k_sah_part(SahArgs A, int level) {
 	__shared__ uint32_t sb[2 * kBinWords];
 	__shared__ uint32_t cnt_l[8 * kPer], cnt_r[8 * kPer]; // per warp and j; then exclusive sums
@@ -888,7 +897,8 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 	team_sync(team, warp);
 	Split s;
 	if (warp == lead) {
-		s = choose_split(sb, fsc, r.count, lane);
+		s = choose_split([&](int a, int k) { return sb[(a * kBins + lane) * 7 + k]; }, fsc, r.count,
+		                 lane);
 		if (r.depth >= kDepthGuard) {
 			s.axis = kHalves;
 			s.n_left = r.count / 2;
@@ -1008,8 +1018,12 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 	}
 }
 
-__global__ void __launch_bounds__(32 * kMidWarps) k_sah_mid(SahArgs A) {
+// (level: the first that was not launched; large tasks left there mean that the trees are not
+// ready for this tier yet.)
+__global__ void __launch_bounds__(32 * kMidWarps) k_sah_mid(SahArgs A, int level) {
 	__shared__ MidShared S;
+	if (n_large(A, level))
+		return;
 	const uint32_t n_tasks = min(A.ctr[kCtrMid], A.max_mid);
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	for (uint32_t ti = blockIdx.x; ti < n_tasks; ti += gridDim.x) {
@@ -1112,7 +1126,9 @@ __device__ __forceinline__ void write_small_node(const SahArgs &A, uint32_t node
 	               nr > 1 ? box_area(rb) : -1.0f);
 }
 
-__global__ void __launch_bounds__(128) k_sah_small(SahArgs A) {
+__global__ void __launch_bounds__(128) k_sah_small(SahArgs A, int level) {
+	if (n_large(A, level))
+		return;
 	__shared__ float4 stage_all[4][2 * 32]; // the task's boxes, by lane
 	__shared__ uint8_t order_all[4][32];    // a sweep's order: the lane of each position
 	const uint32_t n_tasks = min(A.ctr[kCtrSmall], A.max_small);
@@ -1334,6 +1350,14 @@ __global__ void __launch_bounds__(128) k_sah_small(SahArgs A) {
 	}
 }
 
+// What the stages after the binary trees may rely on: every node id handed out was written
+// (the collapse follows the children) and no check failed; else they do nothing.
+__global__ void k_sah_gate(SahArgs A, int level, uint32_t want, uint32_t *gate) {
+	*gate = n_large(A, level)                                            ? kGateLevels
+	        : ((*A.err & kErrSah) || A.ctr[kCtrNodesSah] != want) ? kGateError
+	                                                              : 0u;
+}
+
 __global__ void k_sah_bounds_init(uint32_t *gb, uint32_t n_scenes) {
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 * n_scenes;
 	     i += gridDim.x * blockDim.x)
@@ -1344,32 +1368,25 @@ inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 
 
 struct Layout {
 	size_t max_large, max_mid, max_small, max_chunks;
-	size_t off[12];
+	size_t off[11];
 	size_t total;
 };
 
-// Regions of the scratch, 256-byte aligned: records x2, then per parity large tasks,
-// bins and chunks, then mid tasks, small tasks and counters.
+// Regions of the scratch, 256-byte aligned: records, bins, large tasks and chunks (two each),
+// then mid tasks, small tasks and counters.
 Layout layout(uint32_t n, uint32_t S) {
 	Layout L;
 	L.max_large = n / (kLarge + 1) + S + 1;
 	L.max_mid = n / (kSmall + 1) + S + 1;
 	L.max_small = (size_t)n + S + 1;
 	L.max_chunks = n / kChunk + L.max_large;
-	const size_t sz[12] = {32ull * n,
-	                       32ull * n,
-	                       64 * L.max_large,
-	                       4ull * kBinWords * L.max_large,
-	                       8 * L.max_chunks,
-	                       64 * L.max_large,
-	                       4ull * kBinWords * L.max_large,
-	                       8 * L.max_chunks,
-	                       64 * L.max_mid,
-	                       sizeof(SmallTask) * L.max_small,
-	                       4 * kCtrWordsSah,
-	                       0};
+	const size_t bins = 4ull * kBinWords * L.max_large, large = sizeof(SahTask) * L.max_large,
+	             chunks = 8 * L.max_chunks;
+	const size_t sz[11] = {32ull * n, 32ull * n, bins,   bins, large, large, chunks, chunks,
+	                       sizeof(SahTask) * L.max_mid, sizeof(SmallTask) * L.max_small,
+	                       4 * kCtrWordsSah};
 	size_t at = 0;
-	for (int k = 0; k < 12; ++k) {
+	for (int k = 0; k < 11; ++k) {
 		L.off[k] = at;
 		at += (sz[k] + 255) & ~size_t(255);
 	}
@@ -1381,23 +1398,21 @@ Layout layout(uint32_t n, uint32_t S) {
 
 size_t sah_scratch_bytes(uint32_t n, uint32_t S) { return layout(n, S).total; }
 
-int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &ws,
-                      const uint32_t *d_toff, const uint32_t *scene_of, cudaStream_t st,
-                      uint32_t *d_err, std::string &msg) {
+namespace {
+
+// The kernels' arguments over the reserved scratch; false when it is too small.
+bool sah_args(const BuildPlan &plan, BuildScratch &ws, uint32_t *d_err, Layout &L, SahArgs &A) {
 	const uint32_t n = plan.n, S = plan.S;
-	const Layout L = layout(n, S);
-	if (ws.sah.bytes < L.total || ws.roots.bytes < 4ull * S) {
-		msg = "sah build: scratch not reserved";
-		return PRT_ERR_DEVICE;
-	}
+	L = layout(n, S);
+	if (ws.sah.bytes < L.total || ws.roots.bytes < 4ull * S)
+		return false;
 	char *p = ws.sah.as<char>();
-	SahArgs A;
 	A.rec[0] = reinterpret_cast<float4 *>(p + L.off[0]);
 	A.rec[1] = reinterpret_cast<float4 *>(p + L.off[1]);
 	for (int k = 0; k < 2; ++k) {
-		A.large[k] = reinterpret_cast<SahTask *>(p + L.off[2 + 3 * k]);
-		A.bins[k] = reinterpret_cast<uint32_t *>(p + L.off[3 + 3 * k]);
-		A.chunk[k] = reinterpret_cast<uint2 *>(p + L.off[4 + 3 * k]);
+		A.bins[k] = reinterpret_cast<uint32_t *>(p + L.off[2 + k]);
+		A.large[k] = reinterpret_cast<SahTask *>(p + L.off[4 + k]);
+		A.chunk[k] = reinterpret_cast<uint2 *>(p + L.off[6 + k]);
 	}
 	A.mid = reinterpret_cast<SahTask *>(p + L.off[8]);
 	A.small = reinterpret_cast<SmallTask *>(p + L.off[9]);
@@ -1417,7 +1432,48 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	A.max_chunks = (uint32_t)L.max_chunks;
 	A.n = n;
 	A.err = d_err;
+	return true;
+}
 
+void launch_levels(const SahArgs &A, const BuildPlan &plan, const Layout &L, int &level, int count,
+                   cudaStream_t st) {
+	for (int k = 0; k < count && level < kMaxLevels; ++k, ++level) {
+		// Grids no larger than the work the level can hold: each task has at most two
+		// children, so level L has at most S * 2^L tasks (a small scene's levels are then a
+		// few blocks each instead of 1216 idle ones).
+		const uint64_t tasks =
+		    std::min<uint64_t>((uint64_t)plan.S << std::min(level, 30), L.max_large);
+		const unsigned grid = (unsigned)std::min<uint64_t>(1216, plan.n / kChunk + tasks);
+		k_sah_split<<<(unsigned)std::min<uint64_t>(304, (tasks + 3) / 4), 128, 0, st>>>(A, level);
+		k_sah_part<<<grid, 256, 0, st>>>(A, level);
+	}
+}
+
+// The mid and small tiers and the gate, after large levels 0 .. level - 1.
+void launch_tail(const SahArgs &A, const BuildPlan &plan, const Layout &L, int level,
+                 uint32_t *gate, cudaStream_t st) {
+	k_sah_mid<<<(unsigned)std::min<size_t>(1216, L.max_mid), 32 * kMidWarps, 0, st>>>(A, level);
+	k_sah_small<<<2432, 128, 0, st>>>(A, level);
+	uint64_t want = plan.S;
+	for (uint32_t s = 0; s < plan.S; ++s) {
+		const uint32_t ns = plan.toff[s + 1] - plan.toff[s];
+		want += ns >= 2 ? ns - 2 : 0;
+	}
+	k_sah_gate<<<1, 1, 0, st>>>(A, level, (uint32_t)want, gate);
+}
+
+} // namespace
+
+int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &ws,
+                      const uint32_t *d_toff, const uint32_t *scene_of, cudaStream_t st,
+                      uint32_t *d_err, uint32_t *gate, int &level, std::string &msg) {
+	const uint32_t n = plan.n, S = plan.S;
+	Layout L;
+	SahArgs A;
+	if (!sah_args(plan, ws, d_err, L, A)) {
+		msg = "sah build: scratch not reserved";
+		return PRT_ERR_DEVICE;
+	}
 	uint32_t *gb = ws.bounds.as<uint32_t>();
 	cudaMemsetAsync(A.ctr, 0, 4 * kCtrWordsSah, st);
 	k_sah_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S);
@@ -1426,74 +1482,50 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	k_sah_first_id<<<1, 1, 0, st>>>(A.ctr, S);
 	k_sah_roots<<<blocks_for(32ull * S, 128), 128, 0, st>>>(A, d_toff, S, gb,
 	                                                        ws.roots.as<uint32_t>());
-	// Before the first look at the level counters (a host wait): as many levels as halving
-	// splits need to bring the largest scene under the large-task size, since a split
-	// leaves at least one triangle on each side and most leave about half.
+	// As many levels as halving splits need to bring the largest scene under the large-task
+	// size, and two more, since splits are uneven (an empty level costs about 2 us, a look at
+	// the counters a host wait of about 10); sah_build_more takes up what is left.
 	uint32_t biggest = 0;
 	for (uint32_t sc = 0; sc < S; ++sc)
 		biggest = std::max(biggest, plan.toff[sc + 1] - plan.toff[sc]);
 	int ahead = 0;
 	for (uint64_t c = biggest; c > kLarge; c = (c + 1) / 2)
 		++ahead;
+	level = 0;
 	if (ahead) {
 		k_sah_bin<<<(unsigned)std::min<size_t>(1216, L.max_chunks), 256, 0, st>>>(A);
-		ahead += 2;
+		launch_levels(A, plan, L, level, ahead + 2, st);
 	}
-	for (int level = 0; ahead;) {
-		for (int k = 0; k < ahead && level < kMaxLevels; ++k, ++level) {
-			// Grids no larger than the work the level can hold: each task has at most two
-			// children, so level L has at most S * 2^L tasks (a small scene's levels are then
-			// a few blocks each instead of 1216 idle ones).
-			const uint64_t tasks = std::min<uint64_t>((uint64_t)S << std::min(level, 30), L.max_large);
-			const unsigned g_chunk = (unsigned)std::min<uint64_t>(1216, n / kChunk + tasks);
-			const unsigned g_split = (unsigned)std::min<uint64_t>(304, (tasks + 3) / 4);
-			k_sah_split<<<g_split, 128, 0, st>>>(A, level);
-			k_sah_part<<<g_chunk, 256, 0, st>>>(A, level);
+	launch_tail(A, plan, L, level, gate, st);
+	return PRT_OK;
+}
+
+int sah_build_more(const BuildPlan &plan, BuildScratch &ws, cudaStream_t st, uint32_t *d_err,
+                   uint32_t *gate, int &level, std::string &msg) {
+	Layout L;
+	SahArgs A;
+	if (!sah_args(plan, ws, d_err, L, A)) {
+		msg = "sah build: scratch not reserved";
+		return PRT_ERR_DEVICE;
+	}
+	for (;;) {
+		if (level >= kMaxLevels) {
+			msg = "sah build: more than " + std::to_string(kMaxLevels) + " levels";
+			return PRT_ERR_LIMIT;
 		}
-		uint32_t *h = ws.h_sah;
+		launch_levels(A, plan, L, level, kLevelsPerCheck, st);
 		cudaError_t e =
-		    cudaMemcpyAsync(h, A.ctr + kCtrLarge + level, 4, cudaMemcpyDeviceToHost, st);
+		    cudaMemcpyAsync(ws.h_sah, A.ctr + kCtrLarge + level, 4, cudaMemcpyDeviceToHost, st);
 		if (e == cudaSuccess)
 			e = cudaStreamSynchronize(st);
 		if (e != cudaSuccess) {
 			msg = std::string("sah build: ") + cudaGetErrorString(e);
 			return PRT_ERR_CUDA;
 		}
-		if (h[0] == 0)
+		if (ws.h_sah[0] == 0)
 			break;
-		if (level >= kMaxLevels) {
-			msg = "sah build: more than " + std::to_string(kMaxLevels) + " levels";
-			return PRT_ERR_LIMIT;
-		}
-		ahead = kLevelsPerCheck;
 	}
-	k_sah_mid<<<(unsigned)std::min<size_t>(1216, L.max_mid), 32 * kMidWarps, 0, st>>>(A);
-	k_sah_small<<<2432, 128, 0, st>>>(A);
-	// Every node id handed out must have been written before the collapse follows the
-	// children: check the error word and the node count first.
-	uint64_t want = S;
-	for (uint32_t s = 0; s < S; ++s) {
-		const uint32_t ns = plan.toff[s + 1] - plan.toff[s];
-		want += ns >= 2 ? ns - 2 : 0;
-	}
-	uint32_t *h = ws.h_sah, *h_errw = h + 4;
-	cudaError_t e = cudaMemcpyAsync(h, A.ctr, 16, cudaMemcpyDeviceToHost, st);
-	if (e == cudaSuccess)
-		e = cudaMemcpyAsync(h_errw, d_err, 4, cudaMemcpyDeviceToHost, st);
-	if (e == cudaSuccess)
-		e = cudaStreamSynchronize(st);
-	const uint32_t h_err = *h_errw;
-	if (e != cudaSuccess) {
-		msg = std::string("sah build: ") + cudaGetErrorString(e);
-		return PRT_ERR_CUDA;
-	}
-	if ((h_err & kErrSah) || h[kCtrNodes] != want) {
-		cudaMemsetAsync(d_err, 0, 4, st);
-		cudaStreamSynchronize(st);
-		msg = "sah build: internal check failed (nodes " + std::to_string(h[kCtrNodes]) +
-		      " of " + std::to_string(want) + ")";
-		return PRT_ERR_DEVICE;
-	}
+	launch_tail(A, plan, L, level, gate, st);
 	return PRT_OK;
 }
 

@@ -82,3 +82,32 @@ def test_scenes_across_the_tiers(gpu_backend, oracle_lib):
             _same(got[s].view(lay.numpy_dtype()), oracle_lib.brute_force(t, rays))
     finally:
         batch.close()
+
+
+@pytest.mark.parametrize("n,ratio", [(3000, 1.01), (12_000, 1.003), (40_000, 1.001)])
+def test_more_levels_than_halving(gpu_backend, oracle_lib, n, ratio):
+    """Triangles at geometric distances: every split cuts off a few percent, so the trees need
+    many more large levels than are queued before the first look at the counters.  The scene
+    built before it is another one, so nothing left over from it may show."""
+    rng = np.random.default_rng(n)
+    x = ratio ** np.arange(n)
+    t = rng.uniform(-0.3, 0.3, (n, 3, 3)) * x[:, None, None]
+    t[:, :, 0] += x[:, None]
+    tris = t.reshape(n, 9).astype(np.float32)
+    k = rng.integers(n, size=600)
+    o = np.stack([x[k], rng.uniform(-2, 2, 600) * x[k], 3 * x[k]], 1)
+    d = tris.reshape(-1, 3, 3).mean(1)[k] - o
+    rays = np.concatenate([o, d / np.linalg.norm(d, axis=1, keepdims=True)], 1).astype(np.float32)
+    want = oracle_lib.brute_force(tris, rays)
+    assert (want["valid"] != 0).sum() > 300
+    try:
+        gpu_backend.set_option("build_small", 0)
+        for first in (W.soup_tris(1, 2 * n), tris):
+            gpu_backend.set_tris(first)
+        for leaf in (1, 4):
+            gpu_backend.set_option("leaf_size", leaf)
+            gpu_backend.set_tris(tris)
+            _same(gpu_backend.nearest_hits(rays, hitreg.TAGS), want)
+    finally:
+        gpu_backend.set_option("build_small", 1)
+        gpu_backend.set_option("leaf_size", 1)
