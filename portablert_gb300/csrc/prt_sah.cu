@@ -683,7 +683,9 @@ __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
 // chunk table built by a third, a level of the 1,048,576-triangle heightfield took 60 to 90
 // us; now 33 to 64.  (The split of the children in a task's last block, without a launch of
 // its own: 53 us per level against 38 + 10, with its fences and 80 registers.)
-__global__ void __launch_bounds__(256) k_sah_part(SahArgs A, int level) {
+// (Four blocks per SM: 64 registers; with 76, three blocks, a heightfield build took 1.72 ms
+// where it takes 1.62.)
+__global__ void __launch_bounds__(256, 4) k_sah_part(SahArgs A, int level) {
 	__shared__ uint32_t sb[2 * kBinWords];
 	__shared__ uint32_t cnt_l[8 * kPer], cnt_r[8 * kPer]; // per warp and j; then exclusive sums
 	__shared__ uint32_t base[2];
