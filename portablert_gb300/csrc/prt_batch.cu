@@ -290,12 +290,8 @@ int prt_b200_batch_set_tris_dev(prt_b200_batch *b, const float *d_tris, const ui
 		b->build_ms = ev.elapsed_ms();
 		if (rc != PRT_OK)
 			return bfail(ctx, rc, msg);
-		uint32_t err_word = 0;
-		B_TRY(ctx, cudaMemcpy(&err_word, ctx->d_err(), 4, cudaMemcpyDeviceToHost));
-		if (err_word) {
-			cudaMemset(ctx->d_err(), 0, 4);
+		if (ctx->take_err()) // (the build has been waited for)
 			return bfail(ctx, PRT_ERR_DEVICE, "batch build: kernel reported an error");
-		}
 		if ((int)b->arena.depth > prt::traversal_stack_depth())
 			return bfail(ctx, PRT_ERR_LIMIT, "batch build: tree too deep for the traversal");
 		rc = scene_tables(b);
@@ -439,12 +435,8 @@ int prt_b200_batch_sync(prt_b200_batch *b) {
 		rc = prt::build_finish(b->arena, b->ws, ctx->stream, msg);
 		if (rc != PRT_OK)
 			return bfail(ctx, rc, msg);
-		uint32_t err_word = 0;
-		B_TRY(ctx, cudaMemcpy(&err_word, ctx->d_err(), 4, cudaMemcpyDeviceToHost));
-		if (err_word) {
-			cudaMemset(ctx->d_err(), 0, 4);
+		if (ctx->take_err()) // (the build has been waited for)
 			return bfail(ctx, PRT_ERR_DEVICE, "batch build: kernel reported an error");
-		}
 		b->graph_dirty = false;
 	}
 	return PRT_OK;

@@ -97,6 +97,8 @@ __global__ void k_scene_of(const uint32_t *tri_off, uint32_t n_scenes, uint32_t 
 			scene_of[i] = s;
 }
 
+__global__ void k_clear_word(uint32_t *word) { *word = 0u; }
+
 // Empty bounds, and no split after each scene's last leaf.
 __global__ void k_bounds_init(uint32_t *gb, uint32_t n_scenes, const uint32_t *tri_off,
                               uint4 *splits) {
@@ -1398,7 +1400,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 	int rc = collapse_enqueue(d_tris, plan, sc, ws, svals, roots, st, d_err, host_checks, msg);
 	while (rc == PRT_OK && plan.sah && ws.h_counters[kCtrGate] != 0) {
 		if (ws.h_counters[kCtrGate] != kGateLevels) {
-			BUILD_TRY(cudaMemsetAsync(d_err, 0, 4, st));
+			k_clear_word<<<1, 1, 0, st>>>(d_err); // (reported here)
 			BUILD_TRY(cudaStreamSynchronize(st));
 			msg = "sah build: internal check failed";
 			return PRT_ERR_DEVICE;

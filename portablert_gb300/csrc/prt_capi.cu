@@ -61,13 +61,9 @@ bool cc_ok(int dev) {
 }
 
 int check_device_errors(prt_b200_ctx *ctx) {
-	CAPI_TRY(ctx, cudaMemcpyAsync(ctx->h_err, ctx->d_err(), 4, cudaMemcpyDeviceToHost,
-	                              ctx->stream));
 	CAPI_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-	uint32_t e = *ctx->h_err;
+	const uint32_t e = ctx->take_err();
 	if (e) {
-		cudaMemsetAsync(ctx->d_err(), 0, 4, ctx->stream);
-		cudaStreamSynchronize(ctx->stream);
 		std::string m = "kernel reported:";
 		if (e & prt::kErrStack)
 			m += " traversal stack overflow;";
@@ -294,7 +290,11 @@ int prt_b200_create(int device, prt_b200_ctx **out) {
 	if (e == cudaSuccess)
 		e = cudaMemset(ctx->work.p, 0, 64);
 	if (e == cudaSuccess)
-		e = cudaMallocHost(&ctx->h_err, 16);
+		e = cudaHostAlloc(&ctx->h_err, 16, cudaHostAllocMapped);
+	if (e == cudaSuccess) {
+		*ctx->h_err = 0u;
+		e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->err_dev), ctx->h_err, 0);
+	}
 	if (e == cudaSuccess)
 		e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
 	if (e == cudaSuccess)
@@ -545,7 +545,6 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 				if (ctx->count)
 					CAPI_TRY(ctx, cudaMemcpyAsync(ctx->visits, ctx->d_visits(), 16,
 					                              cudaMemcpyDeviceToHost, ctx->stream));
-				// One wait: the error word's copy is queued after the traversal.
 				return check_device_errors(ctx);
 			}
 		}

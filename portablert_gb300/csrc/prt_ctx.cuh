@@ -49,7 +49,7 @@ struct prt_b200_ctx {
 	prt::BuildScratch ws;
 	prt::DevBuf tris_in;
 	prt::DevBuf rays_buf, out_buf;
-	prt::DevBuf work; // [0..3] ray counter, [4..7] error word, [8..15] deferred-pass
+	prt::DevBuf work; // [0..3] ray counter, [8..15] deferred-pass
 	                  // words, [16..31] visit counters, [32..47] ray counter and deferred
 	                  // words of the second compute stream, [48..51] the read probe's sink
 	// The host-buffer call splits large batches into chunks and overlaps the copy-in of a
@@ -69,7 +69,9 @@ struct prt_b200_ctx {
 		uint32_t *counter;
 	};
 	std::vector<QueryStream> query_streams;
-	uint32_t *h_err = nullptr;
+	uint32_t *h_err = nullptr, *err_dev = nullptr; // error word of the context's kernels: pinned
+	                 // host memory that they set bits of, so the host reads it after its wait
+	                 // without a copy (4 us of every host-buffer query and build)
 	int leaf_size = 1;
 	int node_format = PRT_NODES_FP32;
 	int block = 128;
@@ -92,7 +94,9 @@ struct prt_b200_ctx {
 	unsigned long long visits[2] = {0, 0};
 
 	uint32_t *d_work() { return work.as<uint32_t>(); }
-	uint32_t *d_err() { return work.as<uint32_t>() + 1; }
+	uint32_t *d_err() { return err_dev; }
+	// The bits set so far; they start again at zero.
+	uint32_t take_err() { return __atomic_exchange_n(h_err, 0u, __ATOMIC_SEQ_CST); }
 	unsigned long long *d_visits() {
 		return reinterpret_cast<unsigned long long *>(work.as<uint8_t>() + 16);
 	}
