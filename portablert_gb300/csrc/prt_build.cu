@@ -35,6 +35,7 @@
 #include "../../include/prt_b200.h"
 #include "prt_build.cuh"
 #include "prt_collapse.cuh"
+#include "prt_launch.cuh"
 #include "prt_sah.cuh"
 
 namespace prt {
@@ -447,6 +448,7 @@ __device__ __forceinline__ void up_child(const UpShared &S, uint16_t ref, float4
 // triangles 13.4 -> 12.7 ms; the batch's graph 10.95 -> 10.38 ms).
 template <bool REFIT, bool COST>
 __global__ void __launch_bounds__(kUpLeaves) k_bottom_up(UpArgs A) {
+	chain_enter(); // (launched as usual: only lets k_walk_up be scheduled)
 	__shared__ UpShared S;
 	const uint32_t b0 = blockIdx.x * kUpLeaves, t = threadIdx.x, i = b0 + t;
 	if (A.gate && *A.gate)
@@ -570,6 +572,7 @@ __global__ void __launch_bounds__(kUpLeaves) k_bottom_up(UpArgs A) {
 // because a block of k_bottom_up kept its place for the longest of its walks.
 template <bool REFIT, bool COST>
 __global__ void __launch_bounds__(128) k_walk_up(UpArgs A) {
+	chain_enter();
 	const uint32_t n = min(*A.n_walks, A.walk_cap);
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
 		uint4 at = A.splits[A.walks[k]];
@@ -633,13 +636,14 @@ __device__ __forceinline__ bool is_inner(uint32_t r, uint32_t count, uint32_t le
 		return false;
 	if (count > leaf_size)
 		return true;
-	return cost ? (__ldg(&cost[r].bits) >> 31) == 0u : false;
+	return cost ? (cost[r].bits >> 31) == 0u : false;
 }
 
 // Level-0 frontier: the root of every scene becomes 8-wide node s; the node counter
 // starts after the roots.
 __global__ void k_collapse_roots(const uint32_t *tri_off, const uint32_t *int_off,
                                  uint32_t n_scenes, Item *items, uint32_t *ctr) {
+	chain_enter();
 	const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
 	if (s == 0) {
 		ctr[0] = ctr[kCtrGate] ? 0u : n_scenes; // (incomplete trees: no items, no levels)
@@ -652,7 +656,7 @@ __global__ void k_collapse_roots(const uint32_t *tri_off, const uint32_t *int_of
 	items[s] = Item{ref, s};
 }
 
-__device__ __forceinline__ float open_area(uint32_t r, const float4 *__restrict__ ibox) {
+__device__ __forceinline__ float open_area(uint32_t r, const float4 *ibox) {
 	return (r & kLeafBit) ? -1.0f : half_area(ibox[2 * r], ibox[2 * r + 1]);
 }
 
@@ -834,8 +838,9 @@ constexpr uint32_t kCollapseItems = 32; // frontier items per block (8 lanes eac
 // Builds: 65,790-triangle heightfield 0.89 -> 0.80 ms, 1,048,576 triangles 2.32 -> 2.17 ms; the
 // batch's collapse, compression and records 926 -> 702 us.
 __global__ void __launch_bounds__(8 * kCollapseItems)
-    k_collapse(CollapseArgs A, const Item *__restrict__ in, const uint32_t *in_count, Item *out,
+    k_collapse(CollapseArgs A, const Item *in, const uint32_t *in_count, Item *out,
                uint32_t *out_count) {
+	chain_enter();
 	__shared__ uint32_t xch[8 * kCollapseItems]; // per item: what each child slot receives
 	__shared__ uint32_t need[kCollapseItems];    // per item: inner children | triangles << 16
 	__shared__ uint32_t got[3];                  // the block's nodes, triangles, items
@@ -863,9 +868,8 @@ __global__ void __launch_bounds__(8 * kCollapseItems)
 				uint32_t give = kNone, a = 0;
 				if (span > 1u && !(y & kLeafBit)) {
 					const CostNode *cn = A.cost + y;
-					const uint32_t bits = __ldg(&cn->bits), l = __ldg(&A.left[y]),
-					               r = __ldg(&A.right[y]);
-					const float one = __ldg(&cn->c1), open = __ldg(&cn->cd[span - 2u]);
+					const uint32_t bits = cn->bits, l = A.left[y], r = A.right[y];
+					const float one = cn->c1, open = cn->cd[span - 2u];
 					if (round == 0 || open < one) {
 						a = split_of(bits, span);
 						give = r;
@@ -959,19 +963,19 @@ __global__ void __launch_bounds__(8 * kCollapseItems)
 			const bool single = (y & kLeafBit) != 0u;
 			const uint32_t id = y & ~kLeafBit;
 			const float4 *src = single ? A.lbox + 2 * (size_t)id : A.ibox + 2 * (size_t)id;
-			const float4 l = __ldg(src), h = __ldg(src + 1);
+			const float4 l = *src, h = src[1];
 			lo[0] = l.x;
 			lo[1] = l.y;
 			lo[2] = l.z;
 			hi[0] = h.x;
 			hi[1] = h.y;
 			hi[2] = h.z;
-			first = single ? id : __ldg(&A.rfirst[id]);
-			cnt = single ? 1u : __ldg(&A.rlast[id]) - first + 1u;
+			first = single ? id : A.rfirst[id];
+			cnt = single ? 1u : A.rlast[id] - first + 1u;
 			inner = is_inner(y, cnt, A.leaf_size, A.cost);
 		}
 		const bool leaf = has && !inner;
-		const uint32_t g0 = leaf ? __ldg(&A.vals[first]) : 0u;
+		const uint32_t g0 = leaf ? A.vals[first] : 0u;
 		const uint32_t inners = (__ballot_sync(0xFFFFFFFFu, inner) >> gsh) & 0xFFu;
 		const uint32_t my_tris = leaf ? cnt : 0u;
 		uint32_t sum = my_tris;
@@ -1030,8 +1034,8 @@ __global__ void __launch_bounds__(8 * kCollapseItems)
 				write_cnode(A.cnodes, it.slot, live, gmask, c8, ref, lo, hi);
 			if (leaf)
 				for (uint32_t j = 0; j < cnt; ++j, ++dst) {
-					const uint32_t g = j == 0 ? g0 : __ldg(&A.vals[first + j]);
-					const uint32_t pid = A.scene_of ? g - __ldg(&A.tri_off[A.scene_of[g]]) : g;
+					const uint32_t g = j == 0 ? g0 : A.vals[first + j];
+					const uint32_t pid = A.scene_of ? g - A.tri_off[A.scene_of[g]] : g;
 					const float *t = A.tris + 9 * (size_t)g;
 					A.inv[g] = dst;
 					float4 *to = A.tri4 + 3 * (size_t)dst;
@@ -1276,19 +1280,20 @@ static int collapse_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU
 		const unsigned g_walk = std::min(1216u, blocks_for(n, 128));
 		if (plan.sah) {
 			k_bottom_up<false, true><<<grid, kUpLeaves, 0, st>>>(U);
-			k_walk_up<false, true><<<g_walk, 128, 0, st>>>(U);
+			launch_after(host_checks, k_walk_up<false, true>, g_walk, 128, st, U);
 		} else if (use_cost) {
 			k_bottom_up<true, true><<<grid, kUpLeaves, 0, st>>>(U);
-			k_walk_up<true, true><<<g_walk, 128, 0, st>>>(U);
+			launch_after(host_checks, k_walk_up<true, true>, g_walk, 128, st, U);
 		} else {
 			k_bottom_up<true, false><<<grid, kUpLeaves, 0, st>>>(U);
-			k_walk_up<true, false><<<g_walk, 128, 0, st>>>(U);
+			launch_after(host_checks, k_walk_up<true, false>, g_walk, 128, st, U);
 		}
 	}
 	const CostNode *cost = use_cost ? ws.cost.as<CostNode>() : nullptr;
 
 	Item *items_of[2] = {ws.items_a.as<Item>(), ws.items_b.as<Item>()};
-	k_collapse_roots<<<blocks_for(S, 128), 128, 0, st>>>(d_toff, roots, S, items_of[0], ctr);
+	launch_after(host_checks, k_collapse_roots, blocks_for(S, 128), 128, st, d_toff, roots, S,
+	             items_of[0], ctr);
 	CollapseArgs A;
 	A.tris = d_tris;
 	A.vals = svals;
@@ -1330,9 +1335,9 @@ static int collapse_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU
 			    std::min<uint64_t>((uint64_t)S << std::min(3 * level, 30), plan.node_cap);
 			const unsigned grid = (unsigned)std::min<uint64_t>(
 			    1216, (items + kCollapseItems - 1) / kCollapseItems);
-			k_collapse<<<grid, 8 * kCollapseItems, 0, st>>>(A, items_of[level & 1], ctr + level,
-			                                                items_of[(level + 1) & 1],
-			                                                ctr + level + 1);
+			launch_after(host_checks, k_collapse, grid, 8 * kCollapseItems, st, A,
+			             items_of[level & 1], ctr + level, items_of[(level + 1) & 1],
+			             ctr + level + 1);
 		}
 		if (!host_checks)
 			break;

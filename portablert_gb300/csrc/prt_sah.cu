@@ -29,6 +29,7 @@
 
 #include "../../include/prt_b200.h"
 #include "prt_build.cuh"
+#include "prt_launch.cuh"
 #include "prt_sah.cuh"
 
 namespace prt {
@@ -472,7 +473,8 @@ __device__ __forceinline__ uint32_t file_children(const SahArgs &A, const SahTas
 // Set-up: records, per-scene centre bounds, root tasks.
 
 __global__ void k_sah_records(const float *__restrict__ tris, uint32_t n,
-                              const uint32_t *__restrict__ scene_of, float4 *rec, uint32_t *gb) {
+                              const uint32_t *scene_of, float4 *rec, uint32_t *gb) {
+	chain_enter();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int lane = threadIdx.x & 31;
 	const bool live = i < n;
@@ -555,11 +557,15 @@ __global__ void k_sah_records(const float *__restrict__ tris, uint32_t n,
 	}
 }
 
-__global__ void k_sah_first_id(uint32_t *ctr, uint32_t S) { ctr[kCtrNodesSah] = S; }
+__global__ void k_sah_first_id(uint32_t *ctr, uint32_t S) {
+	chain_enter();
+	ctr[kCtrNodesSah] = S;
+}
 
 // One warp per scene: lane 0 files the root task, the warp clears a large root's bins.
-__global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uint32_t n_scenes,
-                            const uint32_t *__restrict__ gb, uint32_t *roots) {
+__global__ void k_sah_roots(SahArgs A, const uint32_t *tri_off, uint32_t n_scenes,
+                            const uint32_t *gb, uint32_t *roots) {
+	chain_enter();
 	const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
 	if (s >= n_scenes)
@@ -590,6 +596,7 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *__restrict__ tri_off, uin
 
 // The roots' bins (the bins of later levels are filled by the partition above them).
 __global__ void __launch_bounds__(256) k_sah_bin(SahArgs A) {
+	chain_enter();
 	__shared__ uint32_t sb[kBinWords];
 	const uint32_t n = n_chunks(A, 0);
 	const int lane = threadIdx.x & 31;
@@ -624,6 +631,7 @@ __global__ void __launch_bounds__(256) k_sah_bin(SahArgs A) {
 // all axes are read at once, and lanes 0 and 1 file one child each while lane 2 draws the
 // node ids (10 -> 7.5 us per level).
 __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
+	chain_enter();
 	const uint32_t n_tasks = n_large(A, level);
 	const int lane = threadIdx.x & 31;
 	for (uint32_t ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ti < n_tasks;
@@ -686,6 +694,7 @@ __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
 // (Four blocks per SM: 64 registers; with 76, three blocks, a heightfield build took 1.72 ms
 // where it takes 1.62.)
 __global__ void __launch_bounds__(256, 4) k_sah_part(SahArgs A, int level) {
+	chain_enter();
 	__shared__ uint32_t sb[2 * kBinWords];
 	__shared__ uint32_t cnt_l[8 * kPer], cnt_r[8 * kPer]; // per warp and j; then exclusive sums
 	__shared__ uint32_t base[2];
@@ -1023,6 +1032,7 @@ __device__ __forceinline__ void split_range(const SahArgs &A, MidShared &S, cons
 // (level: the first that was not launched; large tasks left there mean that the trees are not
 // ready for this tier yet.)
 __global__ void __launch_bounds__(32 * kMidWarps) k_sah_mid(SahArgs A, int level) {
+	chain_enter();
 	__shared__ MidShared S;
 	if (n_large(A, level))
 		return;
@@ -1129,6 +1139,7 @@ __device__ __forceinline__ void write_small_node(const SahArgs &A, uint32_t node
 }
 
 __global__ void __launch_bounds__(128) k_sah_small(SahArgs A, int level) {
+	chain_enter();
 	if (n_large(A, level))
 		return;
 	__shared__ float4 stage_all[4][2 * 32]; // the task's boxes, by lane
@@ -1355,6 +1366,7 @@ __global__ void __launch_bounds__(128) k_sah_small(SahArgs A, int level) {
 // What the stages after the binary trees may rely on: every node id handed out was written
 // (the collapse follows the children) and no check failed; else they do nothing.
 __global__ void k_sah_gate(SahArgs A, int level, uint32_t want, uint32_t *gate) {
+	chain_enter();
 	*gate = n_large(A, level)                                            ? kGateLevels
 	        : ((*A.err & kErrSah) || A.ctr[kCtrNodesSah] != want) ? kGateError
 	                                                              : 0u;
@@ -1446,22 +1458,24 @@ void launch_levels(const SahArgs &A, const BuildPlan &plan, const Layout &L, int
 		const uint64_t tasks =
 		    std::min<uint64_t>((uint64_t)plan.S << std::min(level, 30), L.max_large);
 		const unsigned grid = (unsigned)std::min<uint64_t>(1216, plan.n / kChunk + tasks);
-		k_sah_split<<<(unsigned)std::min<uint64_t>(304, (tasks + 3) / 4), 128, 0, st>>>(A, level);
-		k_sah_part<<<grid, 256, 0, st>>>(A, level);
+		const unsigned splits = (unsigned)std::min<uint64_t>(304, (tasks + 3) / 4);
+		launch_after(true, k_sah_split, splits, 128, st, A, level);
+		launch_after(true, k_sah_part, grid, 256, st, A, level);
 	}
 }
 
 // The mid and small tiers and the gate, after large levels 0 .. level - 1.
 void launch_tail(const SahArgs &A, const BuildPlan &plan, const Layout &L, int level,
                  uint32_t *gate, cudaStream_t st) {
-	k_sah_mid<<<(unsigned)std::min<size_t>(1216, L.max_mid), 32 * kMidWarps, 0, st>>>(A, level);
-	k_sah_small<<<2432, 128, 0, st>>>(A, level);
+	const unsigned mids = (unsigned)std::min<size_t>(1216, L.max_mid);
+	launch_after(true, k_sah_mid, mids, 32 * kMidWarps, st, A, level);
+	launch_after(true, k_sah_small, 2432, 128, st, A, level);
 	uint64_t want = plan.S;
 	for (uint32_t s = 0; s < plan.S; ++s) {
 		const uint32_t ns = plan.toff[s + 1] - plan.toff[s];
 		want += ns >= 2 ? ns - 2 : 0;
 	}
-	k_sah_gate<<<1, 1, 0, st>>>(A, level, (uint32_t)want, gate);
+	launch_after(true, k_sah_gate, 1, 1, st, A, level, (uint32_t)want, gate);
 }
 
 } // namespace
@@ -1480,10 +1494,11 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	cudaMemsetAsync(A.ctr, 0, 4 * kCtrWordsSah, st);
 	k_sah_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S);
 	if (n)
-		k_sah_records<<<blocks_for(n, 256), 256, 0, st>>>(d_tris, n, scene_of, A.rec[0], gb);
-	k_sah_first_id<<<1, 1, 0, st>>>(A.ctr, S);
-	k_sah_roots<<<blocks_for(32ull * S, 128), 128, 0, st>>>(A, d_toff, S, gb,
-	                                                        ws.roots.as<uint32_t>());
+		launch_after(true, k_sah_records, blocks_for(n, 256), 256, st, d_tris, n, scene_of,
+		             A.rec[0], gb);
+	launch_after(true, k_sah_first_id, 1, 1, st, A.ctr, S);
+	launch_after(true, k_sah_roots, blocks_for(32ull * S, 128), 128, st, A, d_toff, S, gb,
+	             ws.roots.as<uint32_t>());
 	// As many levels as halving splits need to bring the largest scene under the large-task
 	// size, and two more, since splits are uneven (an empty level costs about 2 us, a look at
 	// the counters a host wait of about 10); sah_build_more takes up what is left.
@@ -1495,7 +1510,8 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 		++ahead;
 	level = 0;
 	if (ahead) {
-		k_sah_bin<<<(unsigned)std::min<size_t>(1216, L.max_chunks), 256, 0, st>>>(A);
+		const unsigned bins = (unsigned)std::min<size_t>(1216, L.max_chunks);
+		launch_after(true, k_sah_bin, bins, 256, st, A);
 		launch_levels(A, plan, L, level, ahead + 2, st);
 	}
 	launch_tail(A, plan, L, level, gate, st);
