@@ -81,7 +81,7 @@ __device__ __forceinline__ float lambert(const float4 &A, const float4 &B, const
 	              __fsub_rn(__fmul_rn(e1[0], e2[1]), __fmul_rn(e1[1], e2[0]))};
 	const float len = __fsqrt_rn(
 	    __fadd_rn(__fadd_rn(__fmul_rn(N[0], N[0]), __fmul_rn(N[1], N[1])), __fmul_rn(N[2], N[2])));
-	if ((double)fabsf(len) > 0.001) {
+	if (fabsf(len) >= 0.001f) { // (0.001f is the least float above the reference's double 0.001)
 		N[0] = __fdiv_rn(N[0], len);
 		N[1] = __fdiv_rn(N[1], len);
 		N[2] = __fdiv_rn(N[2], len);
