@@ -39,8 +39,16 @@ constexpr int kBins = 32;
 constexpr uint32_t kLarge = 512;    // larger tasks are binned by many blocks (512 / 1,024
                                     // / 4,096: heightfield build 3.05 / 3.16 / 3.83 ms)
 constexpr uint32_t kSmall = 32;     // tasks up to this size go to one warp each
-constexpr uint32_t kPer = 4;        // triangles per thread of a binning / partition block
-constexpr uint32_t kChunk = 256 * kPer; // triangles per such block
+// Triangles per thread of a binning / partition block (256 threads): chunks of 1,024, or of 512
+// or 256 where fewer than kSpread chunks, the partition blocks the chip holds, would leave
+// SMs without one.  Builds with 256 / 512 / 1,024, us: 16,384 triangles 396 / 411 / 429,
+// 65,790 465 / 482 / 505, 131,072 532 / 553 / 565, 262,144 843 / 817 / 856, 524,288 1126 /
+// 1079 / 1057, 1,048,576 - / 1629 / 1571.
+constexpr uint32_t kMaxPer = 4;
+constexpr uint32_t kSpread = 4 * 152;
+inline uint32_t tris_per_thread(uint32_t n) {
+	return n <= 256u * kSpread ? 1u : n <= 512u * kSpread ? 2u : kMaxPer;
+}
 constexpr uint32_t kDepthGuard = 48;
 constexpr int kMaxLevels = 96;
 constexpr int kLevelsPerCheck = 4;
@@ -93,8 +101,13 @@ struct SahArgs {
 	uint4 *splits;          // out: by leaf position, for the bottom-up cost pass
 	uint32_t node_cap, max_large, max_mid, max_small, max_chunks;
 	uint32_t n;             // triangles (records per buffer)
+	uint32_t chunk_log;     // log2 of the triangles per chunk, 256 * tris_per_thread
 	uint32_t *err;
 };
+
+__device__ __forceinline__ uint32_t chunks_of(const SahArgs &A, uint32_t count) {
+	return (count + (1u << A.chunk_log) - 1u) >> A.chunk_log;
+}
 
 // Counts clamped to the list capacities (a list that overflowed was flagged).
 __device__ __forceinline__ uint32_t n_large(const SahArgs &A, int level) {
@@ -408,14 +421,14 @@ __device__ __forceinline__ void open_large(const SahArgs &A, int level, uint32_t
 	if (slot == kNone)
 		return;
 	bins_init(A.bins[level & 1] + (size_t)slot * kBinWords, lane, 32);
-	const uint32_t n = (count + kChunk - 1) / kChunk;
+	const uint32_t n = chunks_of(A, count);
 	if (at + n > A.max_chunks) {
 		if (lane == 0)
 			flag(A.err);
 		return;
 	}
 	for (uint32_t c = lane; c < n; c += 32)
-		A.chunk[level & 1][at + c] = make_uint2(slot, begin + c * kChunk);
+		A.chunk[level & 1][at + c] = make_uint2(slot, begin + (c << A.chunk_log));
 }
 
 // Writes node `t.node` (box, children, range) for split `s` of a large task and files its
@@ -435,7 +448,7 @@ __device__ __forceinline__ uint32_t file_children(const SahArgs &A, const SahTas
 	if (lane == 2 && n_ids)
 		id = new_node(A, n_ids);
 	if (mine && count > kLarge)
-		at = atomicAdd(&A.ctr[kCtrChunks + level], (count + kChunk - 1) / kChunk);
+		at = atomicAdd(&A.ctr[kCtrChunks + level], chunks_of(A, count));
 	if (mine)
 		slot = list_slot(A, level, count);
 	id = __shfl_sync(0xFFFFFFFFu, id, 2);
@@ -582,7 +595,7 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *tri_off, uint32_t n_scene
 				fsc[k] = frame_scale(flo[k], ord2f(gb[6 * s + 3 + k]));
 			}
 			if (n > kLarge)
-				at = atomicAdd(&A.ctr[kCtrChunks], (n + kChunk - 1) / kChunk);
+				at = atomicAdd(&A.ctr[kCtrChunks], chunks_of(A, n));
 			slot = list_slot(A, 0, n);
 			if (slot != kNone)
 				put_child(A, 0, slot, b, n, n > 1 ? s : kNone, kNone, 0u, 0u, nullptr, flo, fsc);
@@ -595,6 +608,7 @@ __global__ void k_sah_roots(SahArgs A, const uint32_t *tri_off, uint32_t n_scene
 // Large tasks.
 
 // The roots' bins (the bins of later levels are filled by the partition above them).
+template <uint32_t kPer>
 __global__ void __launch_bounds__(256) k_sah_bin(SahArgs A) {
 	chain_enter();
 	__shared__ uint32_t sb[kBinWords];
@@ -603,7 +617,7 @@ __global__ void __launch_bounds__(256) k_sah_bin(SahArgs A) {
 	for (uint32_t c = blockIdx.x; c < n; c += gridDim.x) {
 		const uint2 ch = A.chunk[0][c];
 		const SahTask &t = A.large[0][ch.x];
-		const uint32_t end = min(ch.y + kChunk, t.begin + t.count);
+		const uint32_t end = min(ch.y + 256u * kPer, t.begin + t.count);
 		const float4 *src = A.rec[0];
 		float4 lo[kPer], hi[kPer];
 #pragma unroll
@@ -685,7 +699,7 @@ __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
 
 // Scatters the triangles of the large tasks to the other buffer, left side first, and adds
 // each to the bins of the child it goes to (when that is a large task).  A thread reads its
-// four triangles at once and the block reserves its places with one atomic per side: the
+// triangles (up to four) at once and the block reserves its places with one atomic per side: the
 // level is bound by the latency of its few dependent steps and by the shared-memory bins.
 // As two kernels, each reading every record, with a pair of atomics per 32 triangles and a
 // chunk table built by a third, a level of the 1,048,576-triangle heightfield took 60 to 90
@@ -693,12 +707,13 @@ __global__ void __launch_bounds__(128) k_sah_split(SahArgs A, int level) {
 // its own: 53 us per level against 38 + 10, with its fences and 80 registers.)
 // (Four blocks per SM: 64 registers; with 76, three blocks, a heightfield build took 1.72 ms
 // where it takes 1.62.)
+template <uint32_t kPer>
 __global__ void __launch_bounds__(256, 4) k_sah_part(SahArgs A, int level) {
 	chain_enter();
 	__shared__ uint32_t sb[2 * kBinWords];
 	__shared__ uint32_t cnt_l[8 * kPer], cnt_r[8 * kPer]; // per warp and j; then exclusive sums
 	__shared__ uint32_t base[2];
-	static_assert(8 * kPer == 32, "one warp scans the block's counts");
+	static_assert(8 * kPer <= 32, "one warp scans the block's counts");
 	const uint32_t n = n_chunks(A, level);
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const uint32_t lt = (1u << lane) - 1u;
@@ -707,7 +722,7 @@ __global__ void __launch_bounds__(256, 4) k_sah_part(SahArgs A, int level) {
 		SahTask &t = A.large[level & 1][ch.x];
 		const uint32_t begin = t.begin, count = t.count, nl = t.n_left, axis = t.axis,
 		               split = t.split, buf = t.meta & 1u;
-		const uint32_t end = min(ch.y + kChunk, begin + count);
+		const uint32_t end = min(ch.y + 256u * kPer, begin + count);
 		const uint32_t slot[2] = {t.node, t.parent};
 		const float4 *src = A.rec[buf];
 		float4 *dst = A.rec[buf ^ 1u];
@@ -743,7 +758,8 @@ __global__ void __launch_bounds__(256, 4) k_sah_part(SahArgs A, int level) {
 		__syncthreads();
 		if (warp < 2) { // warp 0 the left side, warp 1 the right
 			uint32_t *cnt = warp ? cnt_r : cnt_l;
-			const uint32_t own = cnt[lane];
+			const bool in = lane < 8 * (int)kPer;
+			const uint32_t own = in ? cnt[lane] : 0u;
 			uint32_t x = own;
 #pragma unroll
 			for (int o = 1; o < 32; o <<= 1) {
@@ -751,7 +767,8 @@ __global__ void __launch_bounds__(256, 4) k_sah_part(SahArgs A, int level) {
 				if (lane >= o)
 					x += y;
 			}
-			cnt[lane] = x - own;
+			if (in)
+				cnt[lane] = x - own;
 			if (lane == 31)
 				base[warp] = x ? atomicAdd(warp ? &t.cur_r : &t.cur_l, x) : 0u;
 		}
@@ -1393,7 +1410,8 @@ Layout layout(uint32_t n, uint32_t S) {
 	L.max_large = n / (kLarge + 1) + S + 1;
 	L.max_mid = n / (kSmall + 1) + S + 1;
 	L.max_small = (size_t)n + S + 1;
-	L.max_chunks = n / kChunk + L.max_large;
+	// (As many for n as for any smaller n: scratch reserved for a size serves those below.)
+	L.max_chunks = std::max(n / (256 * kMaxPer), std::min(n / 256, kSpread)) + L.max_large;
 	const size_t bins = 4ull * kBinWords * L.max_large, large = sizeof(SahTask) * L.max_large,
 	             chunks = 8 * L.max_chunks;
 	const size_t sz[11] = {32ull * n, 32ull * n, bins,   bins, large, large, chunks, chunks,
@@ -1445,6 +1463,8 @@ bool sah_args(const BuildPlan &plan, BuildScratch &ws, uint32_t *d_err, Layout &
 	A.max_small = (uint32_t)L.max_small;
 	A.max_chunks = (uint32_t)L.max_chunks;
 	A.n = n;
+	const uint32_t per = tris_per_thread(n);
+	A.chunk_log = per == 1u ? 8u : per == 2u ? 9u : 10u;
 	A.err = d_err;
 	return true;
 }
@@ -1457,10 +1477,14 @@ void launch_levels(const SahArgs &A, const BuildPlan &plan, const Layout &L, int
 		// few blocks each instead of 1216 idle ones).
 		const uint64_t tasks =
 		    std::min<uint64_t>((uint64_t)plan.S << std::min(level, 30), L.max_large);
-		const unsigned grid = (unsigned)std::min<uint64_t>(1216, plan.n / kChunk + tasks);
+		const unsigned grid = (unsigned)std::min<uint64_t>(1216, (plan.n >> A.chunk_log) + tasks);
 		const unsigned splits = (unsigned)std::min<uint64_t>(304, (tasks + 3) / 4);
 		launch_after(true, k_sah_split, splits, 128, st, A, level);
-		launch_after(true, k_sah_part, grid, 256, st, A, level);
+		launch_after(true,
+		             A.chunk_log == 8   ? k_sah_part<1>
+		             : A.chunk_log == 9 ? k_sah_part<2>
+		                                : k_sah_part<kMaxPer>,
+		             grid, 256, st, A, level);
 	}
 }
 
@@ -1511,7 +1535,11 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	level = 0;
 	if (ahead) {
 		const unsigned bins = (unsigned)std::min<size_t>(1216, L.max_chunks);
-		launch_after(true, k_sah_bin, bins, 256, st, A);
+		launch_after(true,
+		             A.chunk_log == 8   ? k_sah_bin<1>
+		             : A.chunk_log == 9 ? k_sah_bin<2>
+		                                : k_sah_bin<kMaxPer>,
+		             bins, 256, st, A);
 		launch_levels(A, plan, L, level, ahead + 2, st);
 	}
 	launch_tail(A, plan, L, level, gate, st);
