@@ -139,8 +139,9 @@ prt::TravConfig trav_config(const prt_b200_ctx *ctx) {
 #define MADV_POPULATE_WRITE 23
 #endif
 
-// Whether p is pageable memory of which some of a few sampled pages are not resident.  Small
-// buffers (a page or two, mostly from a heap in use) are not looked at.
+// Whether p is pageable memory of which some page is not resident, by one system call for
+// every kPagesAsked pages.  Small buffers (a page or two, mostly from a heap in use) are not
+// looked at.
 bool untouched_pages(const void *p, size_t bytes) {
 	if (bytes < (128u << 10))
 		return false;
@@ -152,13 +153,17 @@ bool untouched_pages(const void *p, size_t bytes) {
 	const long page = sysconf(_SC_PAGESIZE);
 	if (a.type != cudaMemoryTypeUnregistered || page <= 0 || bytes == 0)
 		return false;
+	constexpr size_t kPagesAsked = 4096;
+	unsigned char in[kPagesAsked];
 	const uintptr_t mask = ~(uintptr_t)(page - 1), at = reinterpret_cast<uintptr_t>(p);
-	constexpr int kSamples = 16;
-	for (int k = 0; k <= kSamples; ++k) {
-		const uintptr_t q = (at + (bytes - 1) / kSamples * k) & mask;
-		unsigned char in = 1;
-		if (mincore(reinterpret_cast<void *>(q), (size_t)page, &in) == 0 && !(in & 1))
-			return true;
+	const uintptr_t end = at + bytes;
+	for (uintptr_t q = at & mask; q < end; q += kPagesAsked * (size_t)page) {
+		const size_t pages = std::min<size_t>(kPagesAsked, (end - q + page - 1) / (size_t)page);
+		if (mincore(reinterpret_cast<void *>(q), pages * (size_t)page, in) != 0)
+			return false;
+		for (size_t k = 0; k < pages; ++k)
+			if (!(in[k] & 1))
+				return true;
 	}
 	return false;
 }
