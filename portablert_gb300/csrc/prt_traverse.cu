@@ -335,7 +335,8 @@ __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const
 			if (REGULAR || r.kind == 0)
 				hit = child_passes(q, a, b);
 			else
-				hit = conservative_box(r, child_lo(a.x, a.z), child_hi(a.x, a.z),
+				hit = conservative_box(r, child_lo_x(a.x, a.z, __float_as_uint(b.w)),
+				                       child_hi_x(a.x, a.z, __float_as_uint(b.w)),
 				                       child_lo(a.y, a.w), child_hi(a.y, a.w),
 				                       child_lo(b.x, b.y), child_hi(b.x, b.y));
 			// A node index, or a leaf's first triangle: both below 2^27, under the
