@@ -1120,6 +1120,7 @@ int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compre
 	sc.depth = 0;
 	sc.has_cnodes = false;
 	sc.built_small = false;
+	sc.x_log = 0;
 	sc.h_tri_off.assign(tri_off64, tri_off64 + S + 1);
 
 	const size_t key_bytes = plan.multi ? 8 : 4;
@@ -1152,6 +1153,14 @@ int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compre
 	if (sah && !plan.small) {
 		BUILD_TRY(ws.sah.reserve(sah_scratch_bytes(n, S)));
 		BUILD_TRY(ws.roots.reserve(4ull * S));
+	}
+	plan.x_log = 0;
+	if (sah && !plan.small && !plan.multi && n) {
+		uint32_t log = 10;
+		while ((1ull << log) < 8ull * n)
+			++log;
+		BUILD_TRY(sc.x_faces.reserve(4ull * (kXHead + (1ull << (log - 5u)))));
+		plan.x_log = log;
 	}
 	if (collapse_cost)
 		BUILD_TRY(ws.cost.reserve(sizeof(CostNode) * ni));
@@ -1392,8 +1401,9 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 	int sah_level = 0; // large levels of the SAH build queued so far
 	BUILD_TRY(cudaMemsetAsync(ctr, 0, 4 * kCtrWords, st));
 	if (plan.sah) {
-		int rc = sah_build_enqueue(d_tris, plan, ws, d_toff, scene_of, st, d_err, ctr + kCtrGate,
-		                           sah_level, msg);
+		const XFaces x_faces{sc.x_faces.as<uint32_t>(), plan.x_log};
+		int rc = sah_build_enqueue(d_tris, plan, ws, d_toff, scene_of, x_faces, st, d_err,
+		                           ctr + kCtrGate, sah_level, msg);
 		if (rc != PRT_OK)
 			return rc;
 		roots = ws.roots.as<uint32_t>();
@@ -1419,6 +1429,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 	if (rc != PRT_OK)
 		return rc;
 	sc.has_cnodes = plan.compressed;
+	sc.x_log = plan.x_log;
 	return host_checks ? build_finish(sc, ws, st, msg, true) : PRT_OK;
 }
 

@@ -67,6 +67,8 @@ struct SceneGPU {
 	DevBuf nodes;        // Node8[n_nodes], and the empty node at `dead`
 	DevBuf cnodes;       // CNode8[n_nodes], likewise
 	DevBuf tri_off;      // uint32[n_scenes + 1] (device copy)
+	DevBuf x_faces;      // XFaces words (SAH build of one scene)
+	uint32_t x_log = 0;  // log2 of its bits; 0: not built
 	std::vector<uint64_t> h_tri_off;
 	void release() {
 		tri4.release();
@@ -74,6 +76,8 @@ struct SceneGPU {
 		nodes.release();
 		cnodes.release();
 		tri_off.release();
+		x_faces.release();
+		x_log = 0;
 		h_tri_off.clear();
 		n_scenes = 0;
 		n_tris = 0;
@@ -119,6 +123,7 @@ struct BuildPlan {
 	uint32_t S = 0, n = 0, n_int = 0, node_cap = 0;
 	int leaf_size = 1, scene_digits = 0;
 	bool compressed = false, multi = false;
+	uint32_t x_log = 0;               // log2 of SceneGPU::x_faces' bits (0: not built)
 	bool sah = false;                 // binned-SAH binary trees instead of LBVH
 	bool collapse_cost = true;        // cost-optimal 8-wide collapse (else largest area first)
 	bool small = false;               // one scene of 1..small_build_max() triangles, with the

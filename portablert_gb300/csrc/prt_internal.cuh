@@ -118,6 +118,8 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 //              reciprocal); inner nodes use conservative_box below.
 //   2 all:     a non-finite component or all reciprocals infinite: every inner box
 //              passes and only the exact per-triangle test decides.
+//   3 free:    like 1 with a zero x component, and no triangle's box has its lower x face at
+//              the origin's x (XFaces): the x axis does not constrain a box around it.
 struct RayC {
 	float ox, oy, oz, dx, dy, dz, fx, fy, fz;
 	int kind;
@@ -203,6 +205,29 @@ __device__ __forceinline__ float child_hi_x(float c, float e, uint32_t x16) {
 	return fminf(child_hi(c, e), __uint_as_float(x16 & 0xFFFF0000u));
 }
 
+// Set of the x coordinates at which some triangle's box of a scene has its lower face: a
+// hash set of 2^log bits (8 to 16 per triangle) after kXHead words, of which the first is
+// set when a triangle is not finite.  log 0: there is no set, every x may be one.
+constexpr uint32_t kXHead = 4;
+struct XFaces {
+	uint32_t *words;
+	uint32_t log;
+};
+__device__ __forceinline__ uint32_t x_face_bit(float x, uint32_t log) {
+	return (__float_as_uint(__fadd_rn(x, 0.0f)) * 2654435761u) >> (32u - log); // (-0 as 0)
+}
+__device__ __forceinline__ void x_face_add(const XFaces &f, float x) {
+	const uint32_t k = x_face_bit(x, f.log), bit = 1u << (k & 31u);
+	uint32_t *w = f.words + kXHead + (k >> 5);
+	if (!(*(volatile uint32_t *)w & bit)) // (neighbours of a mesh share most of theirs)
+		atomicOr(w, bit);
+}
+// Whether no triangle's lower x face is at x.
+__device__ __forceinline__ bool x_face_free(const XFaces &f, float x) {
+	const uint32_t k = x_face_bit(x, f.log);
+	return __ldg(f.words) == 0u && !((__ldg(f.words + kXHead + (k >> 5)) >> (k & 31u)) & 1u);
+}
+
 // Slab test of portableRT's ray_box_intersect (bvh.hpp:195-222), bit for bit: each
 // t is (bound - origin) * reciprocal in round-to-nearest, combined with the select
 // min/max in the reference's nesting.  Used on every triangle's own bounding box.
@@ -243,7 +268,8 @@ __device__ __forceinline__ bool regular_box(const RayC &r, float lx, float hx, f
 // (-inf, +inf); origin exactly on the lower face -> NaN, which on the x axis makes the
 // whole reference test pass and on y or z removes that axis from it.  For an inner box
 // the same below/above answer holds for every box under it; otherwise the axis is
-// treated as unconstrained (y, z) or the box passes outright (x).
+// treated as unconstrained (y, z, and x of kind 3) or the box passes outright (x).  (On the
+// upper face the reference rejects, or accepts no more than it would without the axis.)
 __device__ __forceinline__ bool inf_axis(float o, float lo, float hi, float f, bool is_x, float &m,
                                          float &M) {
 	if (o < lo) {
@@ -265,7 +291,7 @@ __device__ __forceinline__ bool conservative_box(const RayC &r, float lx, float 
 		return true;
 	float m0, M0, m1, M1, m2, M2;
 	if (isinf(r.fx)) {
-		if (inf_axis(r.ox, lx, hx, r.fx, true, m0, M0))
+		if (inf_axis(r.ox, lx, hx, r.fx, r.kind != 3, m0, M0))
 			return true;
 	} else {
 		float a = (lx - r.ox) * r.fx, b = (hx - r.ox) * r.fx;

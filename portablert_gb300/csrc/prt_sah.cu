@@ -486,7 +486,8 @@ __device__ __forceinline__ uint32_t file_children(const SahArgs &A, const SahTas
 // Set-up: records, per-scene centre bounds, root tasks.
 
 __global__ void k_sah_records(const float *__restrict__ tris, uint32_t n,
-                              const uint32_t *scene_of, float4 *rec, uint32_t *gb) {
+                              const uint32_t *scene_of, float4 *rec, uint32_t *gb,
+                              XFaces x_faces) {
 	chain_enter();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int lane = threadIdx.x & 31;
@@ -507,6 +508,12 @@ __global__ void k_sah_records(const float *__restrict__ tris, uint32_t n,
 		} else {
 			lo = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, __uint_as_float(i));
 			hi = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
+		}
+		if (x_faces.log) {
+			if (fin)
+				x_face_add(x_faces, lo.x);
+			else
+				x_faces.words[0] = 1u;
 		}
 		rec[2 * (size_t)i] = lo;
 		rec[2 * (size_t)i + 1] = hi;
@@ -1389,7 +1396,13 @@ __global__ void k_sah_gate(SahArgs A, int level, uint32_t want, uint32_t *gate) 
 	                                                              : 0u;
 }
 
-__global__ void k_sah_bounds_init(uint32_t *gb, uint32_t n_scenes) {
+__global__ void k_sah_bounds_init(uint32_t *gb, uint32_t n_scenes, XFaces x_faces) {
+	if (x_faces.log) {
+		const uint32_t quads = (kXHead + (1u << (x_faces.log - 5u))) / 4u;
+		for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < quads;
+		     i += gridDim.x * blockDim.x)
+			reinterpret_cast<uint4 *>(x_faces.words)[i] = make_uint4(0u, 0u, 0u, 0u);
+	}
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 * n_scenes;
 	     i += gridDim.x * blockDim.x)
 		gb[i] = (i % 6) < 3 ? 0xFFFFFFFFu : 0u;
@@ -1505,8 +1518,9 @@ void launch_tail(const SahArgs &A, const BuildPlan &plan, const Layout &L, int l
 } // namespace
 
 int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &ws,
-                      const uint32_t *d_toff, const uint32_t *scene_of, cudaStream_t st,
-                      uint32_t *d_err, uint32_t *gate, int &level, std::string &msg) {
+                      const uint32_t *d_toff, const uint32_t *scene_of, XFaces x_faces,
+                      cudaStream_t st, uint32_t *d_err, uint32_t *gate, int &level,
+                      std::string &msg) {
 	const uint32_t n = plan.n, S = plan.S;
 	Layout L;
 	SahArgs A;
@@ -1516,10 +1530,13 @@ int sah_build_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch &
 	}
 	uint32_t *gb = ws.bounds.as<uint32_t>();
 	cudaMemsetAsync(A.ctr, 0, 4 * kCtrWordsSah, st);
-	k_sah_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S);
+	const uint64_t clear = x_faces.log ? 1ull << (x_faces.log - 5u) : 0u; // words
+	k_sah_bounds_init<<<std::max(blocks_for(6ull * S, 256),
+	                             std::min(blocks_for(clear / 4u, 256), 608u)),
+	                    256, 0, st>>>(gb, S, x_faces);
 	if (n)
 		launch_after(true, k_sah_records, blocks_for(n, 256), 256, st, d_tris, n, scene_of,
-		             A.rec[0], gb);
+		             A.rec[0], gb, x_faces);
 	launch_after(true, k_sah_first_id, 1, 1, st, A.ctr, S);
 	launch_after(true, k_sah_roots, blocks_for(32ull * S, 128), 128, st, A, d_toff, S, gb,
 	             ws.roots.as<uint32_t>());
