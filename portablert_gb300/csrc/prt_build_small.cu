@@ -185,7 +185,6 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *words, uint
 	return (warp ? words[32 + warp - 1] : 0u) + x - v;
 }
 
-// An 8-wide node's child record (an empty slot: NaN bounds and kNone).
 // Position i's nearest neighbour within kRadius positions among m clusters: the least
 // pair in the order (union area, distance, parity of the lower position, lower position;
 // the last three as fields of 4, 1 and 12 bits), a total order, so the loop's order does

@@ -13,7 +13,7 @@
 //
 // Tasks are ranges still to be split, in three tiers by size:
 //   large (> 512 triangles): level by level, one warp per task picks the plane from the
-//         task's 3 x 32 global bins (k_sah_split) and blocks scatter chunks of 1,024
+//         task's 3 x 32 global bins (k_sah_split) and blocks scatter chunks of 256 to 1,024
 //         triangles to the other buffer, adding each to the bins of the child it goes to
 //         (k_sah_part; k_sah_bin fills the roots' bins);
 //   mid   (33-512): one block per task, all its levels in shared memory (k_sah_mid);

@@ -31,7 +31,9 @@
 //    the others, and a deferred pass over those with the conservative test, for instance for
 //    zero direction components (it returns at once when there are none).  Camera queries and
 //    counting runs are one general launch, in which a batch of regular rays takes the
-//    plain test; camera batches start with a packet descent (packet_descent).  A request
+//    plain test; batches of large images of few triangles start with a packet descent
+//    (packet_descent).  Queries of up to some hundred rays per warp and other cameras are
+//    one launch as well (single_batch).  A request
 //    server's serving launch (pass 3) takes its batches from device queues that the host
 //    extends while it runs (claim_batch) and picks the plain or the general test per
 //    batch.
@@ -96,6 +98,7 @@ struct TravArgs {
 	uint32_t max_batches;    // batches per warp before it exits (0 = no bound)
 	uint32_t batch;          // rays a warp takes at a time: 32, or 16 / 8 for one small
 	                         // run (more warps busy, shorter chains per warp)
+	uint32_t claims;         // PASS 4: there are more batches than warps
 	uint32_t *counter;
 	uint32_t *deferred;      // [0] batches the regular pass left to the general one,
 	                         // [1] the deferred pass's batch counter
@@ -504,7 +507,7 @@ __device__ __forceinline__ void packet_descent(const TravArgs &a, const SceneDes
 	}
 }
 
-// (Small launches hold both box tests: 64 registers, which 8 blocks allow, spill nothing.)
+// (One-kernel launches hold both box tests: 64 registers, which 8 blocks allow, spill nothing.)
 #ifndef PRT_TRAVERSE_MIN_BLOCKS_SMALL
 #define PRT_TRAVERSE_MIN_BLOCKS_SMALL 8
 #endif
@@ -601,11 +604,12 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		// no position waits on the lane's previous child.  Pushed inner children go to
 		// the pool; with at most one triangle per hit leaf the queue positions come from
 		// the same ballots.
+		constexpr bool kOneArray = LEAF1 && FMT == PRT_NODES_FP32;
 		uint32_t pp[kChildPerLane], pq[kChildPerLane];
 		uint32_t ptop = top, qtop = q;
 #pragma unroll
 		for (int j = 0; j < kChildPerLane; ++j) {
-			if (LEAF1) {
+			if (kOneArray) {
 				// One place per hit child, in the pool or in the queue, which are one array:
 				// one population count and one store instead of two of each (heightfield
 				// 1,562 -> 1,521 us, 512-scene batch graph 10.42 -> 10.17 ms).
@@ -635,7 +639,7 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 			break;
 		}
 		const uint32_t hi = slot << kIndexBits;
-		if (LEAF1) {
+		if (kOneArray) {
 #pragma unroll
 			for (int j = 0; j < kChildPerLane; ++j)
 				if (hit[j])
@@ -764,8 +768,10 @@ __device__ __forceinline__ bool claim_batch(const ServeQueues &q, uint32_t held[
 // in the kernel at all: 8 % faster), the others counted in a.deferred and skipped; 2 =
 // the skipped batches with the general test (returns at once when there are none); 3 =
 // a serving launch: batches claimed from the serving queues (claim_batch), the plain or
-// the general test chosen per batch, descriptors and rays read around L1; 4 = a small launch
-// of one run: every batch, the test chosen per batch, without counters.
+// the general test chosen per batch, descriptors and rays read around L1; 4 = one kernel for
+// a run of up to some hundred rays per warp, and for most cameras (single_batch): every
+// batch, the test chosen per batch, a warp's first batch by its number and the next ones,
+// if any, from the counter.
 template <int FMT, bool COUNT, bool LEAF1, bool BOUNDED, int PASS>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_MIN_BLOCKS_SMALL
                                                        : FMT == PRT_NODES_FP32
@@ -804,8 +810,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				++S.batches;
 		}
 		// Batches are taken in order from a counter (the deferred pass has its own, so
-		// the few batches it works on spread over all warps); a small launch deals them
-		// out by warp; a serving launch claims them from its queues.
+		// the few batches it works on spread over all warps); a one-kernel launch (4)
+		// deals out the first ones by warp; a serving launch claims them from its queues.
 		uint32_t base = 0;
 		const SegDesc *segs = a.segs;
 		if (PASS == 3) {
@@ -837,8 +843,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 			}
 		} else {
 			if (PASS == 4) {
-				base = dealt;
-				dealt += gridDim.x * (blockDim.x >> 5) * a.batch;
+				base = dealt; // the warp's first batch
+				dealt = kNone;
+				if (base == kNone) { // the next one that no warp has
+					if (!a.claims)
+						break;
+					if (lane == 0)
+						base = atomicAdd(a.counter, a.batch) +
+						       gridDim.x * (blockDim.x >> 5) * a.batch;
+					base = __shfl_sync(0xFFFFFFFFu, base, 0);
+				}
 			} else {
 				if (lane == 0)
 					base = atomicAdd(PASS == 2 ? a.deferred + 1 : a.counter, a.batch);
@@ -1092,41 +1106,71 @@ int warps_for(const TravConfig &cfg) {
 	           : kWarpsPerBlock;
 }
 
-// A launch of one run with at most 32 rays per resident warp (155,648 on 152 SMs): one kernel,
-// no counters, batches of 4 rays while every warp gets at most one, else of 8, dealt out by
-// warp.  The two passes cost two memsets and a second launch more, which is most of a small
-// query, and a warp's serial chain is shorter with fewer rays.  Measured (back to back, us;
-// 4,096-triangle soup / 65,790-triangle heightfield / 1M clustered triangles):
-//     rays       two passes        4 per batch       8                16
-//     1,000      26 / 23 / 36      13 / 12 / 23      18 / 15 / 29     28 / 25 / 39
-//     8,192      26 / 68 / 41      15 / 31 / 25      19 / 43 / 33     29 / 60 / 45
-//     32,768     37 / 79 / 55      29 / 35 / 45      25 / 43 / 45     33 / 68 / 62
-//     65,536     52 / 39 / 65      48 / 28 / 68      45 / 31 / 61     44 / 44 / 68
-//     131,072    87 / 48 / 101     92 / 43 / 119     81 / 39 / 107    84 / 50 / 103
-//     200,000    116 / 65 / 137    138 / 62 / 174    119 / 55 / 148   117 / 56 / 144
-constexpr uint32_t kSmallPerWarp = 32;
+// Rays per batch of a one-kernel launch (PASS 4), by the rays per resident warp (4,864 warps on
+// 152 SMs); 0: too many, the two passes or the camera's packets take it.  The two passes
+// cost a second launch, their batches of 32 make long serial chains, and a batch deferred for
+// one zero direction component starts when all others are done; but with the plain test alone
+// they need fewer registers, which pays in the end.
+//
+// Ray buffers.  One round of batches while 8 rays a warp suffice, else batches claimed from
+// the counter.  Speed against a regular and a deferred pass (mean over five scenes / least of
+// them; FP32 nodes, one triangle per leaf), batches of 8, 16, 32:
+//     30,000     1.34 / 1.16    0.95 / 0.88    0.66 / 0.54
+//     100,000    1.09 / 1.01    0.93 / 0.90    0.77 / 0.67
+//     300,000    1.08 / 0.98    1.03 / 0.96    0.92 / 0.88
+//     600,000    1.38 / 0.92    1.38 / 0.97    1.25 / 0.95
+//     1,300,000  1.33 / 0.95    1.41 / 0.97    1.34 / 0.96
+//     2,000,000  1.11 / 0.93    1.22 / 0.95    1.23 / 0.95
+// (the means above 1.2 come from rays with zero components).  With compressed nodes or
+// larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.
+//
+// Cameras.  The packet descent (batches of 32) pays where a triangle covers many pixels and
+// there are enough batches.  Batches of 8 / 16 / 32 / packets, us:
+//     triangles  900 x 600                1600 x 900               2048 x 2048
+//     256        75 / 60 / 59 / 61        166 / 119 / 103 / 96     440 / 299 / 239 / 210
+//     4,968      105 / 110 / 140 / 148    207 / 171 / 183 / 183    515 / 383 / 332 / 311
+//     65,536     202 / 218 / 277 / 287    284 / 274 / 288 / 294    638 / 514 / 464 / 472
+uint32_t single_batch(const TravArgs &a, const TravConfig &cfg, uint64_t slots) {
+	const uint64_t n = a.n_virtual, per = (n + slots - 1) / slots;
+	if (per <= 8u)
+		return ((uint32_t)per + 3u) & ~3u;
+	if (a.use_cam) {
+		const bool wide = n >= 640ull * a.scene0.n_tris;
+		if (wide)
+			return per <= 32u ? 8u : per <= 120u ? 16u : 0u;
+		return per <= 120u ? 8u : per <= 450u ? 16u : 32u;
+	}
+	if (per <= 64u)
+		return 8u;
+	const bool plain = cfg.format == PRT_NODES_FP32 && a.max_leaf <= 1u;
+	return per <= (plain ? 420u : 130u) ? 16u : 0u;
+}
 
 template <int FMT, bool LEAF1>
-bool launch_small(TravArgs a, int warps, int sm_count, cudaStream_t st) {
+bool launch_single(TravArgs a, const TravConfig &cfg, int warps, int sm_count, cudaStream_t st) {
 	const uint64_t slots = (uint64_t)sm_count * warps *
 	                       blocks_per_sm<FMT, false, LEAF1, false, 4>(warps, a.warp_bytes);
-	const uint64_t per = (a.n_virtual + slots - 1) / slots;
-	if (per > kSmallPerWarp)
+	a.batch = single_batch(a, cfg, slots);
+	if (!a.batch)
 		return false;
-	a.batch = per <= 4u ? 4u : 8u;
+	a.claims = (uint64_t)a.batch * slots < a.n_virtual ? 1u : 0u;
+	if (a.claims && cudaMemsetAsync(a.counter, 0, 4, st) != cudaSuccess)
+		return true; // (dispatch reports the error)
 	launch_t<FMT, false, LEAF1, false, 4>(a, warps, sm_count, st);
 	return true;
 }
 
-bool try_small(const TravArgs &a, const TravConfig &cfg, int warps, int sm_count,
-               cudaStream_t st) {
-	if (a.n_segs || a.use_cam || cfg.count || a.max_batches)
+// Whether one kernel took the launch: of one run, not counting, not bounded.
+bool try_single(const TravArgs &a, const TravConfig &cfg, int warps, int sm_count,
+                cudaStream_t st) {
+	if (a.n_segs || cfg.count || (a.max_batches && !a.use_cam))
 		return false;
 	if (cfg.format == PRT_NODES_COMPRESSED)
-		return a.max_leaf <= 1u ? launch_small<PRT_NODES_COMPRESSED, true>(a, warps, sm_count, st)
-		                        : launch_small<PRT_NODES_COMPRESSED, false>(a, warps, sm_count, st);
-	return a.max_leaf <= 1u ? launch_small<PRT_NODES_FP32, true>(a, warps, sm_count, st)
-	                        : launch_small<PRT_NODES_FP32, false>(a, warps, sm_count, st);
+		return a.max_leaf <= 1u
+		           ? launch_single<PRT_NODES_COMPRESSED, true>(a, cfg, warps, sm_count, st)
+		           : launch_single<PRT_NODES_COMPRESSED, false>(a, cfg, warps, sm_count, st);
+	return a.max_leaf <= 1u ? launch_single<PRT_NODES_FP32, true>(a, cfg, warps, sm_count, st)
+	                        : launch_single<PRT_NODES_FP32, false>(a, cfg, warps, sm_count, st);
 }
 
 template <int FMT, bool LEAF1>
@@ -1179,11 +1223,10 @@ uint32_t batch_rays(uint64_t m, int sm_count, uint32_t max_batches) {
 
 cudaError_t dispatch(const TravArgs &a, const TravConfig &cfg, int sm_count, cudaStream_t st) {
 	const int warps = warps_for(cfg);
-	if (try_small(a, cfg, warps, sm_count, st))
+	if (try_single(a, cfg, warps, sm_count, st))
 		return cudaGetLastError();
-	cudaError_t e = cudaMemsetAsync(a.counter, 0, 4, st);
-	if (e == cudaSuccess)
-		e = cudaMemsetAsync(a.deferred, 0, 8, st);
+	// The counter and the two deferred words, with the unused word between them.
+	const cudaError_t e = cudaMemsetAsync(a.counter, 0, 16, st);
 	if (e != cudaSuccess)
 		return e;
 	if (cfg.format == PRT_NODES_COMPRESSED) {
