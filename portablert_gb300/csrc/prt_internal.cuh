@@ -222,9 +222,7 @@ __device__ __forceinline__ uint32_t x_face_bit(float x, uint32_t log) {
 }
 __device__ __forceinline__ void x_face_add(const XFaces &f, float x) {
 	const uint32_t k = x_face_bit(x, f.log), bit = 1u << (k & 31u);
-	uint32_t *w = f.words + kXHead + (k >> 5);
-	if (!(*(volatile uint32_t *)w & bit)) // (neighbours of a mesh share most of theirs)
-		atomicOr(w, bit);
+	atomicOr(f.words + kXHead + (k >> 5), bit);
 }
 // Whether no triangle's lower x face is at x.
 __device__ __forceinline__ bool x_face_free(const XFaces &f, float x) {
