@@ -240,14 +240,6 @@ __device__ __forceinline__ bool child_passes(const SlabRay &q, const float4 &a, 
 	return tmin <= __fmaf_rn(tmax, 1.0f + 0x1p-20f, 0x1p-120f);
 }
 
-template <bool REGULAR>
-__device__ __forceinline__ bool box_test(const RayC &r, float lx, float hx, float ly, float hy,
-                                         float lz, float hz) {
-	if (REGULAR || r.kind == 0)
-		return regular_box(r, lx, hx, ly, hy, lz, hz);
-	return conservative_box(r, lx, hx, ly, hy, lz, hz);
-}
-
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return (w >> (8 * k)) & 0xFFu; }
 
 // float(byte k of w), exactly: the byte placed in the mantissa of 2^23 (one byte
@@ -255,6 +247,37 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return (w >> (8
 __device__ __forceinline__ float byte_as_float(uint32_t w, int k) {
 	return __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)k)),
 	                 8388608.0f);
+}
+
+// The byte alone in the mantissa of 2^23.
+__device__ __forceinline__ float byte_biased(uint32_t w, int k) {
+	return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)k));
+}
+
+// regular_box on child record ck of a compressed node with origin (oxy, oz) and scales
+// (sxy, sz): the same decode (cdec_f) and products, every operation rounded as the scalar one,
+// x and y and the two z bounds in packed pairs: 12 FP instructions for 24 (a traversal of
+// compressed nodes is bound by issue).  tmax >= 0 and tmin <= tmax as max(tmin, 0) <= tmax.
+// 1,000,003 random rays on as many clustered triangles 934 -> 866 us, 2,097,152 rays on the
+// 1,048,576-triangle heightfield 1,110 -> 1,053 (z scalar: 883, 1,077).
+__device__ __forceinline__ bool compressed_passes(const SlabRay &q, const uint2 &ck,
+                                                  unsigned long long oxy, float oz,
+                                                  unsigned long long sxy, float sz) {
+	const unsigned long long bias = pack2(-8388608.0f, -8388608.0f);
+	const unsigned long long l =
+	    fma2(add2(pack2(byte_biased(ck.x, 0), byte_biased(ck.x, 2)), bias), sxy, oxy);
+	const unsigned long long h =
+	    fma2(add2(pack2(byte_biased(ck.x, 1), byte_biased(ck.x, 3)), bias), sxy, oxy);
+	float t1, t2, t3, t4;
+	unpack2(mul2(add2(l, q.no), q.f), t1, t3);
+	unpack2(mul2(add2(h, q.no), q.f), t2, t4);
+	const unsigned long long z = fma2(add2(pack2(byte_biased(ck.y, 0), byte_biased(ck.y, 1)), bias),
+	                                  pack2(sz, sz), pack2(oz, oz));
+	float t5, t6;
+	unpack2(mul2(add2(z, pack2(-q.oz, -q.oz)), pack2(q.fz, q.fz)), t5, t6);
+	const float tmin = max3f(fminf(t1, t2), fminf(t3, t4), fmaxf(fminf(t5, t6), 0.0f));
+	const float tmax = min3f(fmaxf(t1, t2), fmaxf(t3, t4), fmaxf(t5, t6));
+	return tmin <= tmax;
 }
 
 __device__ __forceinline__ RayC slot_ray(const WarpFixed &S, uint32_t s) {
@@ -365,13 +388,17 @@ __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const
 			const float sz = cscale((uint8_t)byte_of(w0.w, 2));
 			const float ox = __uint_as_float(w0.x), oy = __uint_as_float(w0.y),
 			            oz = __uint_as_float(w0.z);
-			const float lx = cdec_f(ox, byte_as_float(ck.x, 0), sx);
-			const float hx = cdec_f(ox, byte_as_float(ck.x, 1), sx);
-			const float ly = cdec_f(oy, byte_as_float(ck.x, 2), sy);
-			const float hy = cdec_f(oy, byte_as_float(ck.x, 3), sy);
-			const float lz = cdec_f(oz, byte_as_float(ck.y, 0), sz);
-			const float hz = cdec_f(oz, byte_as_float(ck.y, 1), sz);
-			hit = box_test<REGULAR>(r, lx, hx, ly, hy, lz, hz);
+			if (REGULAR || r.kind == 0) {
+				hit = compressed_passes(q, ck, pack2(ox, oy), oz, pack2(sx, sy), sz);
+			} else {
+				const float lx = cdec_f(ox, byte_as_float(ck.x, 0), sx);
+				const float hx = cdec_f(ox, byte_as_float(ck.x, 1), sx);
+				const float ly = cdec_f(oy, byte_as_float(ck.x, 2), sy);
+				const float hy = cdec_f(oy, byte_as_float(ck.x, 3), sy);
+				const float lz = cdec_f(oz, byte_as_float(ck.y, 0), sz);
+				const float hz = cdec_f(oz, byte_as_float(ck.y, 1), sz);
+				hit = conservative_box(r, lx, hx, ly, hy, lz, hz);
+			}
 			if (inner) {
 				child = w1.x + __popc(imask & ((1u << k) - 1u));
 			} else {
