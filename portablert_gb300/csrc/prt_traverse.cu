@@ -1252,8 +1252,12 @@ cudaError_t dispatch(const TravArgs &a, const TravConfig &cfg, int sm_count, cud
 	const int warps = warps_for(cfg);
 	if (try_single(a, cfg, warps, sm_count, st))
 		return cudaGetLastError();
-	// The counter and the two deferred words, with the unused word between them.
-	const cudaError_t e = cudaMemsetAsync(a.counter, 0, 16, st);
+	// The counter and the two deferred words, in one go unless the word between them is the
+	// launch's error word, which stays set until the host reads it.
+	const bool between = a.err == a.counter + 1;
+	cudaError_t e = cudaMemsetAsync(a.counter, 0, between ? 4 : 16, st);
+	if (e == cudaSuccess && between)
+		e = cudaMemsetAsync(a.deferred, 0, 8, st);
 	if (e != cudaSuccess)
 		return e;
 	if (cfg.format == PRT_NODES_COMPRESSED) {
