@@ -796,7 +796,8 @@ __device__ __forceinline__ bool claim_batch(const ServeQueues &q, uint32_t held[
 // the skipped batches with the general test (returns at once when there are none); 3 =
 // a serving launch: batches claimed from the serving queues (claim_batch), the plain or
 // the general test chosen per batch, descriptors and rays read around L1; 4 = one kernel for
-// a run of up to some hundred rays per warp, and for most cameras (single_batch): every
+// a run of up to some hundred rays per warp, several runs of up to 16, and most cameras
+// (single_batch): every
 // batch, the test chosen per batch, a warp's first batch by its number and the next ones,
 // if any, from the counter.
 template <int FMT, bool COUNT, bool LEAF1, bool BOUNDED, int PASS>
@@ -1151,6 +1152,11 @@ int warps_for(const TravConfig &cfg) {
 // (the means above 1.2 come from rays with zero components).  With compressed nodes or
 // larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.
 //
+// Several runs (padded to whole warps of 32).  One round of batches of 4, 8 or 16.  Batch
+// graphs, us: 20 scenes of up to 6,836 triangles and 5,762 rays 324 -> 273, 48 of 18,789 and
+// 4,847 418 -> 362, 7 of 31,983 and 4,384 419 -> 306.  (A server's waves are bounded and keep
+// batches of 32: each batch ends with a system fence, and small ones cost up to 6 %.)
+//
 // Cameras.  The packet descent (batches of 32) pays where a triangle covers many pixels and
 // there are enough batches.  Batches of 8 / 16 / 32 / packets, us:
 //     triangles  900 x 600                1600 x 900               2048 x 2048
@@ -1159,6 +1165,8 @@ int warps_for(const TravConfig &cfg) {
 //     65,536     202 / 218 / 277 / 287    284 / 274 / 288 / 294    638 / 514 / 464 / 472
 uint32_t single_batch(const TravArgs &a, const TravConfig &cfg, uint64_t slots) {
 	const uint64_t n = a.n_virtual, per = (n + slots - 1) / slots;
+	if (a.n_segs)
+		return per <= 4u ? 4u : per <= 8u ? 8u : per <= 16u ? 16u : 0u;
 	if (per <= 8u)
 		return ((uint32_t)per + 3u) & ~3u;
 	if (a.use_cam) {
@@ -1187,10 +1195,10 @@ bool launch_single(TravArgs a, const TravConfig &cfg, int warps, int sm_count, c
 	return true;
 }
 
-// Whether one kernel took the launch: of one run, not counting, not bounded.
+// Whether one kernel took the launch: not counting, not bounded.
 bool try_single(const TravArgs &a, const TravConfig &cfg, int warps, int sm_count,
                 cudaStream_t st) {
-	if (a.n_segs || cfg.count || (a.max_batches && !a.use_cam))
+	if (cfg.count || (a.max_batches && !a.use_cam))
 		return false;
 	if (cfg.format == PRT_NODES_COMPRESSED)
 		return a.max_leaf <= 1u
