@@ -1150,7 +1150,12 @@ int warps_for(const TravConfig &cfg) {
 //     1,300,000  1.33 / 0.95    1.41 / 0.97    1.34 / 0.96
 //     2,000,000  1.11 / 0.93    1.22 / 0.95    1.23 / 0.95
 // (the means above 1.2 come from rays with zero components).  With compressed nodes or
-// larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.
+// larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.  In small scenes
+// a batch is short, and larger ones pay sooner (us; two passes / 8 / 16 / 32):
+//     64 triangles       60,000  20 / 15 / 11 / 12    320,000  41 / 43 / 35 / 31
+//                     1,300,000  103 / 154 / 119 / 98
+//     2,500 triangles    60,000  52 / 28 / 37 / 51    320,000  75 / 76 / 70 / 72
+//                     1,300,000  288 / 272 / 233 / 218
 //
 // Several runs (padded to whole warps of 32).  One round of batches of 4, 8 or 16.  Batch
 // graphs, us: 20 scenes of up to 6,836 triangles and 5,762 rays 324 -> 273, 48 of 18,789 and
@@ -1175,10 +1180,12 @@ uint32_t single_batch(const TravArgs &a, const TravConfig &cfg, uint64_t slots) 
 			return per <= 32u ? 8u : per <= 120u ? 16u : 0u;
 		return per <= 120u ? 8u : per <= 450u ? 16u : 32u;
 	}
-	if (per <= 64u)
+	const bool small = a.scene0.n_tris <= 4096u;
+	if (per <= (small ? 16u : 64u))
 		return 8u;
-	const bool plain = cfg.format == PRT_NODES_FP32 && a.max_leaf <= 1u;
-	return per <= (plain ? 420u : 130u) ? 16u : 0u;
+	if (cfg.format != PRT_NODES_FP32 || a.max_leaf > 1u)
+		return per <= 130u ? 16u : 0u;
+	return per <= (small ? 64u : 300u) ? 16u : per <= 420u ? 32u : 0u;
 }
 
 template <int FMT, bool LEAF1>

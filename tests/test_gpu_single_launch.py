@@ -21,16 +21,18 @@ def _rays():
     return np.ascontiguousarray(r)
 
 
-@pytest.mark.parametrize("leaf,fmt", [(1, 0), (4, 0), (1, 1), (8, 1)])
-def test_routes_give_the_same_records(gpu_backend, oracle_lib, leaf, fmt):
+@pytest.mark.parametrize("leaf,fmt,n_tris", [(1, 0, 5000), (1, 0, 700), (4, 0, 5000),
+                                             (1, 1, 5000), (8, 1, 5000), (8, 1, 700)])
+def test_routes_give_the_same_records(gpu_backend, oracle_lib, leaf, fmt, n_tris):
     import torch
 
     b, lay = gpu_backend, hitreg.layout(TAGS)
-    tris, rays = W.soup_tris(62, 5000), _rays()
+    tris, rays = W.soup_tris(62, n_tris), _rays()
     full = oracle_lib.brute_force(tris, rays[:1500])
     warps = int(b.stat("sms")) * 32
-    sizes = [8 * warps, 8 * warps + 1, 12 * warps + 5, 64 * warps, 64 * warps + 1,
-             130 * warps - 3, 130 * warps + 1, 420 * warps, 420 * warps + 1]
+    sizes = [8 * warps, 8 * warps + 1, 16 * warps, 16 * warps + 5, 64 * warps, 64 * warps + 1,
+             130 * warps - 3, 130 * warps + 1, 300 * warps, 300 * warps + 1, 420 * warps,
+             420 * warps + 1]
     top = 421 * warps
     d = torch.from_numpy(np.tile(rays, (-(-top // TILE), 1))[:top]).cuda()
     try:
