@@ -96,8 +96,8 @@ struct TravArgs {
 	uint32_t warp_bytes;     // shared memory per warp
 	uint32_t max_leaf;       // most triangles in a leaf of any scene of the launch
 	uint32_t max_batches;    // batches per warp before it exits (0 = no bound)
-	uint32_t batch;          // rays a warp takes at a time: 32, or 16 / 8 for one small
-	                         // run (more warps busy, shorter chains per warp)
+	uint32_t batch;          // rays a warp takes at a time: 32, or 4 to 16 where few rays
+	                         // are to keep all warps busy (single_batch, batch_rays)
 	uint32_t claims;         // PASS 4: there are more batches than warps
 	uint32_t *counter;
 	uint32_t *deferred;      // [0] batches the regular pass left to the general one,
@@ -1150,8 +1150,8 @@ int warps_for(const TravConfig &cfg) {
 //     1,300,000  1.33 / 0.95    1.41 / 0.97    1.34 / 0.96
 //     2,000,000  1.11 / 0.93    1.22 / 0.95    1.23 / 0.95
 // (the means above 1.2 come from rays with zero components).  With compressed nodes or
-// larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.  In small scenes
-// a batch is short, and larger ones pay sooner (us; two passes / 8 / 16 / 32):
+// larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.  With FP32 nodes
+// and one triangle per leaf a small scene's batch is short, and larger ones pay sooner (us; two passes / 8 / 16 / 32):
 //     64 triangles       60,000  20 / 15 / 11 / 12    320,000  41 / 43 / 35 / 31
 //                     1,300,000  103 / 154 / 119 / 98
 //     2,500 triangles    60,000  52 / 28 / 37 / 51    320,000  75 / 76 / 70 / 72
@@ -1180,11 +1180,13 @@ uint32_t single_batch(const TravArgs &a, const TravConfig &cfg, uint64_t slots) 
 			return per <= 32u ? 8u : per <= 120u ? 16u : 0u;
 		return per <= 120u ? 8u : per <= 450u ? 16u : 32u;
 	}
+	if (cfg.format != PRT_NODES_FP32 || a.max_leaf > 1u) {
+		const bool tiny = a.scene0.n_tris <= 256u; // (as the small scenes below)
+		return per <= (tiny ? 32u : 64u) ? 8u : per > 130u ? 0u : tiny && per > 64u ? 32u : 16u;
+	}
 	const bool small = a.scene0.n_tris <= 4096u;
 	if (per <= (small ? 16u : 64u))
 		return 8u;
-	if (cfg.format != PRT_NODES_FP32 || a.max_leaf > 1u)
-		return per <= 130u ? 16u : 0u;
 	return per <= (small ? 64u : 300u) ? 16u : per <= 420u ? 32u : 0u;
 }
 
