@@ -1229,7 +1229,7 @@ void launch_passes(const TravArgs &a, int warps, int sm_count, cudaStream_t st) 
 template <int FMT, bool COUNT>
 void launch(const TravArgs &a, int warps, int sm_count, cudaStream_t st) {
 	// A counting run is one general pass over all the work (no bounded warps).  So are
-	// camera rays: the examples' cameras put a zero direction component in one batch of
+	// cameras that take packets: the examples' cameras put a zero direction component in one batch of
 	// every row, and finding those batches again costs the deferred pass a recomputation
 	// of every ray.
 	if (COUNT || a.use_cam) {
