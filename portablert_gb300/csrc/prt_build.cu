@@ -98,7 +98,7 @@ __global__ void k_scene_of(const uint32_t *tri_off, uint32_t n_scenes, uint32_t 
 			scene_of[i] = s;
 }
 
-__global__ void k_clear_word(uint32_t *word) { *word = 0u; }
+__global__ void k_clear_error(uint32_t *err, uint32_t bits) { clear_error_bits(err, bits); }
 
 // Empty bounds, and no split after each scene's last leaf.
 __global__ void k_bounds_init(uint32_t *gb, uint32_t n_scenes, const uint32_t *tri_off,
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kUpLeaves) k_bottom_up(UpArgs A) {
 	S.node[t] = sp.z;
 	if (!REFIT && sp.z != kNone && sp.x >= b0 && sp.y < b0 + kUpLeaves) {
 		if (sp.z >= A.n_ids) {
-			atomicOr(A.err, kErrCollapse);
+			set_error_bits(A.err, kErrCollapse);
 			S.node[t] = 0u;
 		} else {
 			const float4 lo = A.ibox[2 * (size_t)sp.z], hi = A.ibox[2 * (size_t)sp.z + 1];
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kUpLeaves) k_bottom_up(UpArgs A) {
 		if (S.walk_at + t < A.walk_cap)
 			A.walks[S.walk_at + t] = S.escape[t];
 		else
-			atomicOr(A.err, kErrCollapse);
+			set_error_bits(A.err, kErrCollapse);
 	}
 }
 
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(128) k_walk_up(UpArgs A) {
 		for (uint32_t steps = 0;; ++steps) {
 			const uint32_t p = at.z;
 			if (p >= A.n_ids || steps >= A.n_ids || at.y >= A.n) {
-				atomicOr(A.err, kErrCollapse);
+				set_error_bits(A.err, kErrCollapse);
 				break;
 			}
 			const uint32_t l = A.left[p], r = A.right[p];
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(8 * kCollapseItems)
 			__syncwarp();
 			if (lane == 0 && (got[0] + nodes > A.node_cap || got[1] + tris > A.n ||
 			                  got[2] + nodes > A.node_cap)) {
-				atomicOr(A.err, kErrCollapse);
+				set_error_bits(A.err, kErrCollapse);
 				got[0] = kNone; // nothing of the block's items is written
 			}
 		}
@@ -1415,7 +1415,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 	int rc = collapse_enqueue(d_tris, plan, sc, ws, svals, roots, st, d_err, host_checks, msg);
 	while (rc == PRT_OK && plan.sah && ws.h_counters[kCtrGate] != 0) {
 		if (ws.h_counters[kCtrGate] != kGateLevels) {
-			k_clear_word<<<1, 1, 0, st>>>(d_err); // (reported here)
+			k_clear_error<<<1, 1, 0, st>>>(d_err, kErrSah); // (reported here)
 			BUILD_TRY(cudaStreamSynchronize(st));
 			msg = "sah build: internal check failed";
 			return PRT_ERR_DEVICE;

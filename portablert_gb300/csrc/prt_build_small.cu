@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 			const uint32_t i = tid + (uint32_t)k * kThreads;
 			prim[k] = i < n ? (uint32_t)(keys[i] & 0xFFFFFFFFull) : 0u;
 			if (prim[k] >= n) { // cannot happen: the keys of [0, n) sort first
-				atomicOr(err, kErrCollapse);
+				set_error_bits(err, kErrCollapse);
 				prim[k] = 0;
 			}
 		}
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 		m = kept;
 		if (merged == 0u || iter >= n) { // cannot happen (see above); reported, not looped
 			if (tid == 0)
-				atomicOr(err, kErrCollapse);
+				set_error_bits(err, kErrCollapse);
 			return;
 		}
 		__syncthreads();
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 				scan[0] = made;
 				scan[1] = failed;
 				if (failed)
-					atomicOr(err, kErrCollapse);
+					set_error_bits(err, kErrCollapse);
 			}
 		}
 		__syncthreads();
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 			const bool fits = nb + n_inner <= node_cap && ob + n_inner <= kSmallMax &&
 			                  tb + n_tris <= n;
 			if (live && !fits && c8 == 0u)
-				atomicOr(err, kErrCollapse);
+				set_error_bits(err, kErrCollapse);
 			if (live && fits) {
 				if (has) {
 					uint32_t ref;
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 								stack[sp++] = lr_s[z] >> 16;
 								stack[sp++] = lr_s[z] & 0xFFFFu;
 							} else {
-								atomicOr(err, kErrCollapse); // more than 8 leaves: not a leaf
+								set_error_bits(err, kErrCollapse); // more than 8 leaves: not a leaf
 							}
 						}
 					}

@@ -96,7 +96,7 @@ struct prt_b200_ctx {
 	uint32_t *d_work() { return work.as<uint32_t>(); }
 	uint32_t *d_err() { return err_dev; }
 	// The bits set so far; they start again at zero.
-	uint32_t take_err() { return __atomic_exchange_n(h_err, 0u, __ATOMIC_SEQ_CST); }
+	uint32_t take_err() { return prt::take_error_bits(h_err); }
 	unsigned long long *d_visits() {
 		return reinterpret_cast<unsigned long long *>(work.as<uint8_t>() + 16);
 	}

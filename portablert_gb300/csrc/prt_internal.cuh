@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "prt_errword.h"
+
 namespace prt {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;
@@ -27,7 +29,7 @@ constexpr uint64_t kMaxTris = (1ull << 27) - 1;
 constexpr uint32_t kIndexBits = 27;
 constexpr uint32_t kIndexMask = (1u << kIndexBits) - 1u;
 
-// Bits of the device error word.
+// Bits of an error word (prt_errword.h).
 enum : uint32_t {
 	kErrStack = 1u,    // traversal stack overflow (ray abandoned)
 	kErrLookback = 2u, // radix-sort look-back gave up waiting

@@ -146,7 +146,7 @@ __device__ __forceinline__ float rec_c(const float4 &lo, const float4 &hi, int k
 	return k == 0 ? centre(lo.x, hi.x) : (k == 1 ? centre(lo.y, hi.y) : centre(lo.z, hi.z));
 }
 
-__device__ __forceinline__ void flag(uint32_t *err) { atomicOr(err, kErrSah); }
+__device__ __forceinline__ void flag(uint32_t *err) { set_error_bits(err, kErrSah); }
 
 __device__ __forceinline__ void bins_init(uint32_t *b, int at, int step, int words = kBinWords) {
 	for (int k = at; k < words; k += step) {

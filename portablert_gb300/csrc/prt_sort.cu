@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kSortThreads)
 				uint32_t flag = s & ~kStMask;
 				if (flag == 0u) {
 					if (++spins > kSpinLimit) {
-						atomicOr(err, kErrLookback);
+						set_error_bits(err, kErrLookback);
 						break;
 					}
 					__nanosleep(32);

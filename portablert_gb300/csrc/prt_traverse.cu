@@ -473,7 +473,7 @@ __device__ __forceinline__ void packet_descent(const TravArgs &a, const SceneDes
 		const bool mine = (rays >> lane) & 1u;
 		if (++steps > step_limit) { // a malformed tree
 			if (lane == 0)
-				atomicOr(a.err, kErrStack);
+				set_error_bits(a.err, kErrStack);
 			fault = true;
 			break;
 		}
@@ -661,7 +661,7 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		++steps;
 		if (ptop > a.pool_cap || steps > step_limit) {
 			if (lane == 0)
-				atomicOr(a.err, kErrStack);
+				set_error_bits(a.err, kErrStack);
 			fault = true;
 			break;
 		}
