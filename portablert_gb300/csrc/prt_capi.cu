@@ -129,6 +129,24 @@ prt::TravConfig trav_config(const prt_b200_ctx *ctx) {
 	return cfg;
 }
 
+// Waits, unless dismissed, for what a host-buffer call has queued: one that fails halfway
+// returns only when nothing reads or writes its caller's buffers any more.
+class WaitOnFailure {
+  public:
+	explicit WaitOnFailure(prt_b200_ctx *ctx) : ctx_(ctx) {}
+	~WaitOnFailure() {
+		if (ctx_)
+			for (cudaStream_t st : {ctx_->s_in, ctx_->stream, ctx_->s_k2, ctx_->s_out})
+				cudaStreamSynchronize(st);
+	}
+	void dismiss() { ctx_ = nullptr; }
+	WaitOnFailure(const WaitOnFailure &) = delete;
+	WaitOnFailure &operator=(const WaitOnFailure &) = delete;
+
+  private:
+	prt_b200_ctx *ctx_;
+};
+
 // Pageable memory that the host has never touched (a fresh std::vector's or numpy array's
 // pages) has no physical pages yet.  A device store that meets such a page waits for the
 // host's fault handler, about 15 us per 64 KiB page and one at a time: 66 MB of records took
@@ -531,6 +549,7 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 			void *d_out = d_in ? prt::device_alias(ctx, out_host) : nullptr;
 			ctx->last_in_place = d_in && d_out;
 			if (d_in && d_out) {
+				WaitOnFailure in_flight(ctx);
 				const bool untouched = untouched_pages(out_host, (uint64_t)rec_size * n);
 				// (A counting run is one launch: each resets the counters.)
 				const uint64_t piece = untouched && !ctx->count
@@ -550,6 +569,7 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 				if (ctx->count)
 					CAPI_TRY(ctx, cudaMemcpyAsync(ctx->visits, ctx->d_visits(), 16,
 					                              cudaMemcpyDeviceToHost, ctx->stream));
+				in_flight.dismiss();
 				return check_device_errors(ctx);
 			}
 		}
@@ -584,6 +604,7 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 		}
 		cudaStream_t ks[2] = {ctx->stream, ctx->s_k2};
 		uint32_t *ctr[2] = {ctx->d_work(), ctx->d_work() + 8};
+		WaitOnFailure in_flight(ctx);
 		// Earlier work of the context's stream (a _dev call) finishes before the chunks start.
 		CAPI_TRY(ctx, cudaEventRecord(ctx->ev_k[0], ctx->stream));
 		for (cudaStream_t st : {ctx->s_in, ctx->s_out, ctx->s_k2})
@@ -620,6 +641,7 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 		CAPI_TRY(ctx, cudaEventRecord(ctx->ev_in[0], ctx->s_out));
 		CAPI_TRY(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_in[0], 0));
 		CAPI_TRY(ctx, cudaStreamSynchronize(ctx->s_out));
+		in_flight.dismiss();
 		if (ctx->count)
 			CAPI_TRY(ctx, cudaMemcpy(ctx->visits, ctx->d_visits(), 16, cudaMemcpyDeviceToHost));
 		return check_device_errors(ctx);
