@@ -66,7 +66,9 @@ int prt_b200_available(void);
  * state (stream, error word) on `device`. */
 int prt_b200_create(int device, prt_b200_ctx **out);
 
-/* Replaces Backend::shutdown (backend.hpp:22): frees every device and host resource. */
+/* Replaces Backend::shutdown (backend.hpp:22): frees every device and host resource.  Batches
+ * and servers of the context may be destroyed before or after it; what they share with it (a
+ * few streams and words) goes with the last of them. */
 void prt_b200_destroy(prt_b200_ctx *ctx);
 
 /* Message of the last failing call on ctx ("" if none).  With ctx == NULL: the last

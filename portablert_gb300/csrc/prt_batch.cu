@@ -235,6 +235,7 @@ int prt_b200_batch_create(prt_b200_ctx *ctx, prt_b200_batch **out) {
 		delete b;
 		return rc;
 	}
+	++ctx->users;
 	*out = b;
 	return PRT_OK;
 }
@@ -243,10 +244,13 @@ void prt_b200_batch_destroy(prt_b200_batch *b) {
 	if (!b)
 		return;
 	if (b->ctx) {
-		std::lock_guard<std::mutex> lk(b->ctx->mu);
-		cudaSetDevice(b->ctx->device);
-		cudaDeviceSynchronize();
-		release_batch(b);
+		{
+			std::lock_guard<std::mutex> lk(b->ctx->mu);
+			cudaSetDevice(b->ctx->device);
+			cudaDeviceSynchronize();
+			release_batch(b);
+		}
+		prt::drop_context(b->ctx);
 	}
 	delete b;
 }

@@ -264,6 +264,32 @@ int query_stream(prt_b200_ctx *ctx, cudaStream_t st, prt_b200_ctx::QueryStream *
 	return PRT_OK;
 }
 
+// What a context's batches use as well goes with the last of them.
+void drop_context(prt_b200_ctx *ctx) {
+	if (ctx->users.fetch_sub(1) != 1)
+		return;
+	cudaSetDevice(ctx->device);
+	ctx->work.release();
+	if (ctx->h_err)
+		cudaFreeHost(ctx->h_err);
+	for (auto &q : ctx->query_streams) {
+		cudaEventDestroy(q.ev);
+		cudaFree(q.counter);
+	}
+	for (int i = 0; i < prt_b200_ctx::kPipe; ++i) {
+		if (ctx->ev_in[i])
+			cudaEventDestroy(ctx->ev_in[i]);
+		if (ctx->ev_k[i])
+			cudaEventDestroy(ctx->ev_k[i]);
+	}
+	for (cudaStream_t s : {ctx->s_in, ctx->s_out, ctx->s_k2, ctx->stream})
+		if (s) {
+			cudaStreamSynchronize(s);
+			cudaStreamDestroy(s);
+		}
+	delete ctx;
+}
+
 } // namespace prt
 
 extern "C" {
@@ -351,36 +377,22 @@ int prt_b200_create(int device, prt_b200_ctx **out) {
 void prt_b200_destroy(prt_b200_ctx *ctx) {
 	if (!ctx)
 		return;
-	cudaSetDevice(ctx->device);
-	for (cudaStream_t s : {ctx->stream, ctx->s_in, ctx->s_out, ctx->s_k2})
-		if (s)
-			cudaStreamSynchronize(s);
-	for (auto &q : ctx->query_streams)
-		cudaEventSynchronize(q.ev);
-	ctx->scene.release();
-	ctx->ws.release();
-	ctx->tris_in.release();
-	ctx->rays_buf.release();
-	ctx->out_buf.release();
-	ctx->work.release();
-	if (ctx->h_err)
-		cudaFreeHost(ctx->h_err);
-	for (auto &q : ctx->query_streams) {
-		cudaEventDestroy(q.ev);
-		cudaFree(q.counter);
+	{
+		std::lock_guard<std::mutex> lk(ctx->mu);
+		cudaSetDevice(ctx->device);
+		for (cudaStream_t s : {ctx->stream, ctx->s_in, ctx->s_out, ctx->s_k2})
+			if (s)
+				cudaStreamSynchronize(s);
+		for (auto &q : ctx->query_streams)
+			cudaEventSynchronize(q.ev);
+		ctx->scene_set = false;
+		ctx->scene.release();
+		ctx->ws.release();
+		ctx->tris_in.release();
+		ctx->rays_buf.release();
+		ctx->out_buf.release();
 	}
-	for (int i = 0; i < prt_b200_ctx::kPipe; ++i) {
-		if (ctx->ev_in[i])
-			cudaEventDestroy(ctx->ev_in[i]);
-		if (ctx->ev_k[i])
-			cudaEventDestroy(ctx->ev_k[i]);
-	}
-	for (cudaStream_t s : {ctx->s_in, ctx->s_out, ctx->s_k2, ctx->stream})
-		if (s) {
-			cudaStreamSynchronize(s);
-			cudaStreamDestroy(s);
-		}
-	delete ctx;
+	prt::drop_context(ctx);
 }
 
 // The calling thread's copy of the message, valid until its next call here.

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <exception>
 #include <mutex>
 #include <new>
@@ -38,6 +39,9 @@ class ErrorText {
 } // namespace prt
 
 struct prt_b200_ctx {
+	// The handle and one per batch: a batch (a server's too) may outlive the handle, and works
+	// on with the context's streams, lock, options and error word.
+	std::atomic<int> users{1};
 	int device = 0;
 	int sms = 0;
 	int pageable_access = 0; // the device reads pageable host memory in place
@@ -103,6 +107,9 @@ struct prt_b200_ctx {
 };
 
 namespace prt {
+
+// Ends one use of a context (see `users`); the last one frees it.  Its lock is not held.
+void drop_context(prt_b200_ctx *ctx);
 
 // The bookkeeping of a caller's stream that reads the context's scene (created at its
 // first use): record ->ev on the stream after the work, and set_tris waits for it.

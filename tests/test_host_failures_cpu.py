@@ -1,6 +1,7 @@
-"""A host-buffer query that fails halfway: it may return only when nothing that it queued can
-still read or write its caller's buffers.  Runs without a GPU, on a fake CUDA runtime whose
-launches fail on demand (the library's own host code is the real one)."""
+"""A host-buffer query that fails halfway may return only when nothing that it queued can still
+read or write its caller's buffers, and a context may be destroyed before its batches and
+servers.  Runs without a GPU, on a fake CUDA runtime whose launches fail on demand (the
+library's own host code is the real one)."""
 import os
 import subprocess
 import sys
@@ -60,4 +61,40 @@ def run_on_fake(fake, script, *args):
 @pytest.mark.parametrize("direct,launch", [(1, 1), (1, 2), (1, 4), (0, 1), (0, 3)])
 def test_nothing_in_flight_after_a_failed_launch(fake_runtime, direct, launch):
     r = run_on_fake(fake_runtime, FAILING_QUERY, direct, launch)
+    assert r.returncode == 0 and "OK" in r.stdout, r.stdout + r.stderr
+
+
+LIFETIMES = """
+import ctypes, sys
+from portablert_gb300 import _lib
+from portablert_gb300.backend import B200Backend
+from portablert_gb300.batch import Batch
+from portablert_gb300.serve import Server
+
+persistent = int(sys.argv[1])
+b = B200Backend(0)
+b.init()
+b.set_option("serve_persistent", persistent)
+batches = [Batch(b), Batch(b)]
+for k in batches:
+    k.set_tris_dev(0, [0, 0])
+server = Server(b, 0, [0, 0], 1 << 20, lanes=2)
+batches[0].close()
+b.shutdown()
+blocks = [bytearray(256) for _ in range(4096)]  # the freed context's memory is used again
+batches[1].set_tris_dev(0, [0, 0, 0])
+assert batches[1].stat("n_scenes") == 2
+batches[1].sync()
+server.close()
+batches[1].close()
+b.init()
+b.shutdown()
+print("OK")
+"""
+
+
+@pytest.mark.parametrize("persistent", [0, 1])
+def test_context_destroyed_before_its_batches_and_servers(fake_runtime, persistent, monkeypatch):
+    monkeypatch.setenv("MALLOC_PERTURB_", "165")  # freed memory is overwritten
+    r = run_on_fake(fake_runtime, LIFETIMES, persistent)
     assert r.returncode == 0 and "OK" in r.stdout, r.stdout + r.stderr
