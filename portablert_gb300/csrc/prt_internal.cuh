@@ -112,16 +112,20 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 	return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-// Per-ray constants.  `kind` selects the box test used on inner nodes:
+// Per-ray constants.  `kind` selects the box test used on inner nodes (prt_traverse.cu):
 //   0 regular: every origin component within 2^67 and every direction component between
 //              2^-58 and 2^60 in magnitude: the slab test on centres and half extents
-//              (child_passes in prt_traverse.cu) neither overflows nor meets a NaN.
-//   1 axis:    another finite ray, for instance with a zero direction component (infinite
-//              reciprocal); inner nodes use conservative_box below.
-//   2 all:     a non-finite component or all reciprocals infinite: every inner box
-//              passes and only the exact per-triangle test decides.
-//   3 free:    like 1 with a zero x component, and no triangle's box has its lower x face at
-//              the origin's x (XFaces): the x axis does not constrain a box around it.
+//              (SlabRay) neither overflows nor meets a NaN.
+//   2 all:     a non-finite component, all reciprocals infinite or all origin components
+//              past 2^67: every inner box passes and only the exact per-triangle test
+//              decides.
+//   3 axis:    any other ray, for instance with a zero direction component (infinite
+//              reciprocal): the same test with such axes reduced (AxisRay).
+//   4 axis, x: like 3 with an infinite reciprocal on the x axis, where some triangle's box
+//              may have its lower x face at the origin's x (XFaces): a box around it
+//              passes outright.
+// Kinds 3 and 4 have kOdd set where more than infinite reciprocals sets the ray apart.
+constexpr int kOdd = 8;
 struct RayC {
 	float ox, oy, oz, dx, dy, dz, fx, fy, fz;
 	int kind;
@@ -129,6 +133,10 @@ struct RayC {
 
 // (2^67 + 2^67) * 2^58 stays below FLT_MAX; 2^67 is about 1.5e20.
 constexpr float kCoordMax = 0x1p67f, kDirMax = 0x1p60f, kDirMin = 0x1p-58f;
+
+__device__ __forceinline__ bool dir_regular(float d) {
+	return fabsf(d) <= kDirMax && fabsf(d) >= kDirMin;
+}
 
 __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx, float dy,
                                          float dz) {
@@ -141,15 +149,20 @@ __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx,
 	r.fz = __frcp_rn(dz);
 	// (A NaN component fails its comparison, so it is never regular.)
 	const bool regular = fabsf(ox) <= kCoordMax && fabsf(oy) <= kCoordMax &&
-	                     fabsf(oz) <= kCoordMax && fabsf(dx) <= kDirMax &&
-	                     fabsf(dy) <= kDirMax && fabsf(dz) <= kDirMax && fabsf(dx) >= kDirMin &&
-	                     fabsf(dy) >= kDirMin && fabsf(dz) >= kDirMin;
+	                     fabsf(oz) <= kCoordMax && dir_regular(dx) && dir_regular(dy) &&
+	                     dir_regular(dz);
 	r.kind = 0;
 	if (!regular) {
 		const bool fin = isfinite(ox) && isfinite(oy) && isfinite(oz) && isfinite(dx) &&
 		                 isfinite(dy) && isfinite(dz);
-		const int n_inf = (int)isinf(r.fx) + (int)isinf(r.fy) + (int)isinf(r.fz);
-		r.kind = (!fin || n_inf == 3) ? 2 : 1;
+		const bool ix = isinf(r.fx), iy = isinf(r.fy), iz = isinf(r.fz);
+		const bool px = fabsf(ox) > kCoordMax, py = fabsf(oy) > kCoordMax,
+		           pz = fabsf(oz) > kCoordMax;
+		const bool odd = px || py || pz || !(ix || dir_regular(dx)) || !(iy || dir_regular(dy)) ||
+		                 !(iz || dir_regular(dz));
+		r.kind = !fin || (ix && iy && iz) || (px && py && pz)
+		             ? 2
+		             : (ix ? 4 : 3) + (odd ? kOdd : 0);
 	}
 	return r;
 }
@@ -197,15 +210,9 @@ __device__ __forceinline__ Child8 encode_child(const float4 &lo, const float4 &h
 	return ch;
 }
 
-// Bounds that contain the box a record was made from (x: child_lo_x, child_hi_x are closer).
+// Bounds that contain the box a record was made from.
 __device__ __forceinline__ float child_lo(float c, float e) { return __fsub_rd(c, e); }
 __device__ __forceinline__ float child_hi(float c, float e) { return __fadd_ru(c, e); }
-__device__ __forceinline__ float child_lo_x(float c, float e, uint32_t x16) {
-	return fmaxf(child_lo(c, e), __uint_as_float(x16 << 16));
-}
-__device__ __forceinline__ float child_hi_x(float c, float e, uint32_t x16) {
-	return fminf(child_hi(c, e), __uint_as_float(x16 & 0xFFFF0000u));
-}
 
 // Set of the x coordinates at which some triangle's box of a scene has its lower face: a
 // hash set of 2^log bits (8 to 16 per triangle) after kXHead words, of which the first is
@@ -263,61 +270,6 @@ __device__ __forceinline__ bool regular_box(const RayC &r, float lx, float hx, f
 	float t5 = (lz - r.oz) * r.fz, t6 = (hz - r.oz) * r.fz;
 	float tmin = fmaxf(fmaxf(fminf(t1, t2), fminf(t3, t4)), fminf(t5, t6));
 	float tmax = fminf(fminf(fmaxf(t1, t2), fmaxf(t3, t4)), fmaxf(t5, t6));
-	return tmax >= 0.0f && tmin <= tmax;
-}
-
-// One axis of the conservative test for a ray with an infinite reciprocal on it.
-// A triangle box on this axis yields, per ref_slab: origin below the box -> both t's
-// +inf (reciprocal +inf) or -inf; origin above -> the opposite; strictly inside ->
-// (-inf, +inf); origin exactly on the lower face -> NaN, which on the x axis makes the
-// whole reference test pass and on y or z removes that axis from it.  For an inner box
-// the same below/above answer holds for every box under it; otherwise the axis is
-// treated as unconstrained (y, z, and x of kind 3) or the box passes outright (x).  (On the
-// upper face the reference rejects, or accepts no more than it would without the axis.)
-__device__ __forceinline__ bool inf_axis(float o, float lo, float hi, float f, bool is_x, float &m,
-                                         float &M) {
-	if (o < lo) {
-		m = M = (f > 0.0f) ? INFINITY : -INFINITY;
-	} else if (o > hi) {
-		m = M = (f > 0.0f) ? -INFINITY : INFINITY;
-	} else {
-		if (is_x)
-			return true;
-		m = -INFINITY;
-		M = INFINITY;
-	}
-	return false;
-}
-
-__device__ __forceinline__ bool conservative_box(const RayC &r, float lx, float hx, float ly,
-                                                 float hy, float lz, float hz) {
-	if (r.kind == 2)
-		return true;
-	float m0, M0, m1, M1, m2, M2;
-	if (isinf(r.fx)) {
-		if (inf_axis(r.ox, lx, hx, r.fx, r.kind != 3, m0, M0))
-			return true;
-	} else {
-		float a = (lx - r.ox) * r.fx, b = (hx - r.ox) * r.fx;
-		m0 = fminf(a, b);
-		M0 = fmaxf(a, b);
-	}
-	if (isinf(r.fy)) {
-		inf_axis(r.oy, ly, hy, r.fy, false, m1, M1);
-	} else {
-		float a = (ly - r.oy) * r.fy, b = (hy - r.oy) * r.fy;
-		m1 = fminf(a, b);
-		M1 = fmaxf(a, b);
-	}
-	if (isinf(r.fz)) {
-		inf_axis(r.oz, lz, hz, r.fz, false, m2, M2);
-	} else {
-		float a = (lz - r.oz) * r.fz, b = (hz - r.oz) * r.fz;
-		m2 = fminf(a, b);
-		M2 = fmaxf(a, b);
-	}
-	float tmin = fmaxf(fmaxf(m0, m1), m2);
-	float tmax = fminf(fminf(M0, M1), M2);
 	return tmax >= 0.0f && tmin <= tmax;
 }
 

@@ -28,7 +28,7 @@
 //    passes.
 //  * A query of ray buffers is two launches: a regular pass over the batches whose 32
 //    rays are all regular (kind 0: the plain slab test only), which counts and skips
-//    the others, and a deferred pass over those with the conservative test, for instance for
+//    the others, and a deferred pass over those with the other test (AxisRay), for instance for
 //    zero direction components (it returns at once when there are none).  Camera queries and
 //    counting runs are one general launch, in which a batch of regular rays takes the
 //    plain test; batches of large images of few triangles start with a packet descent
@@ -51,6 +51,7 @@
 // Algorithmic bytes per ray: 24 (ray) + R (record) + node bytes visited + 48 per
 // triangle tested; the counting variant (COUNT) measures the visits.
 #include <algorithm>
+#include <type_traits>
 #include <mutex>
 
 #include "../../include/prt_b200.h"
@@ -240,6 +241,92 @@ __device__ __forceinline__ bool child_passes(const SlabRay &q, const float4 &a, 
 	return tmin <= __fmaf_rn(tmax, 1.0f + 0x1p-20f, 0x1p-120f);
 }
 
+// The same test for any other ray (and for a regular one in a batch with such).  `g` and `h`
+// scale near and far, 1 on an axis that is regular.
+//
+// An axis of infinite reciprocal (a zero component) takes +-1 in the reciprocal's place, so
+// that its near and far tell by their signs, exactly, whether the origin lies before, inside
+// or behind the (widened) extent, and is scaled by infinity to what the reference's slab test
+// works with: two equal infinities outside, -inf and +inf inside, where a face's NaN
+// removes y or z from its test.  The face's 0 * inf here is a NaN too, which max3f and min3f
+// pass over.  On the x axis the reference's whole test passes at a lower face, so of kind 4 a
+// box with the origin's x inside passes outright.
+//
+// Odd rays (kOdd): a reciprocal above 2^58 counts as 2^58, which is no more than the
+// reference's near ahead of the origin, with far scaled by infinity; an axis whose origin
+// is past 2^67 is left out (0 * inf).  A reciprocal below 2^-60 needs nothing: the margin's
+// 2^-120 covers what underflow loses.
+//
+// Why: rays in a plane of two axes, a camera's middle row and column among them, are the
+// longest chains of their launch.  Bounds stored as such and a branch per axis / bounds
+// decoded from centre and half extent / this, us: 2,400,000 rays in a z plane of the
+// 1,048,576-triangle heightfield 679 / 721 / 599, 400,000 in an x plane that holds faces
+// 12,734 / 13,513 / 12,254, 320 x 200 pixels on 65,536 triangles 118 / 117 / 108.  (As a third
+// instance of trace_batch, or as a branch for odd rays in the second, those cost regular rays
+// 3 % in registers.)
+struct AxisRay {
+	SlabRay q;
+	unsigned long long g, h; // x and y
+	float gz, hz;
+	float ox;
+	bool inf_x, x_passes, all;
+};
+
+__device__ __forceinline__ void axis_scale(float o, float &f, float &g, float &h, bool odd) {
+	const bool inf = isinf(f);
+	g = h = inf ? INFINITY : 1.0f;
+	f = inf ? copysignf(1.0f, f) : f;
+	if (odd && !inf) {
+		if (fabsf(o) > kCoordMax) {
+			f = 0.0f;
+			g = h = INFINITY;
+		} else if (fabsf(f) > 1.0f / kDirMin) {
+			f = copysignf(1.0f / kDirMin, f);
+			h = INFINITY;
+		}
+	}
+}
+
+__device__ __forceinline__ AxisRay axis_ray(const RayC &r) {
+	RayC m = r;
+	float gx, gy, hx, hy;
+	AxisRay x;
+	axis_scale(r.ox, m.fx, gx, hx, r.kind & kOdd);
+	axis_scale(r.oy, m.fy, gy, hy, r.kind & kOdd);
+	axis_scale(r.oz, m.fz, x.gz, x.hz, r.kind & kOdd);
+	x.q = slab_ray(m);
+	x.g = pack2(gx, gy);
+	x.h = pack2(hx, hy);
+	x.ox = r.ox;
+	x.inf_x = isinf(r.fx);
+	x.x_passes = (r.kind & 7) == 4;
+	x.all = r.kind == 2;
+	return x;
+}
+
+__device__ __forceinline__ bool child_passes(const AxisRay &x, const float4 &a, const float4 &b) {
+	const SlabRay &q = x.q;
+	const unsigned long long t = mul2(add2(pack2(a.x, a.y), q.no), q.f);
+	const unsigned long long e = pack2(a.z, a.w);
+	float nx, ny, fx, fy;
+	unpack2(mul2(fma2(e, q.naf, t), x.g), nx, ny);
+	unpack2(mul2(fma2(e, q.af, t), x.h), fx, fy);
+	const float tz = (b.x - q.oz) * q.fz;
+	const float nz = __fmaf_rn(-b.y, q.afz, tz) * x.gz, fz = __fmaf_rn(b.y, q.afz, tz) * x.hz;
+	bool outright = x.all;
+	if (x.inf_x) {
+		// (Closer bounds: the widened extent of a box that ends near 0 reaches over it.)
+		const uint32_t x16 = __float_as_uint(b.w);
+		if (x.ox < __uint_as_float(x16 << 16) || x.ox > __uint_as_float(x16 & 0xFFFF0000u))
+			nx = INFINITY; // (outside; fx is +inf or a NaN if the test above saw it inside)
+		outright = outright || (x.x_passes && !(nx > 0.0f) && !(fx < 0.0f));
+	}
+	const float tmin = max3f(nx, ny, fmaxf(nz, 0.0f));
+	const float tmax = min3f(fx, fy, fz);
+	// (Every axis may be a NaN: then nothing constrains.)
+	return outright || !(tmin > __fmaf_rn(tmax, 1.0f + 0x1p-20f, 0x1p-120f));
+}
+
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return (w >> (8 * k)) & 0xFFu; }
 
 // float(byte k of w), exactly: the byte placed in the mantissa of 2^23 (one byte
@@ -260,9 +347,12 @@ __device__ __forceinline__ float byte_biased(uint32_t w, int k) {
 // compressed nodes is bound by issue).  tmax >= 0 and tmin <= tmax as max(tmin, 0) <= tmax.
 // 1,000,003 random rays on as many clustered triangles 934 -> 866 us, 2,097,152 rays on the
 // 1,048,576-triangle heightfield 1,110 -> 1,053 (z scalar: 883, 1,077).
-__device__ __forceinline__ bool compressed_passes(const SlabRay &q, const uint2 &ck,
-                                                  unsigned long long oxy, float oz,
-                                                  unsigned long long sxy, float sz) {
+struct CompressedSlab {
+	float nx, fx, ny, fy, nz, fz; // near and far per axis
+};
+__device__ __forceinline__ CompressedSlab compressed_slab(const SlabRay &q, const uint2 &ck,
+                                                          unsigned long long oxy, float oz,
+                                                          unsigned long long sxy, float sz) {
 	const unsigned long long bias = pack2(-8388608.0f, -8388608.0f);
 	const unsigned long long l =
 	    fma2(add2(pack2(byte_biased(ck.x, 0), byte_biased(ck.x, 2)), bias), sxy, oxy);
@@ -275,9 +365,30 @@ __device__ __forceinline__ bool compressed_passes(const SlabRay &q, const uint2 
 	                                  pack2(sz, sz), pack2(oz, oz));
 	float t5, t6;
 	unpack2(mul2(add2(z, pack2(-q.oz, -q.oz)), pack2(q.fz, q.fz)), t5, t6);
-	const float tmin = max3f(fminf(t1, t2), fminf(t3, t4), fmaxf(fminf(t5, t6), 0.0f));
-	const float tmax = min3f(fmaxf(t1, t2), fmaxf(t3, t4), fmaxf(t5, t6));
-	return tmin <= tmax;
+	return CompressedSlab{fminf(t1, t2), fmaxf(t1, t2), fminf(t3, t4),
+	                      fmaxf(t3, t4), fminf(t5, t6), fmaxf(t5, t6)};
+}
+
+__device__ __forceinline__ bool compressed_passes(const SlabRay &q, const uint2 &ck,
+                                                  unsigned long long oxy, float oz,
+                                                  unsigned long long sxy, float sz) {
+	const CompressedSlab c = compressed_slab(q, ck, oxy, oz, sxy, sz);
+	return max3f(c.nx, c.ny, fmaxf(c.nz, 0.0f)) <= min3f(c.fx, c.fy, c.fz);
+}
+
+// The same with the scales of AxisRay.
+__device__ __forceinline__ bool compressed_passes(const AxisRay &x, const uint2 &ck,
+                                                  unsigned long long oxy, float oz,
+                                                  unsigned long long sxy, float sz) {
+	const CompressedSlab c = compressed_slab(x.q, ck, oxy, oz, sxy, sz);
+	float gx, gy, hx, hy;
+	unpack2(x.g, gx, gy);
+	unpack2(x.h, hx, hy);
+	const float nx = c.nx * gx, fx = c.fx * hx;
+	const bool outright = x.all || (x.x_passes && !(nx > 0.0f) && !(fx < 0.0f));
+	const float tmin = max3f(nx, c.ny * gy, fmaxf(c.nz * x.gz, 0.0f));
+	const float tmax = min3f(fx, c.fy * hy, c.fz * x.hz);
+	return outright || !(tmin > tmax);
 }
 
 __device__ __forceinline__ RayC slot_ray(const WarpFixed &S, uint32_t s) {
@@ -342,11 +453,22 @@ __device__ __forceinline__ void test_queued(const float4 *__restrict__ tri4, War
 	}
 }
 
+// What the test of inner boxes takes: of a batch whose rays are all of kind 0, of any other.
+template <bool REGULAR>
+using NodeRay = std::conditional_t<REGULAR, SlabRay, AxisRay>;
+template <bool REGULAR> __device__ __forceinline__ NodeRay<REGULAR> node_ray(const RayC &r) {
+	if constexpr (REGULAR)
+		return slab_ray(r);
+	else
+		return axis_ray(r);
+}
+
 // Child `k` of `node`: slab test and what it refers to.
 template <int FMT, bool REGULAR>
-__device__ __forceinline__ void test_child(const void *__restrict__ nodes, const RayC &r,
-                                           const SlabRay &q, uint32_t node, int k, bool &hit, bool &inner,
-                                           uint32_t &child, uint32_t &leaf_n) {
+__device__ __forceinline__ void test_child(const void *__restrict__ nodes,
+                                           const NodeRay<REGULAR> &q, uint32_t node, int k,
+                                           bool &hit, bool &inner, uint32_t &child,
+                                           uint32_t &leaf_n) {
 	hit = false;
 	inner = false;
 	child = 0;
@@ -356,16 +478,10 @@ __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const
 		ld_nc_256(&(static_cast<const Node8 *>(nodes) + node)->c[k], a, b);
 		const uint32_t ref = __float_as_uint(b.z);
 		// An unused slot has a NaN box, which a regular ray's test never passes; the
-		// conservative test would, so only the general pass checks the reference.
+		// other test would, so only the general pass checks the reference.
 		if (REGULAR || ref != kNone) {
 			inner = !ref_is_leaf(ref);
-			if (REGULAR || r.kind == 0)
-				hit = child_passes(q, a, b);
-			else
-				hit = conservative_box(r, child_lo_x(a.x, a.z, __float_as_uint(b.w)),
-				                       child_hi_x(a.x, a.z, __float_as_uint(b.w)),
-				                       child_lo(a.y, a.w), child_hi(a.y, a.w),
-				                       child_lo(b.x, b.y), child_hi(b.x, b.y));
+			hit = child_passes(q, a, b);
 			// A node index, or a leaf's first triangle: both below 2^27, under the
 			// leaf flag and count bits.
 			child = ref & kIndexMask;
@@ -388,17 +504,7 @@ __device__ __forceinline__ void test_child(const void *__restrict__ nodes, const
 			const float sz = cscale((uint8_t)byte_of(w0.w, 2));
 			const float ox = __uint_as_float(w0.x), oy = __uint_as_float(w0.y),
 			            oz = __uint_as_float(w0.z);
-			if (REGULAR || r.kind == 0) {
-				hit = compressed_passes(q, ck, pack2(ox, oy), oz, pack2(sx, sy), sz);
-			} else {
-				const float lx = cdec_f(ox, byte_as_float(ck.x, 0), sx);
-				const float hx = cdec_f(ox, byte_as_float(ck.x, 1), sx);
-				const float ly = cdec_f(oy, byte_as_float(ck.x, 2), sy);
-				const float hy = cdec_f(oy, byte_as_float(ck.x, 3), sy);
-				const float lz = cdec_f(oz, byte_as_float(ck.y, 0), sz);
-				const float hz = cdec_f(oz, byte_as_float(ck.y, 1), sz);
-				hit = conservative_box(r, lx, hx, ly, hy, lz, hz);
-			}
+			hit = compressed_passes(q, ck, pack2(ox, oy), oz, pack2(sx, sy), sz);
 			if (inner) {
 				child = w1.x + __popc(imask & ((1u << k) - 1u));
 			} else {
@@ -492,7 +598,7 @@ __device__ __forceinline__ void packet_descent(const TravArgs &a, const SceneDes
 		for (int c = 0; c < 8; ++c) {
 			bool hit, inner;
 			uint32_t child, leaf_n;
-			test_child<FMT, true>(nodes, r, sr, node, c, hit, inner, child, leaf_n);
+			test_child<FMT, true>(nodes, sr, node, c, hit, inner, child, leaf_n);
 			const uint32_t b = __ballot_sync(0xFFFFFFFFu, hit && mine);
 			if (lane == c)
 				c_rays = b;
@@ -541,8 +647,7 @@ __device__ __forceinline__ void packet_descent(const TravArgs &a, const SceneDes
 
 // The traversal of one batch of up to 32 rays (slots 0..nb-1 of S) through scene sd.
 // REGULAR: every ray of the batch is regular (kind 0), so inner boxes take the plain slab
-// test only (no branch to the conservative test per child).  PACKET: it starts with a packet
-// descent.
+// test only.  PACKET: it starts with a packet descent.
 template <int FMT, bool COUNT, bool LEAF1, bool REGULAR, bool PACKET = false>
 __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uint32_t *queue,
                                             uint32_t *pool, const SceneDesc &sd, uint32_t nb,
@@ -604,7 +709,7 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		__syncwarp(); // the pops above are read before the pushes below overwrite them
 		const uint32_t slot = item >> kIndexBits, node = item & kIndexMask;
 		const RayC r = slot_ray(S, slot);
-		const SlabRay sr = slab_ray(r); // (FP32 nodes)
+		const NodeRay<REGULAR> sr = node_ray<REGULAR>(r);
 		if (COUNT && work && s == 0)
 			++n_visits;
 
@@ -612,7 +717,7 @@ __device__ __forceinline__ void trace_batch(const TravArgs &a, WarpFixed &S, uin
 		uint32_t child[kChildPerLane], leaf_n[kChildPerLane];
 #pragma unroll
 		for (int j = 0; j < kChildPerLane; ++j) {
-			test_child<FMT, REGULAR>(nodes, r, sr, node, s + kLanesPerNode * j, hit[j], inner[j],
+			test_child<FMT, REGULAR>(nodes, sr, node, s + kLanesPerNode * j, hit[j], inner[j],
 			                         child[j], leaf_n[j]);
 			hit[j] = hit[j] && work;
 		}
@@ -938,9 +1043,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				}
 				r = make_ray(p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
 			}
-			if ((PASS == 0 || PASS == 2 || PASS == 4) && r.kind == 1 && a.x_faces.log &&
-			    isinf(r.fx) && x_face_free(a.x_faces, r.ox))
-				r.kind = 3;
+			if ((PASS == 0 || PASS == 2 || PASS == 4) && (r.kind & 7) == 4 && a.x_faces.log &&
+			    x_face_free(a.x_faces, r.ox))
+				--r.kind;
 			S.ro[lane] = make_float4(r.ox, r.oy, r.oz, __int_as_float(r.kind));
 			S.rf[lane] = make_float4(r.fx, r.fy, r.fz, 0.0f);
 			S.rd[lane] = make_float4(r.dx, r.dy, r.dz, 0.0f);
