@@ -99,7 +99,8 @@ struct TravArgs {
 	uint32_t max_batches;    // batches per warp before it exits (0 = no bound)
 	uint32_t batch;          // rays a warp takes at a time: 32, or 4 to 16 where few rays
 	                         // are to keep all warps busy (single_batch, batch_rays)
-	uint32_t claims;         // PASS 4: there are more batches than warps
+	uint32_t claims;         // PASS 4: rays per batch after a warp's first one (0: there are no
+	                         // more batches than warps)
 	uint32_t *counter;
 	uint32_t *deferred;      // [0] batches the regular pass left to the general one,
 	                         // [1] the deferred pass's batch counter
@@ -945,7 +946,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 		// Batches are taken in order from a counter (the deferred pass has its own, so
 		// the few batches it works on spread over all warps); a one-kernel launch (4)
 		// deals out the first ones by warp; a serving launch claims them from its queues.
-		uint32_t base = 0;
+		uint32_t base = 0, take = PASS == 3 ? 32u : a.batch;
 		const SegDesc *segs = a.segs;
 		if (PASS == 3) {
 			uint32_t qsel = 0, batch = 0;
@@ -981,8 +982,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				if (base == kNone) { // the next one that no warp has
 					if (!a.claims)
 						break;
+					take = a.claims;
 					if (lane == 0)
-						base = atomicAdd(a.counter, a.batch) +
+						base = atomicAdd(a.counter, a.claims) +
 						       gridDim.x * (blockDim.x >> 5) * a.batch;
 					base = __shfl_sync(0xFFFFFFFFu, base, 0);
 				}
@@ -1018,7 +1020,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 		const uint32_t run_rays = S.seg.n_rays;
 		if (local >= run_rays)
 			continue; // padding of the run
-		const uint32_t nb = min(PASS == 3 ? 32u : a.batch, run_rays - local);
+		const uint32_t nb = min(take, run_rays - local);
 		const SceneDesc sd = (PASS == 3 || a.n_segs) ? a.scenes[S.seg.scene] : a.scene0;
 		const float4 *__restrict__ tri4 = sd.tri4;
 
@@ -1245,22 +1247,31 @@ int warps_for(const TravConfig &cfg) {
 // one zero direction component starts when all others are done; but with the plain test alone
 // they need fewer registers, which pays in the end.
 //
-// Ray buffers.  One round of batches while 8 rays a warp suffice, else batches claimed from
-// the counter.  Speed against a regular and a deferred pass (mean over five scenes / least of
-// them; FP32 nodes, one triangle per leaf), batches of 8, 16, 32:
-//     30,000     1.34 / 1.16    0.95 / 0.88    0.66 / 0.54
-//     100,000    1.09 / 1.01    0.93 / 0.90    0.77 / 0.67
-//     300,000    1.08 / 0.98    1.03 / 0.96    0.92 / 0.88
-//     600,000    1.38 / 0.92    1.38 / 0.97    1.25 / 0.95
-//     1,300,000  1.33 / 0.95    1.41 / 0.97    1.34 / 0.96
-//     2,000,000  1.11 / 0.93    1.22 / 0.95    1.23 / 0.95
-// (the means above 1.2 come from rays with zero components).  With compressed nodes or
-// larger leaves 16 loses up to 8 % from 900,000 on where no ray is deferred.  With FP32 nodes
-// and one triangle per leaf a small scene's batch is short, and larger ones pay sooner (us; two passes / 8 / 16 / 32):
+// Ray buffers.  One round of batches while 8 rays a warp suffice; when that leaves a quarter
+// of the rays or less, they are claimed by fours, so that the second round is short (39,000
+// to 50,000 rays 4 to 8 % faster, at most 20 %; with eights some were up to 9 % slower than as
+// two passes); else batches claimed from the counter.  Speed against a regular and a
+// deferred pass (mean over eight scenes, least of them; FP32 nodes, one triangle per leaf), of
+// regular rays alone and with a zero x component in every 977th:
+//                        regular                               with zeros
+//     batches of   8          12         16         32         8          16         32
+//     20,000       1.17 1.10  1.08 0.96  1.01 0.81  0.78 0.52  1.44 1.09  1.21 0.98  0.95 0.59
+//     100,000      1.09 1.01  1.10 0.99  1.07 0.91  1.04 0.85  1.41 1.20  1.32 1.02  1.17 0.85
+//     250,000      1.03 0.88  1.06 1.00  1.07 1.00  1.05 0.95  1.41 1.25  1.44 1.23  1.31 1.09
+//     600,000      0.95 0.73  1.00 0.88  1.04 0.98  1.03 0.96  1.38 1.09  1.49 1.19  1.37 1.10
+//     1,300,000    0.87 0.72  0.93 0.81  0.98 0.94  1.00 0.95  1.17 1.04  1.26 1.08  1.25 1.05
+//     2,000,000    0.83 0.66  0.89 0.75  0.95 0.89  0.99 0.95  1.07 0.91  1.18 1.04  1.19 1.02
+// So from 600,000 on a query without any such ray may lose up to 5 % against two passes, and
+// one with a few gains 19 to 49 % (any camera of even width has them).  With compressed nodes or
+// larger leaves the loss would be up to 10 % from 900,000 on, so two passes take those.
+// Batches of rays that mostly miss are short, and eights cost them 11 % at 250,000 to 310,000
+// rays: twelves there.  With FP32 nodes and one triangle per leaf a small scene's batch is
+// short as well (us; two passes / 8 / 16 / 32):
 //     64 triangles       60,000  20 / 15 / 11 / 12    320,000  41 / 43 / 35 / 31
 //                     1,300,000  103 / 154 / 119 / 98
 //     2,500 triangles    60,000  52 / 28 / 37 / 51    320,000  75 / 76 / 70 / 72
 //                     1,300,000  288 / 272 / 233 / 218
+// (Nine blocks per SM, 56 registers: 4 % slower for regular rays, 2 to 4 % for others.)
 //
 // Several runs (padded to whole warps of 32).  One round of batches of 4, 8 or 16.  Batch
 // graphs, us: 20 scenes of up to 6,836 triangles and 5,762 rays 324 -> 273, 48 of 18,789 and
@@ -1273,6 +1284,7 @@ int warps_for(const TravConfig &cfg) {
 //     256        75 / 60 / 59 / 61        166 / 119 / 103 / 96     440 / 299 / 239 / 210
 //     4,968      105 / 110 / 140 / 148    207 / 171 / 183 / 183    515 / 383 / 332 / 311
 //     65,536     202 / 218 / 277 / 287    284 / 274 / 288 / 294    638 / 514 / 464 / 472
+// (12 triangles, 900 x 600: batches of 16 / 32 47 / 40.)
 uint32_t single_batch(const TravArgs &a, const TravConfig &cfg, uint64_t slots) {
 	const uint64_t n = a.n_virtual, per = (n + slots - 1) / slots;
 	if (a.n_segs)
@@ -1281,18 +1293,25 @@ uint32_t single_batch(const TravArgs &a, const TravConfig &cfg, uint64_t slots) 
 		return ((uint32_t)per + 3u) & ~3u;
 	if (a.use_cam) {
 		const bool wide = n >= 640ull * a.scene0.n_tris;
+		if (wide && per > 120u)
+			return 0u;
 		if (wide)
-			return per <= 32u ? 8u : per <= 120u ? 16u : 0u;
+			return per <= 32u ? 8u : per > 64u && a.scene0.n_tris <= 64u ? 32u : 16u;
 		return per <= 120u ? 8u : per <= 450u ? 16u : 32u;
 	}
 	if (cfg.format != PRT_NODES_FP32 || a.max_leaf > 1u) {
 		const bool tiny = a.scene0.n_tris <= 256u; // (as the small scenes below)
-		return per <= (tiny ? 32u : 64u) ? 8u : per > 130u ? 0u : tiny && per > 64u ? 32u : 16u;
+		return per <= (tiny ? 32u : 36u) ? 8u
+		       : per <= 64u              ? (tiny ? 16u : 12u)
+		       : per <= 130u             ? (tiny ? 32u : 16u)
+		                                 : 0u;
 	}
 	const bool small = a.scene0.n_tris <= 4096u;
-	if (per <= (small ? 16u : 64u))
+	if (per <= (small ? 16u : 36u))
 		return 8u;
-	return per <= (small ? 64u : 300u) ? 16u : per <= 420u ? 32u : 0u;
+	if (per <= 64u)
+		return small ? 16u : 12u;
+	return per <= 300u && !small ? 16u : per <= 420u ? 32u : 0u;
 }
 
 template <int FMT, bool LEAF1>
@@ -1302,7 +1321,8 @@ bool launch_single(TravArgs a, const TravConfig &cfg, int warps, int sm_count, c
 	a.batch = single_batch(a, cfg, slots);
 	if (!a.batch)
 		return false;
-	a.claims = (uint64_t)a.batch * slots < a.n_virtual ? 1u : 0u;
+	const uint64_t dealt = (uint64_t)a.batch * slots;
+	a.claims = dealt >= a.n_virtual ? 0u : 4u * dealt >= 3u * (uint64_t)a.n_virtual ? 4u : a.batch;
 	if (a.claims && cudaMemsetAsync(a.counter, 0, 4, st) != cudaSuccess)
 		return true; // (dispatch reports the error)
 	launch_t<FMT, false, LEAF1, false, 4>(a, warps, sm_count, st);
