@@ -1,12 +1,15 @@
 // A CUDA runtime without a GPU, for tests of host code: preloaded before libcudart it gives the
 // library one device of compute capability 10.3 that reads pageable memory, whose memory is
 // the host's and whose kernels do nothing.  It remembers which streams hold work that nobody
-// has waited for, and a test can make a later kernel launch fail.
+// has waited for and the names of the kernels launched, and a test can make a later launch
+// fail.
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <set>
+#include <string>
 
 #define FAKE extern "C" __attribute__((visibility("default")))
 
@@ -14,6 +17,11 @@ namespace {
 std::set<void *> pending; // streams with work in flight
 long fail_in = 0;         // the launch that fails, counted down (0: none)
 cudaError_t last = cudaSuccess;
+std::map<const void *, std::string> &names() { // of kernels, by their host functions
+	static std::map<const void *, std::string> m;
+	return m;
+}
+std::string launched; // names, one per line
 char handles[4096];
 int n_handles = 0;
 
@@ -22,7 +30,8 @@ cudaError_t queued(void *st) {
 	pending.insert(st);
 	return cudaSuccess;
 }
-cudaError_t launch(void *st) {
+cudaError_t launch(void *st, const void *fun = nullptr) {
+	launched += names()[fun] + "\n";
 	if (fail_in > 0 && --fail_in == 0)
 		return last = cudaErrorLaunchOutOfResources;
 	return queued(st);
@@ -31,6 +40,8 @@ cudaError_t launch(void *st) {
 
 FAKE void fake_fail_launch(long k) { fail_in = k; }
 FAKE long fake_pending() { return (long)pending.size(); }
+FAKE const char *fake_launched() { return launched.c_str(); }
+FAKE void fake_forget_launched() { launched.clear(); }
 
 FAKE cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
 FAKE cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
@@ -129,17 +140,17 @@ FAKE cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, 
                                                                          size_t, unsigned) {
 	return *n = 8, cudaSuccess;
 }
-FAKE cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) {
-	return launch(c->stream);
+FAKE cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *fun, void **) {
+	return launch(c->stream, fun);
 }
-FAKE cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t st) {
-	return launch(st);
+FAKE cudaError_t cudaLaunchKernel(const void *fun, dim3, dim3, void **, size_t, cudaStream_t st) {
+	return launch(st, fun);
 }
-FAKE cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void **, size_t, cudaStream_t st) {
-	return launch(st);
+FAKE cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **, size_t, cudaStream_t st) {
+	return launch(st, k);
 }
-FAKE cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *) {
-	return *k = static_cast<cudaKernel_t>(new_handle()), cudaSuccess;
+FAKE cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *fun) {
+	return *k = static_cast<cudaKernel_t>(const_cast<void *>(fun)), cudaSuccess;
 }
 namespace {
 cudaStream_t configured;
@@ -153,6 +164,8 @@ FAKE cudaError_t __cudaPopCallConfiguration(dim3 *, dim3 *, size_t *, void *st) 
 FAKE void **__cudaRegisterFatBinary(void *) { return static_cast<void **>(new_handle()); }
 FAKE void __cudaRegisterFatBinaryEnd(void **) {}
 FAKE void __cudaUnregisterFatBinary(void **) {}
-FAKE void __cudaRegisterFunction(void **, const char *, char *, const char *, int, uint3 *, uint3 *,
-                                 dim3 *, dim3 *, int *) {}
+FAKE void __cudaRegisterFunction(void **, const char *fun, char *, const char *name, int, uint3 *,
+                                 uint3 *, dim3 *, dim3 *, int *) {
+	names()[fun] = name;
+}
 FAKE void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
