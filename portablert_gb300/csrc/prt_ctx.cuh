@@ -177,13 +177,18 @@ int guarded(ErrorText *err, const char *what, F &&body, cudaStream_t capture = n
 // The address under which the device reaches host buffer p in place, or null: pinned
 // (page-locked, registered) memory through its device alias, pageable memory when the
 // device reads it through the host's page tables (Grace: NVLink-C2C with address
-// translation), managed and device memory as they are.
-inline void *device_alias(const prt_b200_ctx *ctx, const void *p) {
+// translation), managed and device memory as they are.  *pageable: whether p is memory that
+// CUDA knows nothing of.
+inline void *device_alias(const prt_b200_ctx *ctx, const void *p, bool *pageable = nullptr) {
 	cudaPointerAttributes a;
+	if (pageable)
+		*pageable = false;
 	if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
 		cudaGetLastError();
 		return nullptr;
 	}
+	if (pageable)
+		*pageable = a.type == cudaMemoryTypeUnregistered;
 	switch (a.type) {
 	case cudaMemoryTypeHost:
 		return a.devicePointer;
