@@ -102,7 +102,9 @@ __global__ void k_clear_error(uint32_t *err, uint32_t bits) { clear_error_bits(e
 
 // Empty bounds, and no split after each scene's last leaf.
 __global__ void k_bounds_init(uint32_t *gb, uint32_t n_scenes, const uint32_t *tri_off,
-                              uint4 *splits) {
+                              uint4 *splits, uint32_t *x_drop) {
+	if (x_drop && blockIdx.x == 0 && threadIdx.x == 0)
+		x_drop[0] = 1u;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 * n_scenes;
 	     i += gridDim.x * blockDim.x) {
 		gb[i] = (i % 6) < 3 ? 0xFFFFFFFFu : 0u;
@@ -1059,6 +1061,14 @@ __global__ void __launch_bounds__(8 * kCollapseItems)
 
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
+// log2 of the bits of XFaces for n triangles.
+inline uint32_t x_faces_log(uint64_t n) {
+	uint32_t log = 10;
+	while ((1ull << log) < 8ull * n)
+		++log;
+	return log;
+}
+
 } // namespace
 
 int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compressed,
@@ -1154,19 +1164,19 @@ int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compre
 		BUILD_TRY(ws.sah.reserve(sah_scratch_bytes(n, S)));
 		BUILD_TRY(ws.roots.reserve(4ull * S));
 	}
-	plan.x_log = 0;
-	if (sah && !plan.small && !plan.multi && n) {
-		uint32_t log = 10;
-		while ((1ull << log) < 8ull * n)
-			++log;
-		BUILD_TRY(sc.x_faces.reserve(4ull * (kXHead + (1ull << (log - 5u)))));
-		plan.x_log = log;
-	}
 	if (collapse_cost)
 		BUILD_TRY(ws.cost.reserve(sizeof(CostNode) * ni));
 	BUILD_TRY(sc.tri4.reserve(48 * nn));
 	BUILD_TRY(sc.inv.reserve(4 * nn));
 	// One node past the capacity: the empty node the traversal pads partial steps with.
+	// As large as the triangle records' buffer may need: it moves only when that does, so that a
+	// captured query that still finds the one finds the other.
+	plan.x_log = 0;
+	if (sah && !plan.small && !plan.multi && n) {
+		BUILD_TRY(sc.x_faces.reserve(4ull * (kXHead + (1ull << (x_faces_log(sc.tri4.bytes / 48) - 5u)))));
+		plan.x_log = x_faces_log(n);
+	}
+	plan.x_drop = plan.x_log ? nullptr : sc.x_faces.as<uint32_t>();
 	BUILD_TRY(sc.nodes.reserve(sizeof(Node8) * ((size_t)plan.node_cap + 1)));
 	if (compressed)
 		BUILD_TRY(sc.cnodes.reserve(sizeof(CNode8) * ((size_t)plan.node_cap + 1)));
@@ -1195,7 +1205,7 @@ static int lbvh_enqueue(const float *d_tris, const BuildPlan &plan, BuildScratch
 	uint32_t *gb = ws.bounds.as<uint32_t>();
 	svals = ws.vals.as<uint32_t>();
 	k_bounds_init<<<blocks_for(6ull * S, 256), 256, 0, st>>>(gb, S, d_toff,
-	                                                         ws.splits.as<uint4>());
+	                                                         ws.splits.as<uint4>(), plan.x_drop);
 	if (n)
 		k_centroid_bounds<<<std::min(blocks_for(n, 256), 2048u), 256, 0, st>>>(d_tris, n, scene_of,
 		                                                                        gb);
@@ -1379,7 +1389,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
 		uint32_t *ctr = ws.counters.as<uint32_t>();
 		BUILD_TRY(launch_build_small(d_tris, n, (uint32_t)plan.leaf_size, plan.collapse_cost,
 		                             plan.compressed, ws, sc, plan.node_cap, ctr, ws.h_counters,
-		                             d_err, st));
+		                             plan.x_drop, d_err, st));
 		sc.built_small = true;
 		if (plan.compressed) {
 			k_compress<<<blocks_for(8ull * plan.node_cap, 256), 256, 0, st>>>(

@@ -124,6 +124,7 @@ struct BuildPlan {
 	int leaf_size = 1, scene_digits = 0;
 	bool compressed = false, multi = false;
 	uint32_t x_log = 0;               // log2 of SceneGPU::x_faces' bits (0: not built)
+	uint32_t *x_drop = nullptr;       // the set of an earlier build, to be marked unusable
 	bool sah = false;                 // binned-SAH binary trees instead of LBVH
 	bool collapse_cost = true;        // cost-optimal 8-wide collapse (else largest area first)
 	bool small = false;               // one scene of 1..small_build_max() triangles, with the
@@ -178,6 +179,7 @@ int build_scene(const float *d_tris, uint64_t n, int leaf_size, bool compressed,
 uint32_t small_build_max();
 cudaError_t launch_build_small(const float *d_tris, uint32_t n, uint32_t leaf_size, bool use_cost,
                                bool compressed, BuildScratch &ws, SceneGPU &sc, uint32_t node_cap,
-                               uint32_t *ctr, uint32_t *h_ctr, uint32_t *d_err, cudaStream_t st);
+                               uint32_t *ctr, uint32_t *h_ctr, uint32_t *x_drop, uint32_t *d_err,
+                               cudaStream_t st);
 
 } // namespace prt

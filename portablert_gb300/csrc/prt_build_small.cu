@@ -274,10 +274,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                   CostNode *__restrict__ cost, Node8 *__restrict__ nodes, uint32_t node_cap,
                   float4 *__restrict__ tri4, uint32_t *__restrict__ inv, uint32_t *__restrict__ ctr,
                   uint32_t *__restrict__ hctr, Node8 *__restrict__ dead, CNode8 *__restrict__ cdead,
-                  uint32_t *__restrict__ err) {
+                  uint32_t *__restrict__ x_drop, uint32_t *__restrict__ err) {
 	extern __shared__ __align__(16) unsigned char sm[];
 	uint32_t *scan = reinterpret_cast<uint32_t *>(sm + kOffScan);
 	const uint32_t tid = threadIdx.x;
+	if (x_drop && tid == 0)
+		x_drop[0] = 1u; // (this build makes no XFaces)
 	float *box = reinterpret_cast<float *>(sm + kOffBox);
 	uint32_t *word = reinterpret_cast<uint32_t *>(sm + kOffWord);
 	float *crow = reinterpret_cast<float *>(sm + kOffCost);
@@ -884,7 +886,8 @@ uint32_t small_build_max() { return kSmallMax; }
 
 cudaError_t launch_build_small(const float *d_tris, uint32_t n, uint32_t leaf_size, bool use_cost,
                                bool compressed, BuildScratch &ws, SceneGPU &sc, uint32_t node_cap,
-                               uint32_t *ctr, uint32_t *h_ctr, uint32_t *d_err, cudaStream_t st) {
+                               uint32_t *ctr, uint32_t *h_ctr, uint32_t *x_drop, uint32_t *d_err,
+                               cudaStream_t st) {
 	// The shared-memory limit is a per-device attribute: set once per device.
 	static std::atomic<uint32_t> attr_set{0};
 	int dev = 0;
@@ -909,7 +912,7 @@ cudaError_t launch_build_small(const float *d_tris, uint32_t n, uint32_t leaf_si
 	    ws.left.as<uint32_t>(), use_cost ? ws.cost.as<CostNode>() : nullptr,
 	    sc.nodes.as<Node8>(), node_cap, sc.tri4.as<float4>(), sc.inv.as<uint32_t>(), ctr, h_dev,
 	    sc.nodes.as<Node8>() + sc.dead, compressed ? sc.cnodes.as<CNode8>() + sc.dead : nullptr,
-	    d_err);
+	    x_drop, d_err);
 	return cudaGetLastError();
 }
 

@@ -216,7 +216,9 @@ __device__ __forceinline__ float child_hi(float c, float e) { return __fadd_ru(c
 
 // Set of the x coordinates at which some triangle's box of a scene has its lower face: a
 // hash set of 2^log bits (8 to 16 per triangle) after kXHead words, of which the first is
-// set when a triangle is not finite.  log 0: there is no set, every x may be one.
+// set when every x may be one (a triangle is not finite, or a later build made no set) and the
+// second holds log: a query captured in a graph reads both when it runs, whatever has been
+// built into the scene's buffers since.  Builders take log 0 for no set.
 // A ray with a zero x component passed every box around its x, thousands of nodes that were
 // the tail of the launch; off the faces y and z now prune (16,000 camera and secondary rays on
 // a 65,790-triangle heightfield 39 -> 23 us, 6,000 through the host call 63 -> 48; the build
@@ -234,9 +236,12 @@ __device__ __forceinline__ void x_face_add(const XFaces &f, float x) {
 	atomicOr(f.words + kXHead + (k >> 5), bit);
 }
 // Whether no triangle's lower x face is at x.
-__device__ __forceinline__ bool x_face_free(const XFaces &f, float x) {
-	const uint32_t k = x_face_bit(x, f.log);
-	return __ldg(f.words) == 0u && !((__ldg(f.words + kXHead + (k >> 5)) >> (k & 31u)) & 1u);
+__device__ __forceinline__ bool x_face_free(const uint32_t *words, float x) {
+	const uint2 head = __ldg(reinterpret_cast<const uint2 *>(words));
+	if (head.x)
+		return false;
+	const uint32_t k = x_face_bit(x, head.y);
+	return !((__ldg(words + kXHead + (k >> 5)) >> (k & 31u)) & 1u);
 }
 
 // Slab test of portableRT's ray_box_intersect (bvh.hpp:195-222), bit for bit: each

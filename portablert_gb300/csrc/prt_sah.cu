@@ -1401,7 +1401,7 @@ __global__ void k_sah_bounds_init(uint32_t *gb, uint32_t n_scenes, XFaces x_face
 		const uint32_t quads = (kXHead + (1u << (x_faces.log - 5u))) / 4u;
 		for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < quads;
 		     i += gridDim.x * blockDim.x)
-			reinterpret_cast<uint4 *>(x_faces.words)[i] = make_uint4(0u, 0u, 0u, 0u);
+			reinterpret_cast<uint4 *>(x_faces.words)[i] = make_uint4(0u, i ? 0u : x_faces.log, 0u, 0u);
 	}
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 * n_scenes;
 	     i += gridDim.x * blockDim.x)

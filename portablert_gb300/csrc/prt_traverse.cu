@@ -108,7 +108,7 @@ struct TravArgs {
 	unsigned long long *visits;
 	uint32_t use_cam;        // 1: rays of the single run come from `cam`, not seg0.rays
 	prt_b200_camera cam;
-	XFaces x_faces;          // of the single run's scene
+	const uint32_t *x_faces; // of the single run's scene (XFaces; null: none)
 	ServeQueues serve;       // PASS 3 only
 };
 
@@ -1045,7 +1045,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				}
 				r = make_ray(p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
 			}
-			if ((PASS == 0 || PASS == 2 || PASS == 4) && (r.kind & 7) == 4 && a.x_faces.log &&
+			if ((PASS == 0 || PASS == 2 || PASS == 4) && (r.kind & 7) == 4 && a.x_faces &&
 			    x_face_free(a.x_faces, r.ox))
 				--r.kind;
 			S.ro[lane] = make_float4(r.ox, r.oy, r.oz, __int_as_float(r.kind));
@@ -1444,7 +1444,7 @@ cudaError_t launch_nearest_hits(const SceneGPU &sc, const float *d_rays, uint64_
 		a.scene0.nodes = cfg.format == PRT_NODES_COMPRESSED ? sc.cnodes.p : sc.nodes.p;
 		a.scene0.root = 0;
 		a.scene0.n_tris = (uint32_t)sc.n_tris;
-		a.x_faces = XFaces{sc.x_faces.as<uint32_t>(), sc.x_log};
+		a.x_faces = sc.x_log ? sc.x_faces.as<uint32_t>() : nullptr;
 		a.seg0.vbegin = 0;
 		a.seg0.rays = cam ? nullptr : d_rays + 6 * s;
 		a.seg0.out = static_cast<uint8_t *>(d_out) + s * lay.rec_size;
