@@ -113,29 +113,26 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 }
 
 // Per-ray constants.  `kind` selects the box test used on inner nodes (prt_traverse.cu):
-//   0 regular: every origin component within 2^67 and every direction component between
-//              2^-58 and 2^60 in magnitude: the slab test on centres and half extents
-//              (SlabRay) neither overflows nor meets a NaN.
-//   2 all:     a non-finite component, all reciprocals infinite or all origin components
-//              past 2^67: every inner box passes and only the exact per-triangle test
-//              decides.
-//   3 axis:    any other ray, for instance with a zero direction component (infinite
-//              reciprocal): the same test with such axes reduced (AxisRay).
-//   4 axis, x: like 3 with an infinite reciprocal on the x axis, where some triangle's box
+//   0 regular: finite, every origin component within 2^67 and every direction component at
+//              least 2^-58 in magnitude: the slab test on centres and half extents (SlabRay)
+//              neither overflows nor meets a NaN.
+//   2 all:     a non-finite component or all reciprocals infinite: every inner box passes
+//              and only the exact per-triangle test decides.
+//   3 other:   any other ray, for instance with a zero direction component (infinite
+//              reciprocal): the slab test on bounds (AxisRay).
+//   4 x:       like 3 with an infinite reciprocal on the x axis, where some triangle's box
 //              may have its lower x face at the origin's x (XFaces): a box around it
 //              passes outright.
-// Kinds 3 and 4 have kOdd set where more than infinite reciprocals sets the ray apart.
-constexpr int kOdd = 8;
 struct RayC {
 	float ox, oy, oz, dx, dy, dz, fx, fy, fz;
 	int kind;
 };
 
-// (2^67 + 2^67) * 2^58 stays below FLT_MAX; 2^67 is about 1.5e20.
-constexpr float kCoordMax = 0x1p67f, kDirMax = 0x1p60f, kDirMin = 0x1p-58f;
+// (2^67 + 2^67) * 2^58 stays below FLT_MAX; 2^67 is about 1.5e20, 2^-58 about 3.5e-18.
+constexpr float kCoordMax = 0x1p67f, kDirMin = 0x1p-58f, kFltMax = 0x1.fffffep127f;
 
 __device__ __forceinline__ bool dir_regular(float d) {
-	return fabsf(d) <= kDirMax && fabsf(d) >= kDirMin;
+	return fabsf(d) <= kFltMax && fabsf(d) >= kDirMin;
 }
 
 __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx, float dy,
@@ -156,13 +153,7 @@ __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx,
 		const bool fin = isfinite(ox) && isfinite(oy) && isfinite(oz) && isfinite(dx) &&
 		                 isfinite(dy) && isfinite(dz);
 		const bool ix = isinf(r.fx), iy = isinf(r.fy), iz = isinf(r.fz);
-		const bool px = fabsf(ox) > kCoordMax, py = fabsf(oy) > kCoordMax,
-		           pz = fabsf(oz) > kCoordMax;
-		const bool odd = px || py || pz || !(ix || dir_regular(dx)) || !(iy || dir_regular(dy)) ||
-		                 !(iz || dir_regular(dz));
-		r.kind = !fin || (ix && iy && iz) || (px && py && pz)
-		             ? 2
-		             : (ix ? 4 : 3) + (odd ? kOdd : 0);
+		r.kind = !fin || (ix && iy && iz) ? 2 : ix ? 4 : 3;
 	}
 	return r;
 }
@@ -173,7 +164,7 @@ __device__ __forceinline__ RayC make_ray(float ox, float oy, float oz, float dx,
 __device__ __forceinline__ void encode_axis(float lo, float hi, float &c, float &e) {
 	if (!(lo >= -kCoordMax && hi <= kCoordMax)) {
 		c = 0.0f;
-		e = 3.402823466e+38f;
+		e = kFltMax;
 		return;
 	}
 	c = __fadd_rn(__fmul_rn(lo, 0.5f), __fmul_rn(hi, 0.5f));

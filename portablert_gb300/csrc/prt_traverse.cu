@@ -242,90 +242,82 @@ __device__ __forceinline__ bool child_passes(const SlabRay &q, const float4 &a, 
 	return tmin <= __fmaf_rn(tmax, 1.0f + 0x1p-20f, 0x1p-120f);
 }
 
-// The same test for any other ray (and for a regular one in a batch with such).  `g` and `h`
-// scale near and far, 1 on an axis that is regular.
+// The box test of any other ray (and of a regular one in a batch with such): on bounds, which
+// a record's centre and half extent give rounded outwards, with the reference's own
+// (bound - origin) * reciprocal.  That is monotone in the bound, infinities included, so it
+// passes whatever the reference passes inside without a margin.
 //
 // An axis of infinite reciprocal (a zero component) takes +-1 in the reciprocal's place, so
 // that its near and far tell by their signs, exactly, whether the origin lies before, inside
-// or behind the (widened) extent, and is scaled by infinity to what the reference's slab test
-// works with: two equal infinities outside, -inf and +inf inside, where a face's NaN
-// removes y or z from its test.  The face's 0 * inf here is a NaN too, which max3f and min3f
-// pass over.  On the x axis the reference's whole test passes at a lower face, so of kind 4 a
-// box with the origin's x inside passes outright.
-//
-// Odd rays (kOdd): a reciprocal above 2^58 counts as 2^58, which is no more than the
-// reference's near ahead of the origin, with far scaled by infinity; an axis whose origin
-// is past 2^67 is left out (0 * inf).  A reciprocal below 2^-60 needs nothing: the margin's
-// 2^-120 covers what underflow loses.
+// or behind the box, and `g`, infinite there and 1 elsewhere, scales them to what the
+// reference's slab test works with: two equal infinities outside, -inf and +inf inside, where
+// a face's NaN removes y or z from its test.  The face's 0 * inf here is a NaN too, which
+// max3f and min3f pass over (all axes may be: nothing constrains then).  On the x axis the
+// reference's whole test passes at a lower face, so of kind 4 a box with the origin's x
+// inside passes outright.
 //
 // Why: rays in a plane of two axes, a camera's middle row and column among them, are the
-// longest chains of their launch.  Bounds stored as such and a branch per axis / bounds
-// decoded from centre and half extent / this, us: 2,400,000 rays in a z plane of the
-// 1,048,576-triangle heightfield 679 / 721 / 599, 400,000 in an x plane that holds faces
-// 12,734 / 13,513 / 12,254, 320 x 200 pixels on 65,536 triangles 118 / 117 / 108.  (As a third
-// instance of trace_batch, or as a branch for odd rays in the second, those cost regular rays
-// 3 % in registers.)
+// longest chains of their launch.  Bounds stored as such and a branch per axis / decoded, with
+// those branches / this, us: 2,400,000 rays in a z plane of the 1,048,576-triangle
+// heightfield 679 / 721 / 578, 400,000 in an x plane that holds faces 12,734 / 13,513 / 12,121,
+// 320 x 200 pixels on 65,536 triangles 118 / 117 / 108.  (The test on centre and half extent
+// with the axes reduced the same way: 599 / 12,254 / 108, and 2 % slower for regular rays, by
+// its registers; as a third instance of trace_batch 3 %.)
 struct AxisRay {
-	SlabRay q;
-	unsigned long long g, h; // x and y
-	float gz, hz;
-	float ox;
+	unsigned long long no, f, g; // x and y: -origin, reciprocal, scale
+	float noz, fz, gz;
 	bool inf_x, x_passes, all;
 };
 
-__device__ __forceinline__ void axis_scale(float o, float &f, float &g, float &h, bool odd) {
-	const bool inf = isinf(f);
-	g = h = inf ? INFINITY : 1.0f;
-	f = inf ? copysignf(1.0f, f) : f;
-	if (odd && !inf) {
-		if (fabsf(o) > kCoordMax) {
-			f = 0.0f;
-			g = h = INFINITY;
-		} else if (fabsf(f) > 1.0f / kDirMin) {
-			f = copysignf(1.0f / kDirMin, f);
-			h = INFINITY;
-		}
-	}
-}
-
 __device__ __forceinline__ AxisRay axis_ray(const RayC &r) {
-	RayC m = r;
-	float gx, gy, hx, hy;
+	const bool ix = isinf(r.fx), iy = isinf(r.fy), iz = isinf(r.fz);
 	AxisRay x;
-	axis_scale(r.ox, m.fx, gx, hx, r.kind & kOdd);
-	axis_scale(r.oy, m.fy, gy, hy, r.kind & kOdd);
-	axis_scale(r.oz, m.fz, x.gz, x.hz, r.kind & kOdd);
-	x.q = slab_ray(m);
-	x.g = pack2(gx, gy);
-	x.h = pack2(hx, hy);
-	x.ox = r.ox;
-	x.inf_x = isinf(r.fx);
-	x.x_passes = (r.kind & 7) == 4;
+	x.no = pack2(-r.ox, -r.oy);
+	x.f = pack2(ix ? copysignf(1.0f, r.fx) : r.fx, iy ? copysignf(1.0f, r.fy) : r.fy);
+	x.g = pack2(ix ? INFINITY : 1.0f, iy ? INFINITY : 1.0f);
+	x.noz = -r.oz;
+	x.fz = iz ? copysignf(1.0f, r.fz) : r.fz;
+	x.gz = iz ? INFINITY : 1.0f;
+	x.inf_x = ix;
+	x.x_passes = r.kind == 4;
 	x.all = r.kind == 2;
 	return x;
 }
 
+// Bounds: lower x and y, upper x and y, lower and upper z; outside: known to be so on an x axis
+// of infinite reciprocal.
+__device__ __forceinline__ bool axis_passes(const AxisRay &x, unsigned long long l,
+                                            unsigned long long h, unsigned long long z,
+                                            bool outside) {
+	float t1, t2, t3, t4, t5, t6, gx, gy;
+	unpack2(mul2(add2(l, x.no), x.f), t1, t3);
+	unpack2(mul2(add2(h, x.no), x.f), t2, t4);
+	unpack2(mul2(add2(z, pack2(x.noz, x.noz)), pack2(x.fz, x.fz)), t5, t6);
+	unpack2(x.g, gx, gy);
+	float nx = fminf(t1, t2) * gx;
+	const float fx = fmaxf(t1, t2) * gx;
+	if (outside)
+		nx = INFINITY; // (fx is +inf or a NaN if the bounds hold the origin)
+	const bool outright = x.all || (x.x_passes && !(nx > 0.0f) && !(fx < 0.0f));
+	const float tmin = max3f(nx, fminf(t3, t4) * gy, fmaxf(fminf(t5, t6) * x.gz, 0.0f));
+	const float tmax = min3f(fx, fmaxf(t3, t4) * gy, fmaxf(t5, t6) * x.gz);
+	return outright || !(tmin > tmax);
+}
+
 __device__ __forceinline__ bool child_passes(const AxisRay &x, const float4 &a, const float4 &b) {
-	const SlabRay &q = x.q;
-	const unsigned long long t = mul2(add2(pack2(a.x, a.y), q.no), q.f);
-	const unsigned long long e = pack2(a.z, a.w);
-	float nx, ny, fx, fy;
-	unpack2(mul2(fma2(e, q.naf, t), x.g), nx, ny);
-	unpack2(mul2(fma2(e, q.af, t), x.h), fx, fy);
-	const float tz = (b.x - q.oz) * q.fz;
-	const float nz = __fmaf_rn(-b.y, q.afz, tz) * x.gz, fz = __fmaf_rn(b.y, q.afz, tz) * x.hz;
-	bool outright = x.all;
+	unsigned long long l, h;
+	const unsigned long long c = pack2(a.x, a.y), e = pack2(a.z, a.w);
+	asm("sub.rm.f32x2 %0, %1, %2;" : "=l"(l) : "l"(c), "l"(e)); // child_lo
+	asm("add.rp.f32x2 %0, %1, %2;" : "=l"(h) : "l"(c), "l"(e)); // child_hi
+	bool outside = false;
 	if (x.inf_x) {
+		float ox, oy;
+		unpack2(x.no, ox, oy);
 		// (Closer bounds: the widened extent of a box that ends near 0 reaches over it.)
 		const uint32_t x16 = __float_as_uint(b.w);
-		if (x.ox < __uint_as_float(x16 << 16) || x.ox > __uint_as_float(x16 & 0xFFFF0000u))
-			nx = INFINITY; // (outside; fx is +inf or a NaN if the test above saw it inside)
-		outright = outright || (x.x_passes && !(nx > 0.0f) && !(fx < 0.0f));
+		outside = -ox < __uint_as_float(x16 << 16) || -ox > __uint_as_float(x16 & 0xFFFF0000u);
 	}
-	const float tmin = max3f(nx, ny, fmaxf(nz, 0.0f));
-	const float tmax = min3f(fx, fy, fz);
-	// (Every axis may be a NaN: then nothing constrains.)
-	return outright || !(tmin > __fmaf_rn(tmax, 1.0f + 0x1p-20f, 0x1p-120f));
+	return axis_passes(x, l, h, pack2(child_lo(b.x, b.y), child_hi(b.x, b.y)), outside);
 }
 
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return (w >> (8 * k)) & 0xFFu; }
@@ -342,54 +334,45 @@ __device__ __forceinline__ float byte_biased(uint32_t w, int k) {
 	return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)k));
 }
 
-// regular_box on child record ck of a compressed node with origin (oxy, oz) and scales
-// (sxy, sz): the same decode (cdec_f) and products, every operation rounded as the scalar one,
-// x and y and the two z bounds in packed pairs: 12 FP instructions for 24 (a traversal of
+// The bounds of child record ck of a compressed node with origin (oxy, oz) and scales (sxy,
+// sz) as axis_passes takes them: the same decode (cdec_f), x and y and the two z in pairs.
+__device__ __forceinline__ void compressed_bounds(const uint2 &ck, unsigned long long oxy, float oz,
+                                                  unsigned long long sxy, float sz,
+                                                  unsigned long long &l, unsigned long long &h,
+                                                  unsigned long long &z) {
+	const unsigned long long bias = pack2(-8388608.0f, -8388608.0f);
+	l = fma2(add2(pack2(byte_biased(ck.x, 0), byte_biased(ck.x, 2)), bias), sxy, oxy);
+	h = fma2(add2(pack2(byte_biased(ck.x, 1), byte_biased(ck.x, 3)), bias), sxy, oxy);
+	z = fma2(add2(pack2(byte_biased(ck.y, 0), byte_biased(ck.y, 1)), bias), pack2(sz, sz),
+	         pack2(oz, oz));
+}
+
+// regular_box on a child of a compressed node: the same decode and products, every operation
+// rounded as the scalar one, in packed pairs: 12 FP instructions for 24 (a traversal of
 // compressed nodes is bound by issue).  tmax >= 0 and tmin <= tmax as max(tmin, 0) <= tmax.
 // 1,000,003 random rays on as many clustered triangles 934 -> 866 us, 2,097,152 rays on the
 // 1,048,576-triangle heightfield 1,110 -> 1,053 (z scalar: 883, 1,077).
-struct CompressedSlab {
-	float nx, fx, ny, fy, nz, fz; // near and far per axis
-};
-__device__ __forceinline__ CompressedSlab compressed_slab(const SlabRay &q, const uint2 &ck,
-                                                          unsigned long long oxy, float oz,
-                                                          unsigned long long sxy, float sz) {
-	const unsigned long long bias = pack2(-8388608.0f, -8388608.0f);
-	const unsigned long long l =
-	    fma2(add2(pack2(byte_biased(ck.x, 0), byte_biased(ck.x, 2)), bias), sxy, oxy);
-	const unsigned long long h =
-	    fma2(add2(pack2(byte_biased(ck.x, 1), byte_biased(ck.x, 3)), bias), sxy, oxy);
-	float t1, t2, t3, t4;
-	unpack2(mul2(add2(l, q.no), q.f), t1, t3);
-	unpack2(mul2(add2(h, q.no), q.f), t2, t4);
-	const unsigned long long z = fma2(add2(pack2(byte_biased(ck.y, 0), byte_biased(ck.y, 1)), bias),
-	                                  pack2(sz, sz), pack2(oz, oz));
-	float t5, t6;
-	unpack2(mul2(add2(z, pack2(-q.oz, -q.oz)), pack2(q.fz, q.fz)), t5, t6);
-	return CompressedSlab{fminf(t1, t2), fmaxf(t1, t2), fminf(t3, t4),
-	                      fmaxf(t3, t4), fminf(t5, t6), fmaxf(t5, t6)};
-}
-
 __device__ __forceinline__ bool compressed_passes(const SlabRay &q, const uint2 &ck,
                                                   unsigned long long oxy, float oz,
                                                   unsigned long long sxy, float sz) {
-	const CompressedSlab c = compressed_slab(q, ck, oxy, oz, sxy, sz);
-	return max3f(c.nx, c.ny, fmaxf(c.nz, 0.0f)) <= min3f(c.fx, c.fy, c.fz);
+	unsigned long long l, h, z;
+	compressed_bounds(ck, oxy, oz, sxy, sz, l, h, z);
+	float t1, t2, t3, t4, t5, t6;
+	unpack2(mul2(add2(l, q.no), q.f), t1, t3);
+	unpack2(mul2(add2(h, q.no), q.f), t2, t4);
+	unpack2(mul2(add2(z, pack2(-q.oz, -q.oz)), pack2(q.fz, q.fz)), t5, t6);
+	const float tmin = max3f(fminf(t1, t2), fminf(t3, t4), fmaxf(fminf(t5, t6), 0.0f));
+	const float tmax = min3f(fmaxf(t1, t2), fmaxf(t3, t4), fmaxf(t5, t6));
+	return tmin <= tmax;
 }
 
-// The same with the scales of AxisRay.
+// The same of any other ray.
 __device__ __forceinline__ bool compressed_passes(const AxisRay &x, const uint2 &ck,
                                                   unsigned long long oxy, float oz,
                                                   unsigned long long sxy, float sz) {
-	const CompressedSlab c = compressed_slab(x.q, ck, oxy, oz, sxy, sz);
-	float gx, gy, hx, hy;
-	unpack2(x.g, gx, gy);
-	unpack2(x.h, hx, hy);
-	const float nx = c.nx * gx, fx = c.fx * hx;
-	const bool outright = x.all || (x.x_passes && !(nx > 0.0f) && !(fx < 0.0f));
-	const float tmin = max3f(nx, c.ny * gy, fmaxf(c.nz * x.gz, 0.0f));
-	const float tmax = min3f(fx, c.fy * hy, c.fz * x.hz);
-	return outright || !(tmin > tmax);
+	unsigned long long l, h, z;
+	compressed_bounds(ck, oxy, oz, sxy, sz, l, h, z);
+	return axis_passes(x, l, h, z, false);
 }
 
 __device__ __forceinline__ RayC slot_ray(const WarpFixed &S, uint32_t s) {
@@ -1045,7 +1028,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				}
 				r = make_ray(p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
 			}
-			if ((PASS == 0 || PASS == 2 || PASS == 4) && (r.kind & 7) == 4 && a.x_faces &&
+			if ((PASS == 0 || PASS == 2 || PASS == 4) && r.kind == 4 && a.x_faces &&
 			    x_face_free(a.x_faces, r.ox))
 				--r.kind;
 			S.ro[lane] = make_float4(r.ox, r.oy, r.oz, __int_as_float(r.kind));

@@ -1,10 +1,12 @@
-"""The inner-box test of rays with zero direction components (prt_traverse.cu, AxisRay) must pass
-every box that holds a triangle box on which the reference's slab test passes: its arithmetic
-restated in numpy, with origins on, beside and between faces, both zeros and denormals."""
+"""The inner-box test of rays that are not regular (prt_traverse.cu, AxisRay) must pass every box
+that holds a triangle box on which the reference's slab test passes: its arithmetic restated in
+numpy, with origins on, beside and between faces, both zeros, denormals, components out of the
+regular ranges and origins up to the largest floats."""
 import numpy as np
 import pytest
 
-from test_slab_margin import COORD_MAX, DIR_MIN, F, FLT_MAX, _cases, _encode
+from test_slab_margin import DIR_MIN, F, FLT_MAX, _cases, _encode, _passes, _up
+from test_slab_margin import _reference as _regular_reference
 
 INF = F(np.inf)
 
@@ -34,39 +36,24 @@ def _bounds16(lo, hi):
     return ((down(lo).astype(np.uint32) & top).view(F), (up(hi).astype(np.uint32) & top).view(F))
 
 
-def _ray(o, d):
-    """Reciprocals, the scales of near and far, and which of the ray's axes are infinite."""
+def _bounds(c, e):
+    """Centre and half extent to bounds, rounded outwards."""
+    c, e = c.astype(np.float64), e.astype(np.float64)
+    with np.errstate(over="ignore"):
+        return -_up(e - c), _up(c + e)
+
+
+def _passes_other(lo, hi, x16, o, d, x_passes):
     with np.errstate(all="ignore"):
         f = F(1) / d
-    inf = np.isinf(f)
-    past, tiny = np.abs(o) > COORD_MAX, ~inf & (np.abs(f) > F(1) / DIR_MIN)
-    g = np.where(inf | past, INF, F(1))
-    h = np.where(inf | past | tiny, INF, F(1))
-    f = np.where(past, F(0), np.where(tiny, np.copysign(F(1) / DIR_MIN, f), f))
-    return np.where(inf, np.copysign(F(1), 1 / np.where(inf, d, F(1))), f), g, h, inf
-
-
-def _axis_passes(c, e, x16, o, d, x_passes):
-    with np.errstate(all="ignore"):
-        f, g, h, inf = _ray(o, d)
-        t = ((c - o) * f).astype(np.float64)
-        w = e.astype(np.float64) * np.abs(f).astype(np.float64)
-        near, far = (t - w).astype(F) * g, (t + w).astype(F) * h
-        outside = inf[:, 0] & ((o[:, 0] < x16[0]) | (o[:, 0] > x16[1]))
-        near[:, 0] = np.where(outside, INF, near[:, 0])
-        outright = inf[:, 0] & x_passes & ~(near[:, 0] > 0) & ~(far[:, 0] < 0)
-        tmin = np.fmax(np.fmax.reduce(near, axis=1), F(0))
-        tmax = np.fmin.reduce(far, axis=1)
-        return outright | ~(tmin > (tmax.astype(np.float64) * (1 + 2.0 ** -20)
-                                    + 2.0 ** -120).astype(F))
-
-
-def _plain_passes(lo, hi, o, d, x_passes):
-    """The same on bounds (compressed nodes)."""
-    with np.errstate(all="ignore"):
-        f, g, h, inf = _ray(o, d)
+        inf = np.isinf(f)
+        g = np.where(inf, INF, F(1))
+        f = np.where(inf, np.copysign(F(1), f), f)
         t1, t2 = (lo - o) * f, (hi - o) * f
-        near, far = np.fmin(t1, t2) * g, np.fmax(t1, t2) * h
+        near, far = np.fmin(t1, t2) * g, np.fmax(t1, t2) * g
+        if x16 is not None:
+            outside = inf[:, 0] & ((o[:, 0] < x16[0]) | (o[:, 0] > x16[1]))
+            near[:, 0] = np.where(outside, INF, near[:, 0])
         outright = inf[:, 0] & x_passes & ~(near[:, 0] > 0) & ~(far[:, 0] < 0)
         return outright | ~(np.fmax(np.fmax.reduce(near, axis=1), F(0))
                             > np.fmin.reduce(far, axis=1))
@@ -96,8 +83,8 @@ def test_passes_whatever_the_reference_passes(seed, odd):
         k = rng.integers(0, 4, (n, 3))
         d = np.where(k == 0, (d * 2.0 ** rng.uniform(-125, -58, (n, 3))).astype(F), d)
         d = np.where(rng.random((n, 1)) < 0.3, (d * F(2.0 ** 63)).astype(F), d)
-        o = np.where((k == 1) & (rng.random((n, 1)) < 0.3), F(2.0 ** 70) * np.sign(o), o)
-        ok &= ~(np.abs(o) > COORD_MAX).all(1)
+        far = (2.0 ** rng.uniform(67, 127, (n, 3))).astype(F) * np.sign(o)
+        o = np.where((k == 1) & (rng.random((n, 1)) < 0.3), far, o)
         with np.errstate(all="ignore"):
             ok &= ~np.isinf(F(1) / d).all(1)
     lo, hi, olo, ohi, o, d = (k[ok] for k in (lo, hi, olo, ohi, o, d))
@@ -108,14 +95,29 @@ def test_passes_whatever_the_reference_passes(seed, odd):
     # Where no lower face is at the origin's x, the x axis need not pass a box outright.
     free = o[:, 0] != lo[:, 0]
     for x_passes in (np.ones(len(lo), bool), ~free):
-        assert (_axis_passes(c, e, x16, o, d, x_passes) | ~want).all()
-        assert (_plain_passes(olo, ohi, o, d, x_passes) | ~want).all()
+        assert (_passes_other(*_bounds(c, e), x16, o, d, x_passes) | ~want).all()
+        assert (_passes_other(olo, ohi, None, o, d, x_passes) | ~want).all()  # compressed nodes
     # The box of a non-finite triangle, or one past the coordinate limit.
     big = np.full_like(lo, FLT_MAX)
     b16 = _bounds16(-big[:, 0], big[:, 0].copy())
     bc, be = _encode(-big, big)
     seen = _reference(-big, big, o, d)
-    assert (_axis_passes(bc, be, b16, o, d, ~free) | ~seen).all()
+    assert (_passes_other(*_bounds(bc, be), b16, o, d, ~free) | ~seen).all()
     if not odd:  # It prunes: of rays that miss by a direction component that is not zero.
         missed = ~want & free & (np.abs(o - (olo + ohi) / 2) > 4 * (ohi - olo)).any(1)
-        assert _axis_passes(c, e, x16, o, d, ~free)[missed].mean() < 0.2
+        assert _passes_other(*_bounds(c, e), x16, o, d, ~free)[missed].mean() < 0.2
+
+
+@pytest.mark.parametrize("seed", range(3))
+def test_long_directions_are_regular(seed):
+    """Reciprocals down to the denormals: what underflow loses, the margin's 2^-120 covers."""
+    rng = np.random.default_rng(200 + seed)
+    lo, hi, olo, ohi, o, d = _cases(rng, 200_000)
+    with np.errstate(over="ignore"):
+        d = (d * 2.0 ** rng.uniform(30, 127, (len(d), 1))).astype(F)
+    ok = np.isfinite(d).all(1) & (np.abs(d) >= DIR_MIN).all(1)
+    lo, hi, olo, ohi, o, d = (k[ok] for k in (lo, hi, olo, ohi, o, d))
+    want = _regular_reference(lo, hi, o, d)
+    assert want.sum() > 10_000
+    c, e = _encode(olo, ohi)
+    assert (_passes(c, e, o, d) | ~want).all()
