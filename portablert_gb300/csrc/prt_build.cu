@@ -644,7 +644,8 @@ __device__ __forceinline__ bool is_inner(uint32_t r, uint32_t count, uint32_t le
 // Level-0 frontier: the root of every scene becomes 8-wide node s; the node counter
 // starts after the roots.
 __global__ void k_collapse_roots(const uint32_t *tri_off, const uint32_t *int_off,
-                                 uint32_t n_scenes, Item *items, uint32_t *ctr) {
+                                 uint32_t n_scenes, Item *items, uint32_t *ctr,
+                                 const uint32_t *gb, float4 *far) {
 	chain_enter();
 	const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
 	if (s == 0) {
@@ -656,6 +657,9 @@ __global__ void k_collapse_roots(const uint32_t *tri_off, const uint32_t *int_of
 	const uint32_t n = tri_off[s + 1] - tri_off[s];
 	const uint32_t ref = n == 0 ? kNone : (n == 1 ? (kLeafBit | tri_off[s]) : int_off[s]);
 	items[s] = Item{ref, s};
+	const float lo[3] = {ord2f(gb[6 * s]), ord2f(gb[6 * s + 1]), ord2f(gb[6 * s + 2])};
+	const float hi[3] = {ord2f(gb[6 * s + 3]), ord2f(gb[6 * s + 4]), ord2f(gb[6 * s + 5])};
+	far[s] = far_scene(lo, hi, n);
 }
 
 __device__ __forceinline__ float open_area(uint32_t r, const float4 *ibox) {
@@ -1168,7 +1172,8 @@ int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compre
 		BUILD_TRY(ws.cost.reserve(sizeof(CostNode) * ni));
 	BUILD_TRY(sc.tri4.reserve(48 * nn));
 	BUILD_TRY(sc.inv.reserve(4 * nn));
-	// One node past the capacity: the empty node the traversal pads partial steps with.
+	// One node past the capacity: the empty node the traversal pads partial steps with; after
+	// it what tells far rays, per scene (far_scenes).
 	// As large as the triangle records' buffer may need: it moves only when that does, so that a
 	// captured query that still finds the one finds the other.
 	plan.x_log = 0;
@@ -1177,7 +1182,7 @@ int build_plan(const uint64_t *tri_off64, uint32_t S, int leaf_size, bool compre
 		plan.x_log = x_faces_log(n);
 	}
 	plan.x_drop = plan.x_log ? nullptr : sc.x_faces.as<uint32_t>();
-	BUILD_TRY(sc.nodes.reserve(sizeof(Node8) * ((size_t)plan.node_cap + 1)));
+	BUILD_TRY(sc.nodes.reserve(sizeof(Node8) * ((size_t)plan.node_cap + 1) + sizeof(float4) * S));
 	if (compressed)
 		BUILD_TRY(sc.cnodes.reserve(sizeof(CNode8) * ((size_t)plan.node_cap + 1)));
 	// Work items hold 27-bit node indices; a tree's nodes stay below n - 1 < 2^27 - 1.
@@ -1312,7 +1317,7 @@ static int collapse_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU
 
 	Item *items_of[2] = {ws.items_a.as<Item>(), ws.items_b.as<Item>()};
 	launch_after(host_checks, k_collapse_roots, blocks_for(S, 128), 128, st, d_toff, roots, S,
-	             items_of[0], ctr);
+	             items_of[0], ctr, ws.bounds.as<uint32_t>(), far_scenes(sc.nodes.p, sc.dead));
 	CollapseArgs A;
 	A.tris = d_tris;
 	A.vals = svals;

@@ -362,6 +362,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 					scan[q] = __float_as_uint(mn[q]);
 					scan[3 + q] = __float_as_uint(mx[q]);
 				}
+			if (tid == 0)
+				*reinterpret_cast<float4 *>(dead + 1) = far_scene(mn, mx, n);
 		}
 		__syncthreads();
 	}

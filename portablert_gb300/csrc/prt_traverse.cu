@@ -409,7 +409,7 @@ __device__ __forceinline__ void test_queued(const float4 *__restrict__ tri4, War
 		const float4 A = __ldg(p), B = __ldg(p + 1), C = __ldg(p + 2);
 		float t, u, v;
 		// Finite ray and triangle (nearly always): the box test with plain min/max.
-		if (tri_test(r, A, B, C, t, u, v, r.kind == 0 && tri_record_finite(B)) && t < INFINITY) {
+		if (tri_test(r, A, B, C, t, u, v, r.kind <= 1 && tri_record_finite(B)) && t < INFINITY) {
 			mykey = hit_key(t, __float_as_uint(A.w));
 			atomicMin(&S.key[slot], mykey);
 			my_slot = slot;
@@ -1006,6 +1006,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 		const uint32_t nb = min(take, run_rays - local);
 		const SceneDesc sd = (PASS == 3 || a.n_segs) ? a.scenes[S.seg.scene] : a.scene0;
 		const float4 *__restrict__ tri4 = sd.tri4;
+		float4 far = make_float4(0.0f, 0.0f, 0.0f, INFINITY);
+		if (FMT == PRT_NODES_FP32)
+			far = __ldg(reinterpret_cast<const float4 *>(static_cast<const Node8 *>(sd.nodes) + a.dead +
+			                                             1u) + sd.root);
 
 		if ((uint32_t)lane < nb) {
 			RayC r;
@@ -1028,6 +1032,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				}
 				r = make_ray(p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
 			}
+			if (FMT == PRT_NODES_FP32 && r.kind == 0 &&
+			    max3f(fabsf(r.ox - far.x), fabsf(r.oy - far.y), fabsf(r.oz - far.z)) > far.w)
+				r.kind = 1;
 			if ((PASS == 0 || PASS == 2 || PASS == 4) && r.kind == 4 && a.x_faces &&
 			    x_face_free(a.x_faces, r.ox))
 				--r.kind;
@@ -1088,7 +1095,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 				const float4 *p = tri4 + 3 * (size_t)__ldg(&sd.inv[pid]);
 				const float4 A = __ldg(p), B = __ldg(p + 1), C = __ldg(p + 2);
 				float t, u, v;
-				if (tri_test(r, A, B, C, t, u, v, r.kind == 0 && tri_record_finite(B))) {
+				if (tri_test(r, A, B, C, t, u, v, r.kind <= 1 && tri_record_finite(B))) {
 					best.t = t;
 					best.u = u;
 					best.v = v;
