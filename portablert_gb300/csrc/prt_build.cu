@@ -1383,7 +1383,7 @@ int build_enqueue(const float *d_tris, const BuildPlan &plan, SceneGPU &sc, Buil
                   cudaStream_t st, uint32_t *d_err, bool host_checks, std::string &msg) {
 	const uint32_t S = plan.S, n = plan.n;
 	if (plan.sah && !host_checks) {
-		msg = "the SAH build reads its level counters on the host";
+		msg = "the SAH build needs a look at its gate on the host";
 		return PRT_ERR_ARG;
 	}
 	if (plan.small) {

@@ -902,7 +902,7 @@ extern "C" int prt_b200_nearest_hits_noalloc(prt_b200_ctx *ctx, const float *ray
 			return fail(ctx, PRT_ERR_DEVICE, "nearest_hits_noalloc: kernel reported an error");
 		// Errors that earlier asynchronous calls on this context (the _dev calls) left in the
 		// context's own error word are reported here too, as prt_b200_nearest_hits reports
-		// them; reading it copies 4 bytes into the context's pinned word, no allocation.
+		// them; it is pinned host memory, so nothing is copied or allocated.
 		return check_device_errors(ctx);
 	});
 }

@@ -11,9 +11,9 @@
 // visit order changes the answer; ties in t go to the smaller primitive id.
 //
 // Execution: one warp = 8 groups of 4 lanes; all state for 32 rays is in shared memory.
-//  * A warp takes up to 32 consecutive rays from a global counter ("slots": 32 per
-//    batch, or 8 or 16 when one small run would leave most warps idle): origin,
-//    direction, reciprocal and best-hit key per slot live in shared memory.
+//  * A warp takes up to 32 consecutive rays ("slots": 32 per batch, or 4 to 16 where 32
+//    would leave most warps idle, single_batch): origin, direction, reciprocal and
+//    best-hit key per slot live in shared memory.
 //  * Work items (slot, node) sit in a warp-local LIFO pool.  Each step every group
 //    pops one item and each of its 4 lanes loads and slab-tests 2 of the node's 8
 //    children: lane s takes children s and s + 4, so each of the two 256-bit loads of a
@@ -26,17 +26,16 @@
 //    pipe is what bounds it).  Roots of new rays are admitted whenever fewer than 8
 //    items are left.  Unused child slots hold NaN boxes, which no plain slab test
 //    passes.
-//  * A query of ray buffers is two launches: a regular pass over the batches whose 32
-//    rays are all regular (kind 0: the plain slab test only), which counts and skips
-//    the others, and a deferred pass over those with the other test (AxisRay), for instance for
-//    zero direction components (it returns at once when there are none).  Camera queries and
-//    counting runs are one general launch, in which a batch of regular rays takes the
-//    plain test; batches of large images of few triangles start with a packet descent
-//    (packet_descent).  Queries of up to some hundred rays per warp and other cameras are
-//    one launch as well (single_batch).  A request
-//    server's serving launch (pass 3) takes its batches from device queues that the host
-//    extends while it runs (claim_batch) and picks the plain or the general test per
-//    batch.
+//  * A batch whose rays are all regular (kind 0) takes the plain slab test (SlabRay) on
+//    FP32 nodes, any other the test on bounds (AxisRay): rays with zero direction
+//    components, mostly, and rays from far away.  Queries of up to some hundred rays per
+//    warp and most cameras are one launch with both (pass 4, single_batch).  Larger
+//    queries of ray buffers are two: a regular pass (1), which holds the plain test alone
+//    and counts and skips the other batches, and a deferred pass (2) over those (it
+//    returns at once when there are none).  Large images of few triangles (pass 0) start
+//    each regular batch with a packet descent (packet_descent); counting runs are pass 0
+//    as well.  A request server's serving launch (pass 3) takes its batches from device
+//    queues that the host extends while it runs (claim_batch).
 //  * When 32 triangles are queued, the 32 lanes test one each with the exact reference
 //    test and fold (t, primitive id) into the slot's 64-bit key with a shared atomicMin;
 //    with FP32 nodes the lane whose key the slot kept records its u, v (and a zero t's
@@ -50,6 +49,10 @@
 //
 // Algorithmic bytes per ray: 24 (ray) + R (record) + node bytes visited + 48 per
 // triangle tested; the counting variant (COUNT) measures the visits.
+//
+// Times in these comments are of the step they stand beside, both sides in turn on one GPU;
+// the same workload differs by up to a tenth from one sitting to another, and later steps
+// have shortened it since.
 #include <algorithm>
 #include <type_traits>
 #include <mutex>
@@ -98,7 +101,7 @@ struct TravArgs {
 	uint32_t max_leaf;       // most triangles in a leaf of any scene of the launch
 	uint32_t max_batches;    // batches per warp before it exits (0 = no bound)
 	uint32_t batch;          // rays a warp takes at a time: 32, or 4 to 16 where few rays
-	                         // are to keep all warps busy (single_batch, batch_rays)
+	                         // are to keep all warps busy (single_batch)
 	uint32_t claims;         // PASS 4: rays per batch after a warp's first one (0: there are no
 	                         // more batches than warps)
 	uint32_t *counter;
@@ -880,7 +883,7 @@ __device__ __forceinline__ bool claim_batch(const ServeQueues &q, uint32_t held[
 // BOUNDED: a warp takes at most a.max_batches batches (a separate instantiation, so the
 // unbounded kernels keep their register allocation).
 // PASS: 0 = every batch with the general box test (the counting runs); 1 = batches whose
-// rays all have finite reciprocals, with the plain slab test only (no conservative code
+// rays are all regular, with the plain slab test only (no conservative code
 // in the kernel at all: 8 % faster), the others counted in a.deferred and skipped; 2 =
 // the skipped batches with the general test (returns at once when there are none); 3 =
 // a serving launch: batches claimed from the serving queues (claim_batch), the plain or
@@ -1047,7 +1050,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 
 		bool fault = false; // the batch's traversal reported an error (warp-uniform)
 		if (sd.n_tris) {
-			// Nearly every batch has only rays with finite reciprocals.
+			// Nearly every batch has only regular rays.
 			const bool regular =
 			    __all_sync(0xFFFFFFFFu, (uint32_t)lane >= nb || __float_as_int(S.ro[lane].w) == 0);
 			if (PASS == 1 && !regular) {
@@ -1128,7 +1131,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, PASS == 4 ? PRT_TRAVERSE_
 		uint8_t *dst = S.seg.out + (size_t)local * rec;
 		const uint32_t bytes = nb * rec;
 		const uint32_t mode = S.seg.store_mode;
-		if (mode == 0 && (bytes & 15u) == 0u) { // local is a multiple of 8: 16-byte aligned
+		if (mode == 0 && (bytes & 15u) == 0u) { // local is a multiple of 4: 16-byte aligned
 			uint4 *d4 = reinterpret_cast<uint4 *>(dst);
 			const uint4 *s4 = reinterpret_cast<const uint4 *>(stage);
 			for (uint32_t k = lane; k < bytes / 16u; k += 32u)
@@ -1369,10 +1372,9 @@ void size_smem(TravArgs &a, uint32_t depth, int leaf_size) {
 	a.warp_bytes = (warp_smem_bytes(a.pool_cap, a.queue_cap) + 15u) & ~15u;
 }
 
-// Rays per warp batch for one run of m rays: 32 when the launch holds at least two
-// batches for every resident warp (about 36 per SM), else 16, else 8: a small query
-// then spreads over all warps instead of leaving most of them idle while a few walk 32
-// rays each (bounded waves keep 32: their batch count per warp is the caller's).
+// Rays per batch of a run of m rays that is not one kernel: 32, but for counting runs of few
+// rays, where 8 or 16 keep more warps busy (bounded waves keep 32: their batch count per warp
+// is the caller's).
 uint32_t batch_rays(uint64_t m, int sm_count, uint32_t max_batches) {
 	const uint64_t wave = (uint64_t)std::max(sm_count, 1) * 36u * 32u;
 	if (max_batches > 0 || m >= 2 * wave)
