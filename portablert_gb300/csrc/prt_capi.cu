@@ -615,8 +615,17 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 		ctx->last_in_place = false;
 		bool pageable = false;
 		prt::device_alias(ctx, out_host, &pageable);
-		if (pageable && pages_to_populate(out_host, (uint64_t)rec_size * n, rays6, 24ull * n))
-			populate_pages(out_host, (uint64_t)rec_size * n); // (the copies out fault as well)
+		// The copies out fault as well.  One piece of output at once, a larger one piece by
+		// piece between the chunks below (6.4, 66 and 192 MB of records: 522, 3,440 and 9,400 us
+		// all at once, 535, 3,300 and 8,970 in pieces).
+		const uint64_t out_bytes = (uint64_t)rec_size * n;
+		uint64_t populated = out_bytes;
+		if (pageable && pages_to_populate(out_host, out_bytes, rays6, 24ull * n)) {
+			if (out_bytes > kPopulateBytes)
+				populated = 0;
+			else
+				populate_pages(out_host, out_bytes);
+		}
 		CAPI_TRY(ctx, ctx->rays_buf.reserve(24ull * n));
 		CAPI_TRY(ctx, ctx->out_buf.reserve((uint64_t)rec_size * n));
 		// Chunks: pipe_chunks of them (fewer when a chunk would hold under pipe_min_rays), one
@@ -668,9 +677,16 @@ int prt_b200_nearest_hits(prt_b200_ctx *ctx, const float *rays6, uint64_t n, uin
 			}
 			// The copy-out of the chunk before is queued after this chunk's copy-in, so that
 			// with pageable host memory (where the copy calls return only when done) the
-			// copy-in still overlaps the traversal.
+			// copy-in still overlaps the traversal.  Its pages are populated here, while the
+			// device works on both chunks.
 			if (c > 0) {
 				const uint64_t b = bnd[c - 1], m = bnd[c] - bnd[c - 1];
+				if (populated < (uint64_t)rec_size * bnd[c]) {
+					const uint64_t to = std::min(
+					    out_bytes, std::max((uint64_t)rec_size * bnd[c], populated + kPopulateBytes));
+					populate_pages(rout + populated, to - populated);
+					populated = to;
+				}
 				CAPI_TRY(ctx, cudaStreamWaitEvent(ctx->s_out, ctx->ev_k[c - 1], 0));
 				CAPI_TRY(ctx, cudaMemcpyAsync(rout + (uint64_t)rec_size * b,
 				                              ctx->out_buf.as<uint8_t>() + (uint64_t)rec_size * b,

@@ -1,9 +1,11 @@
 // A CUDA runtime without a GPU, for tests of host code: preloaded before libcudart it gives the
 // library one device of compute capability 10.3 that reads pageable memory, whose memory is
 // the host's and whose kernels do nothing.  It remembers which streams hold work that nobody
-// has waited for and the names of the kernels launched, and a test can make a later launch
-// fail.
+// has waited for, the names of the kernels launched and the pages populated between them, and
+// a test can make a later launch fail.
 #include <cuda_runtime_api.h>
+#include <sys/syscall.h>
+#include <unistd.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -22,6 +24,8 @@ std::map<const void *, std::string> &names() { // of kernels, by their host func
 	return m;
 }
 std::string launched; // names, one per line
+std::string populated; // "launches before it, bytes" of each MADV_POPULATE_WRITE, one per line
+long n_launches = 0;
 char handles[4096];
 int n_handles = 0;
 
@@ -32,6 +36,7 @@ cudaError_t queued(void *st) {
 }
 cudaError_t launch(void *st, const void *fun = nullptr) {
 	launched += names()[fun] + "\n";
+	++n_launches;
 	if (fail_in > 0 && --fail_in == 0)
 		return last = cudaErrorLaunchOutOfResources;
 	return queued(st);
@@ -41,7 +46,14 @@ cudaError_t launch(void *st, const void *fun = nullptr) {
 FAKE void fake_fail_launch(long k) { fail_in = k; }
 FAKE long fake_pending() { return (long)pending.size(); }
 FAKE const char *fake_launched() { return launched.c_str(); }
-FAKE void fake_forget_launched() { launched.clear(); }
+FAKE void fake_forget_launched() { launched.clear(), populated.clear(), n_launches = 0; }
+FAKE const char *fake_populated() { return populated.c_str(); }
+
+FAKE int madvise(void *p, size_t n, int advice) noexcept {
+	if (advice == 23) // MADV_POPULATE_WRITE
+		populated += std::to_string(n_launches) + " " + std::to_string(n) + "\n";
+	return (int)syscall(SYS_madvise, p, n, advice);
+}
 
 FAKE cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
 FAKE cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
