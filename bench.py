@@ -73,14 +73,16 @@ def traversal_rooflines(n, per_launch_s, b_ray, v_nodes, v_tris, node_size, rec_
 
     * issue: warp instructions per launch (ncu, committed summary) over the launch time,
       against 4 issue slots per SM per cycle at the median SM clock of the timed region;
-    * l2: the node and triangle bytes the traversal requests (visits x 256 B + tests x
-      48 B per ray) against the read bandwidth of its own 32-byte loads from an
-      L2-resident buffer (prt_b200_probe_read, measured in this run);
+    * l2: the bytes that L1 reads from L2 per launch (ncu, committed summary) against the
+      read bandwidth of the traversal's own 32-byte loads from an L2-resident buffer
+      (prt_b200_probe_read, measured in this run); beside it the node and triangle bytes
+      that it requests (visits x 256 B + tests x 48 B per ray), of which L1 serves the rest;
     * hbm: DRAM bytes per launch (ncu, committed summary) against the measured HBM peak;
       beside it the per-ray algorithmic bytes (24 B ray + record + node and triangle
       fetches) against the same peak, which exceeds 1 because L2 serves most fetches."""
     traffic = committed_profile("dram_bytes_per_launch")
     inst = committed_profile("warp_instructions_per_launch")
+    l2_read = committed_profile("l2_read_bytes_per_launch")
     at = committed_profile("captured_at", text=True)
     src = f"{PROFILE} (ncu, traversal of commit {at})"
     alg = n * b_ray / per_launch_s / 1e9
@@ -91,8 +93,10 @@ def traversal_rooflines(n, per_launch_s, b_ray, v_nodes, v_tris, node_size, rec_
                   "warp_instructions_per_ray": inst / n if inst else None,
                   "warp_instructions_per_node_visit": inst / n / v_nodes if inst else None,
                   "source": src, "sm_mhz": sm_mhz, "sms": sms},
-        "l2": {"achieved": fetch, "peak": l2_peak, "unit": "GB/s",
-               "bytes_per_ray": v_nodes * node_size + v_tris * 48,
+        "l2": {"achieved": l2_read / per_launch_s / 1e9 if l2_read else None,
+               "peak": l2_peak, "unit": "GB/s", "traffic": l2_read, "traffic_source": src,
+               "requested": {"achieved": fetch,
+                             "bytes_per_ray": v_nodes * node_size + v_tris * 48},
                "peak_source": "prt_b200_probe_read: 32-byte loads over a 48 MiB buffer, "
                               "this run"},
         "hbm": {"achieved": traffic / per_launch_s / 1e9 if traffic else None, "peak": peak,
